@@ -7,6 +7,33 @@
 
 namespace nbg {
 
+// Programmatic dependent launch: a kernel launched with launch_dependent may start
+// while its predecessor in the stream still runs.  pdl_wait returns when the
+// predecessor has finished and its writes are visible; pdl_trigger lets the successor
+// start (once every CTA has called it or left).
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... Params, class... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, int threads, size_t smem,
+                             cudaStream_t stream, Args... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Integrate (or write accelerations for) one real particle.
 __device__ __forceinline__ void finish_particle(const ForceArgs& a, const SystemDesc& sd,
                                                 int64_t gi, float fx, float fy, float fz,

@@ -19,6 +19,27 @@ cudaError_t launch_force(int index, bool compensated, bool per_pair_mass, bool l
 cudaError_t force_blocks_per_sm(int index, bool compensated, bool per_pair_mass, bool live,
                                 int* blocks);
 
+// ---- symmetric force step (symmetric_kernel.cuh, symmetric_add.cu) -------------------
+struct SymSegment;
+struct SymTile;
+struct SymArgs {
+  ForceArgs f;               // pos, pos_next, vel, accel_out, sys, partials, eps2, dt, ...
+  const SymSegment* segs;    // the band's, linked (link_segments)
+  const SymTile* tiles;      // every i-tile
+  float* rows;               // [3][plane] j-side sums
+  int64_t plane;
+  float4* carry;             // [n_pad][2] running sums between bands
+  int32_t tile0, tile1;      // the band's i-tiles
+};
+int num_symmetric_shapes();
+KernelShape symmetric_shape(int index);  // threads, i-particles per thread, j-tile, 0 stages
+cudaError_t symmetric_blocks_per_sm(int index, bool compensated, bool per_pair_mass, int* blocks);
+cudaError_t launch_symmetric(int index, bool compensated, bool per_pair_mass, const SymArgs& a,
+                             int grid, cudaStream_t stream);
+// Add the rows and parts of the band's i-tiles and integrate; `tiles` i-tiles from a.tile0.
+cudaError_t launch_symmetric_add(bool compensated, const SymArgs& a, int tiles, int bi,
+                                 cudaStream_t stream);
+
 // ---- compatibility kernel (aux_kernels.cu) ------------------------------------------
 // The reference's PREDICATED variant as shipped, one thread per i-particle over one
 // system (simulator.cu:186-229 with the (i == id) mask of :208-209).

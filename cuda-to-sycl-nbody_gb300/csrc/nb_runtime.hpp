@@ -14,11 +14,12 @@
 #include "nb_kernels.hpp"
 #include "nb_render.hpp"
 #include "nbody_gb300.h"
+#include "symmetric.hpp"
 
 namespace nbg {
 
-// A work list on the device.  cfg >= 0: a shape of the tuned force kernel;
-// cfg < 0: reference-order shape -1 - cfg.
+// A work list on the device.  cfg >= 0: a shape of the tuned force kernel, or, from
+// num_force_configs() on, of the symmetric one; cfg < 0: reference-order shape -1 - cfg.
 struct WorkListDev {
   int32_t cfg = -1;
   bool live = false;  // the force kernel's live-slot variant (planned with its weights)
@@ -30,6 +31,11 @@ struct WorkListDev {
   Segment* segs = nullptr;
   int32_t* seg_begin = nullptr;
   Fixup* fix = nullptr;
+  // Symmetric kernel: its segments and i-tiles, and the bands they run in.
+  SymSegment* sym_segs = nullptr;
+  SymTile* sym_tiles = nullptr;
+  std::vector<SymBand> bands;
+  int64_t row_values = 0;
 };
 
 // Checkpoints and work buffers of the adjoint (allocated on first use).
@@ -82,7 +88,9 @@ struct nb_sim {
   int32_t inject = 0;  // one-shot failure-detection hook for the next force launch (kInject*)
 
   int cfg = 0;
+  bool cfg_default = true;       // cfg is default_config's choice
   nbg::WorkListDev wl;
+  nbg::WorkListDev inject_wl;    // a tuned-kernel list for failure-detection launches
   std::vector<nbg::WorkListDev> wl_sys;
   int wl_sys_policy = -1;  // how wl_sys was planned (kPerSystem*), -1: not yet
   int wl_sys_cfg = 0;      // and with which shape, for kPerSystemSimShape
@@ -90,6 +98,9 @@ struct nb_sim {
   size_t partials_cap = 0;
   int32_t* counters_d = nullptr;
   size_t counters_cap = 0;
+  float* rows_d = nullptr;       // symmetric kernel: [3][row values] j-side sums
+  size_t rows_cap = 0;
+  float4* carry_d = nullptr;     // symmetric kernel, several bands: [n_pad][2]
 
   // NB_ACC_REFERENCE_ORDER: the reference-order kernel's shape, its work list
   // (config index -1 - shape) and the duplicated j-layout of the positions.

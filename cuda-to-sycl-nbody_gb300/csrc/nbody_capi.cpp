@@ -73,6 +73,8 @@ void free_worklist(WorkListDev& w) {
   dev_free(w.segs);
   dev_free(w.seg_begin);
   dev_free(w.fix);
+  dev_free(w.sym_segs);
+  dev_free(w.sym_tiles);
   w = WorkListDev{};
 }
 
@@ -178,9 +180,27 @@ static void drop_graphs(nb_sim* s) {
   s->graph_iters = 0;
 }
 
-// Shape of work-list config `cfg` (>= 0: tuned kernel; < 0: reference order).
+// Config indices: the tuned kernel's shapes, then the symmetric kernel's.
+static int num_configs() { return num_force_configs() + num_symmetric_shapes(); }
+static bool is_symmetric(int cfg) { return cfg >= num_force_configs(); }
+
+// Shape of work-list config `cfg` (>= 0: tuned or symmetric kernel; < 0: reference order).
 static KernelShape shape_of(int cfg) {
+  if (is_symmetric(cfg)) return symmetric_shape(cfg - num_force_configs());
   return cfg >= 0 ? force_config_shape(cfg) : reference_order_shape(-1 - cfg);
+}
+
+// Replace *p by a larger buffer; the current one stays (and serves the current work
+// list) when the allocation fails.
+template <class T>
+static int grow(T** p, size_t* cap, size_t need) {
+  if (need <= *cap) return NB_OK;
+  T* q = nullptr;
+  NB_TRY(dev_alloc(&q, need));
+  dev_free(*p);
+  *p = q;
+  *cap = need;
+  return NB_OK;
 }
 
 static int ensure_scratch(nb_sim* s, const WorkListDev& w) {
@@ -189,17 +209,17 @@ static int ensure_scratch(nb_sim* s, const WorkListDev& w) {
   // otherwise (the reference-order kernel's hand-over holds one float4 per particle).
   const size_t rec = (w.cfg >= 0 && s->params.accumulator == NB_ACC_COMPENSATED) ? 2 : 1;
   const size_t need = static_cast<size_t>(w.slots) * sh.bi() * rec;
-  if (need > s->partials_cap || static_cast<size_t>(w.nfix) > s->counters_cap) drop_graphs(s);
-  if (need > s->partials_cap) {
-    dev_free(s->partials_d);
-    NB_TRY(dev_alloc(&s->partials_d, need));
-    s->partials_cap = need;
-  }
+  const size_t rows = 3 * static_cast<size_t>(w.row_values);
+  if (need > s->partials_cap || static_cast<size_t>(w.nfix) > s->counters_cap ||
+      rows > s->rows_cap)
+    drop_graphs(s);
+  NB_TRY(grow(&s->rows_d, &s->rows_cap, rows));
+  NB_TRY(grow(&s->partials_d, &s->partials_cap, need));
+  if (w.bands.size() > 1 && !s->carry_d)
+    NB_TRY(dev_alloc(&s->carry_d, 2 * static_cast<size_t>(s->n_pad)));
   if (static_cast<size_t>(w.nfix) > s->counters_cap) {
-    dev_free(s->counters_d);
-    NB_TRY(dev_alloc(&s->counters_d, static_cast<size_t>(w.nfix)));
+    NB_TRY(grow(&s->counters_d, &s->counters_cap, static_cast<size_t>(w.nfix)));
     NB_CUDA(cudaMemsetAsync(s->counters_d, 0, w.nfix * sizeof(int32_t), s->stream));
-    s->counters_cap = w.nfix;
   }
   return NB_OK;
 }
@@ -207,10 +227,13 @@ static int ensure_scratch(nb_sim* s, const WorkListDev& w) {
 static int max_grid_for(nb_sim* s, int cfg, bool live = false) {
   int blocks = 0;
   const bool comp = s->params.accumulator == NB_ACC_COMPENSATED;
-  const cudaError_t e =
-      cfg >= 0 ? force_blocks_per_sm(cfg, comp, s->per_pair_mass, live, &blocks)
-               : reference_order_blocks_per_sm(-1 - cfg, s->params.calc_method == NB_PREDICATED,
-                                               &blocks);
+  cudaError_t e;
+  if (is_symmetric(cfg))
+    e = symmetric_blocks_per_sm(cfg - num_force_configs(), comp, s->per_pair_mass, &blocks);
+  else if (cfg >= 0)
+    e = force_blocks_per_sm(cfg, comp, s->per_pair_mass, live, &blocks);
+  else
+    e = reference_order_blocks_per_sm(-1 - cfg, s->params.calc_method == NB_PREDICATED, &blocks);
   if (e != cudaSuccess || blocks < 1) blocks = 1;
   return blocks * s->sms;
 }
@@ -266,17 +289,58 @@ static int plan_tuned(nb_sim* s, int cfg, int32_t first, int32_t count, int grid
   return NB_OK;
 }
 
+// Plan systems [first, first + count) for symmetric-kernel config `cfg`.
+static int plan_sym(nb_sim* s, int cfg, int32_t first, int32_t count, WorkListDev* out) {
+  const KernelShape sh = shape_of(cfg);
+  const SymPlanHost h = plan_symmetric(s->sys_h.data(), first, count, sh.bi(), sh.bj,
+                                       max_grid_for(s, cfg), kSymScratchBytes / kSymRowBytes);
+  WorkListDev w;
+  w.cfg = cfg;
+  w.grid = h.bands[0].grid;
+  w.nseg = static_cast<int32_t>(h.segs.size());
+  w.slots = h.slots;
+  w.split = h.split_tiles;
+  w.bands = h.bands;
+  w.row_values = h.row_values;
+  const std::vector<SymSegment> segs = link_segments(h);
+  int st = dev_alloc(&w.sym_segs, segs.size());
+  if (st == NB_OK) st = dev_alloc(&w.sym_tiles, h.tiles.size());
+  if (st == NB_OK) st = ensure_scratch(s, w);
+  if (st != NB_OK) {
+    free_worklist(w);
+    return st;
+  }
+  cudaError_t e = cudaMemcpyAsync(w.sym_segs, segs.data(), segs.size() * sizeof(SymSegment),
+                                  cudaMemcpyHostToDevice, s->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(w.sym_tiles, h.tiles.data(), h.tiles.size() * sizeof(SymTile),
+                        cudaMemcpyHostToDevice, s->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);  // host vectors die on return
+  if (e != cudaSuccess) {
+    free_worklist(w);
+    return cuda_error(e, "upload work list");
+  }
+  *out = w;
+  return NB_OK;
+}
+
+// Plan systems [first, first + count) for config `cfg` >= 0 at its full grid.
+static int plan_config(nb_sim* s, int cfg, int32_t first, int32_t count, WorkListDev* out) {
+  return is_symmetric(cfg) ? plan_sym(s, cfg, first, count, out)
+                           : plan_tuned(s, cfg, first, count, 0, out);
+}
+
 // (Re)build the all-systems work list for kernel config `cfg`.
 static int build_main_worklist(nb_sim* s, int cfg) {
   WorkListDev w;
-  NB_TRY(plan_tuned(s, cfg, 0, static_cast<int32_t>(s->sys_h.size()), 0, &w));
+  NB_TRY(plan_config(s, cfg, 0, static_cast<int32_t>(s->sys_h.size()), &w));
   drop_graphs(s);
   free_worklist(s->wl);
   s->wl = w;
   return NB_OK;
 }
 
-static int default_config_for(nb_sim* s, int32_t first, int32_t count);
+static int default_config_for(nb_sim* s, int32_t first, int32_t count, bool symmetric = true);
 static int default_reference_order_for(nb_sim* s, int32_t first, int32_t count);
 
 static bool reference_order_mode(const nb_sim* s) {
@@ -328,7 +392,7 @@ static int build_per_system_worklists(nb_sim* s, int policy) {
       cfg = ro ? -1 - default_reference_order_for(s, k, 1) : default_config_for(s, k, 1);
     WorkListDev w;
     if (cfg >= 0) {
-      NB_TRY(plan_tuned(s, cfg, k, 1, 0, &w));
+      NB_TRY(plan_config(s, cfg, k, 1, &w));
     } else {
       const KernelShape sh = shape_of(cfg);
       const WorkListHost h = plan_worklist(s->sys_h.data(), k, 1, sh.bi(), sh.bj,
@@ -366,9 +430,30 @@ ForceArgs base_args(nb_sim* s) {
   return a;
 }
 
-int launch_with(nb_sim* s, ForceArgs a, const WorkListDev& w) {
+int launch_with(nb_sim* s, ForceArgs a, const WorkListDev& list) {
   a.inject = s->inject;
   s->inject = 0;
+  // The failure hooks make a bounded wait run out; the symmetric kernel has none.
+  const WorkListDev& w = a.inject != 0 && is_symmetric(list.cfg) ? s->inject_wl : list;
+  if (is_symmetric(w.cfg)) {
+    const int shape = w.cfg - num_force_configs();
+    const int bi = shape_of(w.cfg).bi();
+    const bool comp = s->params.accumulator == NB_ACC_COMPENSATED;
+    SymArgs sa{};
+    sa.f = a;
+    sa.tiles = w.sym_tiles;
+    sa.rows = s->rows_d;
+    sa.plane = w.row_values;
+    sa.carry = s->carry_d;
+    for (const SymBand& b : w.bands) {
+      sa.segs = w.sym_segs + b.seg0;
+      sa.tile0 = b.tile0;
+      sa.tile1 = b.tile1;
+      NB_CUDA(launch_symmetric(shape, comp, s->per_pair_mass, sa, b.grid, s->stream));
+      NB_CUDA(launch_symmetric_add(comp, sa, b.end - b.tile0, bi, s->stream));
+    }
+    return NB_OK;
+  }
   a.segs = w.segs;
   a.seg_begin = w.seg_begin;
   a.fix = w.fix;
@@ -428,14 +513,63 @@ int check_error_word(nb_sim* s) {
   return NB_OK;
 }
 
-// Default kernel shape: the one with the largest tiles whose work list still gives
-// every CTA at least 16 (i-tile, j-tile) blocks, so that the stream-K split balances
-// to within a few percent; the smallest shape otherwise.  Deterministic (the
-// autotuner may pick otherwise, and shapes round differently).  Measured against
-// the autotuner's pick: N = 25,600 -> 256 x 2 x 256 (0.24 ms, the 1M shape takes
-// 0.32), 65,536 -> 256 x 4 x 1024, 262,144 and 1M -> 256 x 4 x 2048.
-// default_config_for judges systems [first, first + count) alone.
-static int default_config_for(nb_sim* s, int32_t first, int32_t count) {
+static bool sharded(const nb_sim* s) {
+  return s->sys_h[0].shard_first != 0 || s->sys_h[0].shard_count != 0;
+}
+
+// Default symmetric-kernel config for systems [first, first + count).  Larger i-tiles
+// run their pairs at a higher rate but leave more of them on the diagonal and in a
+// system's last tile, and make fewer blocks to balance.  So: the shape with the lowest
+// charge over rate among those with enough blocks per CTA.  Rates are measured at
+// N = 1,048,576 (229.9, 251.8, 267.2 and 373.1 ms per step, where all are balanced and
+// nearly nothing is diagonal); the blocks, at the sizes of single systems where two
+// neighbouring shapes meet (thin disks, us per step with the larger / the smaller
+// i-tiles): 36,000 319 / 315 and 50,000 587 / 598 for 4,096 against 512 particles;
+// 12,800 55.2 / 50.7 and 25,600 167.4 / 172.5 for 512 against 256; 4,096 14.7 / 14.0
+// and 8,192 25.7 / 30.3 for 256 against 64.
+static int default_symmetric_for(nb_sim* s, int32_t first, int32_t count) {
+  static const struct {
+    double rate, blocks_per_cta;
+  } kShapes[] = {{1.0, 12.0}, {0.913, 7.0}, {0.86, 0.8}, {0.617, 0.0}};
+  const int shapes = num_symmetric_shapes();
+  int best = shapes - 1;
+  double best_time = DBL_MAX;
+  for (int k = 0; k < shapes; ++k) {
+    const KernelShape sh = symmetric_shape(k);
+    double charge = 0, blocks = 0;
+    for (int32_t q = first; q < first + count; ++q) {
+      const double npad = s->sys_h[q].npad, bi = sh.bi();
+      const double tiles = (s->sys_h[q].n + sh.bi() - 1) / sh.bi();
+      const double last = npad - (tiles - 1) * bi;                // columns of the last i-tile
+      const double cols = tiles * npad - bi * tiles * (tiles - 1) / 2;
+      const double diag = (tiles - 1) * bi + last;
+      charge += bi * (kSymDiagCost * diag + kSymPairCost * (cols - diag));
+      blocks += cols / sh.bj;
+    }
+    const double time = charge / kShapes[k].rate;
+    if (time < best_time &&
+        blocks >= kShapes[k].blocks_per_cta * max_grid_for(s, num_force_configs() + k)) {
+      best = k;
+      best_time = time;
+    }
+  }
+  return num_force_configs() + best;
+}
+
+// Default kernel shape of systems [first, first + count), judged alone: a symmetric one,
+// at every size (thin disks, us per step, tuned / symmetric: N = 64 4.9 / 4.1, 2,048
+// 12.3 / 8.5, 25,600 242 / 167, 262,144 21,712 / 14,494, 1,048,576 346,673 / 229,887;
+// ensembles of 4,096 systems up to 8,192 particles 10,577 / 7,739, of 2,000 up to 300
+// 49.8 / 43.4).  Deterministic (the autotuner may pick otherwise, and shapes round
+// differently).  A shard integrates part of a system against all of it, which is not
+// symmetric, and launches that must fail on purpose need the tuned kernel's waits
+// (`symmetric` false): there, the tuned shape with the largest tiles whose work list
+// still gives every CTA at least 16 (i-tile, j-tile) blocks, so that the stream-K split
+// balances to within a few percent; the smallest shape otherwise.  Measured against the
+// autotuner's pick among the tuned shapes: N = 25,600 -> 256 x 2 x 256 (0.24 ms, the 1M
+// shape takes 0.32), 65,536 -> 256 x 4 x 1024, 262,144 and 1M -> 256 x 4 x 2048.
+static int default_config_for(nb_sim* s, int32_t first, int32_t count, bool symmetric) {
+  if (symmetric && !sharded(s)) return default_symmetric_for(s, first, count);
   static const int kCandidates[] = {9, 8, 10, 3, 4};  // largest tiles first
   for (const int cfg : kCandidates) {
     const KernelShape sh = force_config_shape(cfg);
@@ -450,8 +584,20 @@ static int default_config_for(nb_sim* s, int32_t first, int32_t count) {
   return 4;
 }
 
-static int default_config(nb_sim* s) {
-  return default_config_for(s, 0, static_cast<int32_t>(s->sys_h.size()));
+// The all-systems work list of the default config.  Where the symmetric kernel's
+// scratch does not fit the device any more, the tuned kernel's shape instead.
+static int build_default_worklist(nb_sim* s) {
+  const int32_t nsys = static_cast<int32_t>(s->sys_h.size());
+  int cfg = default_config_for(s, 0, nsys);
+  int st = build_main_worklist(s, cfg);
+  if (st == NB_ERR_OUT_OF_MEMORY && is_symmetric(cfg)) {
+    cfg = default_config_for(s, 0, nsys, false);
+    st = build_main_worklist(s, cfg);
+  }
+  NB_TRY(st);
+  s->cfg = cfg;
+  s->cfg_default = true;
+  return NB_OK;
 }
 
 // i-tiles of reference-order shape `shape` over systems [first, first + count).
@@ -582,8 +728,7 @@ static int create_impl(const nb_params* p, uint32_t num_systems, const uint32_t*
   if ((e = cudaMemcpyAsync(s->pos_d[1], s->pos_d[0], 4 * sizeof(float) * s->n_pad,
                            cudaMemcpyDeviceToDevice, s->stream)) != cudaSuccess)
     return fail(cuda_error(e, "copy state"));
-  s->cfg = default_config(s);
-  if ((st = build_main_worklist(s, s->cfg)) != NB_OK) return fail(st);
+  if ((st = build_default_worklist(s)) != NB_OK) return fail(st);
   if (sequential_order_mode(s)) {
     s->ro_shape = default_reference_order_for(s, 0, static_cast<int32_t>(s->sys_h.size()));
     if ((st = build_reference_order_worklist(s, s->ro_shape)) != NB_OK) return fail(st);
@@ -743,7 +888,10 @@ int nb_sim_destroy(nb_sim* s) {
     if (s->graph[b]) cudaGraphDestroy(s->graph[b]);
   }
   free_worklist(s->wl);
+  free_worklist(s->inject_wl);
   for (auto& w : s->wl_sys) free_worklist(w);
+  dev_free(s->rows_d);
+  dev_free(s->carry_d);
   dev_free(s->sys_d);
   dev_free(s->map_d);
   dev_free(s->pos_d[0]);
@@ -931,12 +1079,12 @@ int nb_sim_export_device(nb_sim* s, float* pos_xyzm_device, float* vel_xyzw_devi
   return NB_OK;
 }
 
-int nb_num_kernel_configs(void) { return num_force_configs(); }
+int nb_num_kernel_configs(void) { return num_configs(); }
 
 int nb_kernel_config_info(int32_t index, nb_kernel_info* info) {
-  if (!info || index < -reference_order_num_shapes() || index >= num_force_configs())
+  if (!info || index < -reference_order_num_shapes() || index >= num_configs())
     return set_error(NB_ERR_INVALID_ARGUMENT, "bad config index");
-  const KernelShape sh = index >= 0 ? force_config_shape(index) : reference_order_shape(-1 - index);
+  const KernelShape sh = shape_of(index);
   *info = nb_kernel_info{index, sh.threads, sh.r, sh.bj, sh.stages, 0, 0, 0, 0};
   return NB_OK;
 }
@@ -955,11 +1103,14 @@ int nb_sim_set_kernel_config(nb_sim* s, int32_t index) {
     s->ro_shape = shape;
     return NB_OK;
   }
-  if (index < -1 || index >= num_force_configs())
+  if (index < -1 || index >= num_configs())
     return set_error(NB_ERR_INVALID_ARGUMENT, "bad config index");
-  const int cfg = index < 0 ? default_config(s) : index;
-  NB_TRY(build_main_worklist(s, cfg));
-  s->cfg = cfg;
+  if (index < 0) return build_default_worklist(s);
+  if (is_symmetric(index) && sharded(s))
+    return set_error(NB_ERR_INVALID_ARGUMENT, "the symmetric shapes need the whole system");
+  NB_TRY(build_main_worklist(s, index));
+  s->cfg = index;
+  s->cfg_default = false;
   return NB_OK;
 }
 
@@ -971,7 +1122,7 @@ int nb_sim_kernel_info(const nb_sim* s, nb_kernel_info* info) {
                            s->ro_wl.grid, s->ro_wl.nseg, s->ro_wl.split, 0};
     return NB_OK;
   }
-  const KernelShape sh = force_config_shape(s->cfg);
+  const KernelShape sh = shape_of(s->cfg);
   *info = nb_kernel_info{s->cfg, sh.threads, sh.r, sh.bj, sh.stages,
                          s->wl.grid, s->wl.nseg, s->wl.split, s->wl.live ? 1 : 0};
   return NB_OK;
@@ -1013,8 +1164,10 @@ int nb_sim_autotune(nb_sim* s, int32_t* chosen) {
   }
   int best = s->cfg;
   float best_ms = 1e30f;
-  for (int c = 0; c < num_force_configs(); ++c) {
-    NB_TRY(build_main_worklist(s, c));
+  for (int c = 0; c < (sharded(s) ? num_force_configs() : num_configs()); ++c) {
+    const int st = build_main_worklist(s, c);
+    if (st == NB_ERR_OUT_OF_MEMORY && is_symmetric(c)) continue;  // no room for its rows
+    NB_TRY(st);
     s->cfg = c;
     NB_TRY(force_pass(s, s->acc_d, kPerSystemNone));  // warm-up
     NB_CUDA(cudaEventRecord(s->ev0, s->stream));
@@ -1040,6 +1193,7 @@ int nb_sim_autotune(nb_sim* s, int32_t* chosen) {
   }
   NB_TRY(build_main_worklist(s, best));
   s->cfg = best;
+  s->cfg_default = false;
   if (chosen) *chosen = best;
   return NB_OK;
 }
@@ -1050,7 +1204,7 @@ int nb_plan_work(uint32_t num_systems, const uint32_t* sizes, int32_t config_ind
                  int32_t* num_partial_slots) {
   static_assert(sizeof(nb_segment) == sizeof(Segment), "nb_segment mirrors Segment");
   if (num_systems == 0 || !sizes) return set_error(NB_ERR_INVALID_ARGUMENT, "no systems");
-  if (config_index < -reference_order_num_shapes() || config_index >= num_force_configs())
+  if (config_index < -reference_order_num_shapes() || config_index >= num_configs())
     return set_error(NB_ERR_INVALID_ARGUMENT, "bad config index");
   if (max_grid < 1) return set_error(NB_ERR_INVALID_ARGUMENT, "max_grid must be >= 1");
   std::vector<SystemDesc> sys(num_systems);
@@ -1064,8 +1218,32 @@ int nb_plan_work(uint32_t num_systems, const uint32_t* sizes, int32_t config_ind
     off += sys[k].npad;
   }
   const bool tuned = config_index >= 0;
-  const KernelShape sh =
-      tuned ? force_config_shape(config_index) : reference_order_shape(-1 - config_index);
+  const KernelShape sh = shape_of(config_index);
+  if (is_symmetric(config_index)) {
+    // One band: the list of a simulation whose rows fit the scratch.
+    const SymPlanHost h = plan_symmetric(sys.data(), 0, static_cast<int32_t>(num_systems), sh.bi(),
+                                         sh.bj, max_grid, INT64_MAX);
+    if (grid) *grid = h.bands[0].grid;
+    if (num_segments) *num_segments = static_cast<int32_t>(h.segs.size());
+    if (num_fixups) *num_fixups = h.split_tiles;
+    if (num_partial_slots) *num_partial_slots = h.slots;
+    if (segments) {
+      if (max_segments < static_cast<int32_t>(h.segs.size()))
+        return set_error(NB_ERR_INVALID_ARGUMENT, "segments buffer too small");
+      int32_t fix = 0;
+      for (const SymTile& t : h.tiles) {
+        for (int32_t p = 0; p < t.nslots; ++p) {
+          const SymSegment& sg = h.segs[t.slot0 + p];
+          segments[t.slot0 + p] = nb_segment{sg.sys, sg.itile, sg.jt0, sg.jt1,
+                                             t.nslots > 1 ? fix : -1, p};
+        }
+        if (t.nslots > 1) ++fix;
+      }
+    }
+    if (seg_begin)
+      std::memcpy(seg_begin, h.seg_begin.data(), h.seg_begin.size() * sizeof(int32_t));
+    return NB_OK;
+  }
   // The rule of every launch: the tuned kernel's live-slot variant where it pays.
   const bool live = tuned && live_slots_pay(sys.data(), 0, static_cast<int32_t>(num_systems),
                                             sh.threads, sh.r);
@@ -1106,7 +1284,11 @@ int nb_sim_set_shard(nb_sim* s, uint64_t first, uint64_t count) {
   d.shard_first = static_cast<int32_t>(first);
   d.shard_count = (first == 0 && count == n) ? 0 : static_cast<int32_t>(count);
   NB_TRY(upload_systems(s));
-  NB_TRY(build_main_worklist(s, s->cfg));
+  // The symmetric shapes need the whole system.
+  if (s->cfg_default || (sharded(s) && is_symmetric(s->cfg)))
+    NB_TRY(build_default_worklist(s));
+  else
+    NB_TRY(build_main_worklist(s, s->cfg));
   if (reference_order_mode(s)) NB_TRY(build_reference_order_worklist(s, s->ro_shape));
   for (auto& w : s->wl_sys) free_worklist(w);
   s->wl_sys.clear();
@@ -1231,6 +1413,10 @@ int nb_sim_inject_failure(nb_sim* s, int32_t kind) {
     return set_error(NB_ERR_STATE, "the failure hooks cover the BRANCH kernels only");
   if (kind == NB_INJECT_HAND_OVER_WITHHELD && !reference_order_mode(s))
     return set_error(NB_ERR_STATE, "hand-overs exist in NB_ACC_REFERENCE_ORDER only");
+  if (is_symmetric(s->cfg) && s->inject_wl.segs == nullptr) {
+    const int32_t nsys = static_cast<int32_t>(s->sys_h.size());
+    NB_TRY(plan_tuned(s, default_config_for(s, 0, nsys, false), 0, nsys, 0, &s->inject_wl));
+  }
   s->inject = kind == NB_INJECT_TILE_NEVER_COPIED ? kInjectSkipFirstTile : kInjectWithholdHandOver;
   return NB_OK;
 }

@@ -1,0 +1,90 @@
+// Work lists of the symmetric force kernel (symmetric_kernel.cuh) and their planner.
+//
+// The unit of work is one (system, i-tile, j-tile) block on or above the diagonal: an
+// i-tile I of bi particles meets the j-tiles from its own first particle to the end of
+// its system, so every unordered pair of particles in different i-tiles is in exactly
+// one block.  The j-tiles inside the i-tile (the diagonal block) are summed for the i
+// side only, over all ordered pairs; the others for both sides.
+//
+// Units are laid out in (system, i-tile, j-tile) order and charged their particles
+// times the pair loop's lane operations (kSymDiagCost, kSymPairCost), and cut into one
+// contiguous run per CTA of the same charge to within one unit, as in worklist.hpp.
+//
+// The j-side sums of i-tile I are one row of scratch, a value per component and
+// particle behind the tile; the rows of a system of n particles take about n^2 / (2 bi)
+// values.  Where all rows together pass the scratch's bound, the i-tiles are cut into
+// bands that are run (and their rows added up) one after another in the same scratch.
+#pragma once
+
+#include <cstdint>
+#include <vector>
+
+#include "nb_internal.hpp"
+
+namespace nbg {
+
+// Lane operations per pair on the FMA pipe (symmetric_kernel.cuh): one side, both sides.
+constexpr int kSymDiagCost = 11;
+constexpr int kSymPairCost = 14;
+constexpr int64_t kSymRowBytes = 3 * sizeof(float);  // scratch per row value
+constexpr int64_t kSymScratchBytes = int64_t{1} << 29;
+
+// One entry of a CTA's list: i-tile `itile` of system `sys` against j-tiles [jt0, jt1).
+// The j-side sum of particle j goes to value row + j of each plane of the row scratch,
+// the i-side sums to slot `slot` of the partial sums.
+struct SymSegment {
+  int32_t sys;
+  int32_t itile;
+  int32_t jt0;
+  int32_t jt1;
+  int64_t row;
+  int64_t offset;  // first particle of the system, and its particles
+  int32_t n;
+  int32_t slot;
+  int32_t next;    // the CTA's next segment, -1 for none; CTA k starts with segment k
+  int32_t pad_;
+};
+
+// One i-tile: its row, and its first slot (its slots run to the next i-tile's first).
+struct SymTile {
+  int64_t row;
+  int64_t offset;  // first particle of the system, and its particles
+  int32_t n;
+  int32_t sys;
+  int32_t itile;
+  int32_t slot0;
+  int32_t nslots;
+  int32_t pad_;
+};
+
+// A band of i-tiles [tile0, tile1): its work list and what the adding pass covers.
+struct SymBand {
+  int32_t tile0 = 0, tile1 = 0;
+  int32_t end = 0;       // one past the last i-tile of the last system it touches
+  int32_t grid = 0;
+  int32_t begin0 = 0;    // first of its grid + 1 entries of seg_begin
+  int32_t seg0 = 0;      // its first segment
+};
+
+struct SymPlanHost {
+  std::vector<SymSegment> segs;
+  std::vector<int32_t> seg_begin;
+  std::vector<SymTile> tiles;
+  std::vector<int32_t> sys_tile0;  // first i-tile of each planned system, by its index
+  std::vector<SymBand> bands;
+  int64_t row_values = 0;          // largest band's row values (per plane)
+  int32_t slots = 0;               // largest band's slots
+  int32_t split_tiles = 0;
+};
+
+// The segments in the order the kernel wants them: per band, the first of every CTA and
+// then the others, linked by `next` (relative to the band's seg0).
+std::vector<SymSegment> link_segments(const SymPlanHost& plan);
+
+// Plan systems [first, first + count) (whole systems, no shards) for i-tiles of bi and
+// j-tiles of bj particles (bi % bj == 0) on at most max_grid CTAs, with at most
+// max_row_values row values per band (one i-tile at least).
+SymPlanHost plan_symmetric(const SystemDesc* sys, int32_t first, int32_t count, int32_t bi,
+                           int32_t bj, int32_t max_grid, int64_t max_row_values);
+
+}  // namespace nbg
