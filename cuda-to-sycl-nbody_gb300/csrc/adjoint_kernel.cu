@@ -10,195 +10,263 @@
 // symmetric in i and j,
 //   (J^T mu)_i = sum_{j != i} K_ij u_ij,  u_ij = m_i mu_j - m_j mu_i
 //              = sum_{j != i} s_ij (u_ij + c_ij r_ij),  c_ij = -3 (r_ij . u_ij) / (r^2 + eps).
-// Per pair that is 22 FP32 lane operations and one MUFU rsqrt (equal masses: u = mu_j - mu_i
-// and the common mass goes into the final scale), on the packed FP32x2 pipe, with three
-// accumulators per i-particle.
+// u_ji = -u_ij, so K_ij u_ij is the term of both particles, with opposite signs, and an
+// unordered pair is evaluated once.
 //
-// Work decomposition: one CTA per (i-tile, j-chunk); each writes its partial sum per
-// i-particle, and a second kernel adds the chunks in order (deterministic) and applies
-// lx = lx' + dt G (J^T mu).
+// What bounds it: the FP32 FMA pipe.  A pair is 25 lane operations for both sides (22
+// for one, the diagonal block's) and one MUFU rsqrt; equal masses: u = mu_j - mu_i, and
+// the common mass goes into the final scale.  A backward step (this product; every
+// ordered pair evaluated before) takes 131 us at N = 16,384 (207 before), 143 with
+// per-particle masses (232), 28.7 at 4,690 (47.2), 1,730 at 65,536 (3,454).
+//
+// The tiling is that of the symmetric force kernel (symmetric_kernel.cuh) with one warp
+// per CTA: a warp's 32 j-particles, with their cotangents and running sums, rotate
+// through its lanes past 64 P i-particles held two per packed register pair; the j-side
+// sums go to rows of scratch, and adjoint_add_kernel adds a particle's rows and i-side
+// parts in order and applies lx = lx' + dt G (J^T mu), lv = d mu.  Lanes past the end of
+// a system hold zeros and are masked by index, as j-particles: as i-particles they are
+// in a system's last i-tile, whose blocks are all diagonal.
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
+#include "nb_device.cuh"
 #include "nb_internal.hpp"
 #include "nb_kernels.hpp"
+#include "symmetric.hpp"
+#include "symmetric_add.cuh"
 
 namespace nbg {
 namespace {
 
-constexpr int kAdjThreads = 128;
-constexpr int kAdjR = 4;                      // i-particles per thread
-constexpr int kAdjBI = kAdjThreads * kAdjR;   // i-particles per CTA
-constexpr int kAdjBJ = 256;                   // j-particles per shared tile
+constexpr int kAdjBJ = 32;     // j-particles a warp rotates at a time
+constexpr int kAdjFold = 512;  // j-particles between two folds of the i-side sums
 
-__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
-
-// Pairs [0, npairs) of one shared tile.  kMask: zero the rsqrt of the self pair and
-// of j >= jn (a padding lane at the end of the system).
-template <bool kMass, bool kMask>
-__device__ __forceinline__ void adj_tile(const float4 (*tile)[4], int npairs, float2 e2,
-                                         const float2 (&nx)[kAdjR], const float2 (&ny)[kAdjR],
-                                         const float2 (&nz)[kAdjR], const float2 (&wx)[kAdjR],
-                                         const float2 (&wy)[kAdjR], const float2 (&wz)[kAdjR],
-                                         const float2 (&mi)[kAdjR], float2 (&gx)[kAdjR],
-                                         float2 (&gy)[kAdjR], float2 (&gz)[kAdjR], int j_base,
-                                         int jn, const int (&li)[kAdjR]) {
-  const float2 m3c = f2(-3.f, -3.f);
-#pragma unroll 2
-  for (int p = 0; p < npairs; ++p) {
-    const float4 P0 = tile[p][0], P1 = tile[p][1], M0 = tile[p][2], M1 = tile[p][3];
-#pragma unroll
-    for (int r = 0; r < kAdjR; ++r) {
-      const float2 dx = __fadd2_rn(f2(P0.x, P0.y), nx[r]);
-      const float2 dy = __fadd2_rn(f2(P0.z, P0.w), ny[r]);
-      const float2 dz = __fadd2_rn(f2(P1.x, P1.y), nz[r]);
-      float2 ux, uy, uz;
-      if (kMass) {
-        const float2 mj = f2(P1.z, P1.w);
-        ux = __ffma2_rn(mj, wx[r], __fmul2_rn(mi[r], f2(M0.x, M0.y)));
-        uy = __ffma2_rn(mj, wy[r], __fmul2_rn(mi[r], f2(M0.z, M0.w)));
-        uz = __ffma2_rn(mj, wz[r], __fmul2_rn(mi[r], f2(M1.x, M1.y)));
-      } else {
-        ux = __fadd2_rn(f2(M0.x, M0.y), wx[r]);
-        uy = __fadd2_rn(f2(M0.z, M0.w), wy[r]);
-        uz = __fadd2_rn(f2(M1.x, M1.y), wz[r]);
-      }
-      float2 d2 = __ffma2_rn(dx, dx, e2);
-      d2 = __ffma2_rn(dy, dy, d2);
-      d2 = __ffma2_rn(dz, dz, d2);
-      float2 inv = f2(rsqrtf(d2.x), rsqrtf(d2.y));
-      if (kMask) {
-        const int j = j_base + 2 * p;
-        if (j == li[r] || j >= jn) inv.x = 0.f;
-        if (j + 1 == li[r] || j + 1 >= jn) inv.y = 0.f;
-      }
-      const float2 inv2 = __fmul2_rn(inv, inv);
-      const float2 s = __fmul2_rn(inv2, inv);
-      const float2 m3 = __fmul2_rn(inv2, m3c);
-      float2 rw = __fmul2_rn(dx, ux);
-      rw = __ffma2_rn(dy, uy, rw);
-      rw = __ffma2_rn(dz, uz, rw);
-      const float2 c = __fmul2_rn(rw, m3);
-      gx[r] = __ffma2_rn(s, __ffma2_rn(c, dx, ux), gx[r]);
-      gy[r] = __ffma2_rn(s, __ffma2_rn(c, dy, uy), gy[r]);
-      gz[r] = __ffma2_rn(s, __ffma2_rn(c, dz, uz), gz[r]);
-    }
-  }
+__device__ __forceinline__ float adj_rot(float v, int src) {
+  return __shfl_sync(0xffffffffu, v, src);
 }
 
-template <bool kMass>
-__global__ void __launch_bounds__(kAdjThreads) adjoint_partial_kernel(const AdjointArgs a) {
-  // Tile of j-pairs: { x0 x1 y0 y1 } { z0 z1 m0 m1 } { mx0 mx1 my0 my1 } { mz0 mz1 0 0 }
-  __shared__ __align__(16) float4 tile[kAdjBJ / 2][4];
-  const SystemDesc sd = a.sys[a.tile_sys[blockIdx.x]];
-  const int ibase = a.tile_idx[blockIdx.x] * kAdjBI;
-  const int split = blockIdx.y;
-  const int chunk = ((sd.n + a.num_splits - 1) / a.num_splits + 1) & ~1;
-  const int j_lo = split * chunk;
-  const int j_hi = min(sd.n, j_lo + chunk);
-  const int tid = threadIdx.x;
+template <int P>
+struct AdjI {
+  float2 nx[P], ny[P], nz[P];  // minus the positions
+  float2 wx[P], wy[P], wz[P];  // minus mu
+  float2 m[P];
+  float2 gx[P], gy[P], gz[P];  // sums since the last fold
+};
 
-  float2 nx[kAdjR], ny[kAdjR], nz[kAdjR], wx[kAdjR], wy[kAdjR], wz[kAdjR], mi[kAdjR];
-  float2 gx[kAdjR], gy[kAdjR], gz[kAdjR];
-  int li[kAdjR];
+struct AdjJ {
+  float x, y, z, m, ux, uy, uz;  // position, mass, mu
+};
+
+// 32 rotations of the warp's j-particles against its i-particles.  kPair: both sides
+// (out: the j side's sums of the i side's terms); kMask: leave out j == i and j >= n.
+template <int P, int U, bool kMass, bool kPair, bool kMask>
+__device__ __forceinline__ void adj_chunk(AdjI<P>& q, AdjJ v, float2 e2, float (&out)[3], int jj,
+                                          int li0, int n) {
+  const int src = (threadIdx.x + 1) & 31;
+  const float2 m3c = make_float2(-3.f, -3.f);
+  float2 fx = make_float2(0.f, 0.f), fy = fx, fz = fx;
+#pragma unroll 1
+  for (int k = 0; k < kAdjBJ; k += U) {
 #pragma unroll
-  for (int r = 0; r < kAdjR; ++r) {
-    li[r] = ibase + r * kAdjThreads + tid;
-    const int64_t g = sd.offset + (li[r] < sd.n ? li[r] : sd.n - 1);
-    const float x = a.pos[pair_index(g, 0)], y = a.pos[pair_index(g, 1)],
-                z = a.pos[pair_index(g, 2)], m = a.pos[pair_index(g, 3)];
-    const float4 lx = a.lam_x[g], lv = a.lam_v[g];  // mu = lv' + dt lx'
-    const float4 mu = make_float4(fmaf(a.dt, lx.x, lv.x), fmaf(a.dt, lx.y, lv.y),
-                                  fmaf(a.dt, lx.z, lv.z), 0.f);
-    nx[r] = f2(-x, -x);
-    ny[r] = f2(-y, -y);
-    nz[r] = f2(-z, -z);
-    wx[r] = f2(-mu.x, -mu.x);
-    wy[r] = f2(-mu.y, -mu.y);
-    wz[r] = f2(-mu.z, -mu.z);
-    mi[r] = f2(m, m);
-    gx[r] = gy[r] = gz[r] = f2(0.f, 0.f);
+    for (int u = 0; u < U; ++u) {
+      const float2 xx = make_float2(v.x, v.x), yy = make_float2(v.y, v.y),
+                   zz = make_float2(v.z, v.z), mm = make_float2(v.m, v.m);
+      const float2 jx = make_float2(v.ux, v.ux), jy = make_float2(v.uy, v.uy),
+                   jz = make_float2(v.uz, v.uz);
+#pragma unroll
+      for (int r = 0; r < P; ++r) {
+        const float2 dx = __fadd2_rn(xx, q.nx[r]);
+        const float2 dy = __fadd2_rn(yy, q.ny[r]);
+        const float2 dz = __fadd2_rn(zz, q.nz[r]);
+        float2 ux, uy, uz;
+        if (kMass) {
+          ux = __ffma2_rn(mm, q.wx[r], __fmul2_rn(q.m[r], jx));
+          uy = __ffma2_rn(mm, q.wy[r], __fmul2_rn(q.m[r], jy));
+          uz = __ffma2_rn(mm, q.wz[r], __fmul2_rn(q.m[r], jz));
+        } else {
+          ux = __fadd2_rn(jx, q.wx[r]);
+          uy = __fadd2_rn(jy, q.wy[r]);
+          uz = __fadd2_rn(jz, q.wz[r]);
+        }
+        float2 d2 = __ffma2_rn(dx, dx, e2);
+        d2 = __ffma2_rn(dy, dy, d2);
+        d2 = __ffma2_rn(dz, dz, d2);
+        float2 inv = make_float2(rsqrtf(d2.x), rsqrtf(d2.y));
+        if (kMask) {
+          if (jj == li0 + 64 * r || jj >= n) inv.x = 0.f;
+          if (jj == li0 + 64 * r + 32 || jj >= n) inv.y = 0.f;
+        }
+        const float2 inv2 = __fmul2_rn(inv, inv);
+        const float2 s = __fmul2_rn(inv2, inv);
+        const float2 m3 = __fmul2_rn(inv2, m3c);
+        float2 rw = __fmul2_rn(dx, ux);
+        rw = __ffma2_rn(dy, uy, rw);
+        rw = __ffma2_rn(dz, uz, rw);
+        const float2 c = __fmul2_rn(rw, m3);
+        const float2 tx = __ffma2_rn(c, dx, ux);
+        const float2 ty = __ffma2_rn(c, dy, uy);
+        const float2 tz = __ffma2_rn(c, dz, uz);
+        q.gx[r] = __ffma2_rn(s, tx, q.gx[r]);
+        q.gy[r] = __ffma2_rn(s, ty, q.gy[r]);
+        q.gz[r] = __ffma2_rn(s, tz, q.gz[r]);
+        if (kPair) {
+          fx = __ffma2_rn(s, tx, fx);
+          fy = __ffma2_rn(s, ty, fy);
+          fz = __ffma2_rn(s, tz, fz);
+        }
+      }
+      v.x = adj_rot(v.x, src);
+      v.y = adj_rot(v.y, src);
+      v.z = adj_rot(v.z, src);
+      if (kMass) v.m = adj_rot(v.m, src);
+      v.ux = adj_rot(v.ux, src);
+      v.uy = adj_rot(v.uy, src);
+      v.uz = adj_rot(v.uz, src);
+      if (kMask) jj = __shfl_sync(0xffffffffu, jj, src);
+      if (kPair) {
+        fx.x = adj_rot(fx.x, src);
+        fx.y = adj_rot(fx.y, src);
+        fy.x = adj_rot(fy.x, src);
+        fy.y = adj_rot(fy.y, src);
+        fz.x = adj_rot(fz.x, src);
+        fz.y = adj_rot(fz.y, src);
+      }
+    }
   }
-  const float2 e2 = f2(a.eps2, a.eps2);
+  out[0] = fx.x + fx.y;
+  out[1] = fy.x + fy.y;
+  out[2] = fz.x + fz.y;
+}
 
-  for (int j0 = j_lo; j0 < j_hi; j0 += kAdjBJ) {
-    const int cnt = min(kAdjBJ, j_hi - j0);
-    __syncthreads();
-    for (int p = tid; p < kAdjBJ / 2; p += kAdjThreads) {
+// mu = lv' + dt lx' of particle g.
+__device__ __forceinline__ float3 adj_mu(const AdjointArgs& a, int64_t g) {
+  const float4 lx = a.lam_x[g], lv = a.lam_v[g];
+  return make_float3(fmaf(a.dt, lx.x, lv.x), fmaf(a.dt, lx.y, lv.y), fmaf(a.dt, lx.z, lv.z));
+}
+
+template <int P, int U, bool kMass>
+__global__ void __launch_bounds__(32, 8) adjoint_pair_kernel(const AdjointArgs a) {
+  constexpr int BI = 64 * P;
+  __shared__ float2 sums[3 * P][32];
+  const int lane = threadIdx.x;
+  const float2 e2 = make_float2(a.eps2, a.eps2);
+  const float2 zero = make_float2(0.f, 0.f);
+  pdl_trigger();
+  SymSegment sg = a.segs[blockIdx.x];
+  pdl_wait();
+  for (int next = blockIdx.x; next >= 0;) {
+    if (next != static_cast<int>(blockIdx.x)) sg = a.segs[next];
+    next = sg.next;
+    const int ibase = sg.itile * BI;
+    const float* pos = a.pos + 4 * sg.offset;
+    AdjI<P> q;
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
       float v[2][7];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int lj = j0 + 2 * p + h;
-        if (2 * p + h < cnt) {
-          const int64_t gj = sd.offset + lj;
-          const float4 lx = a.lam_x[gj], lv = a.lam_v[gj];
-          const float4 mu = make_float4(fmaf(a.dt, lx.x, lv.x), fmaf(a.dt, lx.y, lv.y),
-                                        fmaf(a.dt, lx.z, lv.z), 0.f);
-          v[h][0] = a.pos[pair_index(gj, 0)];
-          v[h][1] = a.pos[pair_index(gj, 1)];
-          v[h][2] = a.pos[pair_index(gj, 2)];
-          v[h][3] = a.pos[pair_index(gj, 3)];
-          v[h][4] = mu.x;
-          v[h][5] = mu.y;
-          v[h][6] = mu.z;
-        } else {
-          // past the chunk: at the origin with zero mass and cotangent (masked below)
-          v[h][0] = v[h][1] = v[h][2] = v[h][3] = v[h][4] = v[h][5] = v[h][6] = 0.f;
-        }
-      }
-      tile[p][0] = make_float4(v[0][0], v[1][0], v[0][1], v[1][1]);
-      tile[p][1] = make_float4(v[0][2], v[1][2], v[0][3], v[1][3]);
-      tile[p][2] = make_float4(v[0][4], v[1][4], v[0][5], v[1][5]);
-      tile[p][3] = make_float4(v[0][6], v[1][6], 0.f, 0.f);
-    }
-    __syncthreads();
-    const int npairs = (cnt + 1) / 2;
-    const bool diag = a.mask_self && (j0 < ibase + kAdjBI) && (ibase < j0 + cnt);
-    if (diag || (cnt & 1)) {
-      adj_tile<kMass, true>(tile, npairs, e2, nx, ny, nz, wx, wy, wz, mi, gx, gy, gz, j0,
-                            j0 + cnt, li);
-    } else {
-      adj_tile<kMass, false>(tile, npairs, e2, nx, ny, nz, wx, wy, wz, mi, gx, gy, gz, j0,
-                             j0 + cnt, li);
-    }
-  }
-
-  float4* part = a.partial + static_cast<int64_t>(split) * a.n_pad;
+        const int li = min(ibase + 64 * r + 32 * h + lane, sg.n - 1);
+        const float3 mu = adj_mu(a, sg.offset + li);
 #pragma unroll
-  for (int r = 0; r < kAdjR; ++r) {
-    if (li[r] >= sd.n) continue;
-    part[sd.offset + li[r]] =
-        make_float4(gx[r].x + gx[r].y, gy[r].x + gy[r].y, gz[r].x + gz[r].y, 0.f);
+        for (int c = 0; c < 4; ++c) v[h][c] = pos[pair_index(li, c)];
+        v[h][4] = mu.x, v[h][5] = mu.y, v[h][6] = mu.z;
+      }
+      q.nx[r] = make_float2(-v[0][0], -v[1][0]);
+      q.ny[r] = make_float2(-v[0][1], -v[1][1]);
+      q.nz[r] = make_float2(-v[0][2], -v[1][2]);
+      q.m[r] = make_float2(v[0][3], v[1][3]);
+      q.wx[r] = make_float2(-v[0][4], -v[1][4]);
+      q.wy[r] = make_float2(-v[0][5], -v[1][5]);
+      q.wz[r] = make_float2(-v[0][6], -v[1][6]);
+      q.gx[r] = q.gy[r] = q.gz[r] = zero;
+    }
+
+    AdjJ nj;  // the lane's j-particle of the next chunk, loaded one chunk ahead
+    auto fetch = [&](int jt) {
+      const int j = jt * kAdjBJ + lane;
+      nj = AdjJ{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (jt < sg.jt1 && j < sg.n) {
+        const float3 mu = adj_mu(a, sg.offset + j);
+        nj.x = pos[pair_index(j, 0)];
+        nj.y = pos[pair_index(j, 1)];
+        nj.z = pos[pair_index(j, 2)];
+        if (kMass) nj.m = pos[pair_index(j, 3)];
+        nj.ux = mu.x, nj.uy = mu.y, nj.uz = mu.z;
+      }
+    };
+    fetch(sg.jt0);
+    bool folded = false;
+    for (int jt = sg.jt0; jt < sg.jt1; ++jt) {
+      const AdjJ v = nj;
+      const int j0 = jt * kAdjBJ, j = j0 + lane;
+      fetch(jt + 1);
+      const bool diag = j0 < ibase + BI;
+      const bool ragged = j0 + kAdjBJ > sg.n;
+      float out[3];
+      if (!diag) {
+        if (ragged)
+          adj_chunk<P, 1, kMass, true, true>(q, v, e2, out, j, -BI, sg.n);
+        else
+          adj_chunk<P, U, kMass, true, false>(q, v, e2, out, j, 0, sg.n);
+        if (j < sg.n) {
+          a.rows[sg.row + j] = out[0];
+          a.rows[a.plane + sg.row + j] = out[1];
+          a.rows[2 * a.plane + sg.row + j] = out[2];
+        }
+      } else if (ragged || a.mask_self) {
+        adj_chunk<P, 1, kMass, false, true>(q, v, e2, out, j,
+                                            a.mask_self ? ibase + lane : -BI, sg.n);
+      } else {
+        adj_chunk<P, U, kMass, false, false>(q, v, e2, out, j, 0, sg.n);
+      }
+      if (jt + 1 == sg.jt1 ? folded : (jt + 1 - sg.jt0) % (kAdjFold / kAdjBJ) == 0) {
+#pragma unroll
+        for (int r = 0; r < P; ++r) {
+          sums[r][lane] = folded ? __fadd2_rn(sums[r][lane], q.gx[r]) : q.gx[r];
+          sums[P + r][lane] = folded ? __fadd2_rn(sums[P + r][lane], q.gy[r]) : q.gy[r];
+          sums[2 * P + r][lane] = folded ? __fadd2_rn(sums[2 * P + r][lane], q.gz[r]) : q.gz[r];
+          q.gx[r] = q.gy[r] = q.gz[r] = zero;
+        }
+        folded = true;
+      }
+    }
+    float4* part = a.partials + static_cast<int64_t>(sg.slot) * BI;
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+      const float2 sx = folded ? sums[r][lane] : q.gx[r];
+      const float2 sy = folded ? sums[P + r][lane] : q.gy[r];
+      const float2 sz = folded ? sums[2 * P + r][lane] : q.gz[r];
+      part[64 * r + lane] = make_float4(sx.x, sy.x, sz.x, 0.f);
+      part[64 * r + 32 + lane] = make_float4(sx.y, sy.y, sz.y, 0.f);
+    }
   }
 }
 
-// lx = lx' + dt * gscale * sum over chunks (in chunk order) and lv = damping * mu,
-// real particles only.  One thread per particle, kCombineThreads particles of an
-// i-tile per CTA (blockIdx.y picks them); the chunk loop is unrolled so that several
-// of its loads are in flight (the additions keep their order).
-constexpr int kCombineThreads = 128;
-static_assert(kAdjBI % kCombineThreads == 0, "whole i-tiles");
-
-__global__ void __launch_bounds__(kCombineThreads) adjoint_combine_kernel(const AdjointArgs a) {
-  const SystemDesc sd = a.sys[a.tile_sys[blockIdx.x]];
-  const int ibase = a.tile_idx[blockIdx.x] * kAdjBI;
-  const float c = a.dt * sd.gscale;
-  const int li = ibase + blockIdx.y * kCombineThreads + threadIdx.x;
-  if (li >= sd.n) return;
-  const int64_t g = sd.offset + li;
-  float sx = 0.f, sy = 0.f, sz = 0.f;
-#pragma unroll 8
-  for (int s = 0; s < a.num_splits; ++s) {
-    const float4 p = a.partial[static_cast<int64_t>(s) * a.n_pad + g];
-    sx += p.x;
-    sy += p.y;
-    sz += p.z;
+struct EarlyAdjoint {
+  const AdjointArgs& a;
+  float gscale;
+  float4 lx, lv;
+  __device__ void lists(int sys) { gscale = a.sys[sys].gscale; }
+  __device__ void state(int64_t g) {
+    lx = a.lam_x[g];
+    lv = a.lam_v[g];
   }
-  const float4 l = a.lam_x[g], v = a.lam_v[g];
-  a.lam_x_out[g] = make_float4(fmaf(c, sx, l.x), fmaf(c, sy, l.y), fmaf(c, sz, l.z), 0.f);
-  a.lam_v_out[g] = make_float4(a.damping * fmaf(a.dt, l.x, v.x), a.damping * fmaf(a.dt, l.y, v.y),
-                               a.damping * fmaf(a.dt, l.z, v.z), 0.f);
+};
+
+template <int kLanes, int kGroups>
+__global__ void __launch_bounds__(kLanes * kGroups) adjoint_add_kernel(const AdjointArgs a,
+                                                                       int bi) {
+  const AddTerms t{a.tiles, a.rows, a.plane, a.carry, a.partials, a.tile0, a.tile1};
+  EarlyAdjoint e{a, 0.f, {}, {}};
+  AddResult r;
+  if (!add_terms<kLanes, kGroups, false>(t, bi, e, r)) return;
+  const float c = a.dt * e.gscale;
+  const float4 l = e.lx, v = e.lv;
+  a.lam_x_out[r.g] = make_float4(fmaf(c, r.x, l.x), fmaf(c, r.y, l.y), fmaf(c, r.z, l.z), 0.f);
+  a.lam_v_out[r.g] =
+      make_float4(a.damping * fmaf(a.dt, l.x, v.x), a.damping * fmaf(a.dt, l.y, v.y),
+                  a.damping * fmaf(a.dt, l.z, v.z), 0.f);
 }
 
 __global__ void unpack_vec3_kernel(const float* __restrict__ in, int64_t n,
@@ -227,30 +295,36 @@ int grid_for(int64_t n) {
   return static_cast<int>(b < 1 ? 1 : (b > 1 << 20 ? 1 << 20 : b));
 }
 
+struct AdjEntry {
+  int pairs;
+  void (*kernel[2])(const AdjointArgs);  // [per-particle masses]
+};
+#define NBG_ADJ(P, U) {P, {adjoint_pair_kernel<P, U, false>, adjoint_pair_kernel<P, U, true>}}
+const AdjEntry kAdjShapes[] = {NBG_ADJ(6, 1), NBG_ADJ(4, 2), NBG_ADJ(1, 4)};
+
 }  // namespace
 
-int adjoint_tile() { return kAdjBI; }
+int num_adjoint_shapes() { return static_cast<int>(sizeof(kAdjShapes) / sizeof(kAdjShapes[0])); }
 
-cudaError_t adjoint_blocks_per_sm(bool per_pair_mass, int* blocks) {
-  return per_pair_mass
-             ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, adjoint_partial_kernel<true>,
-                                                             kAdjThreads, 0)
-             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, adjoint_partial_kernel<false>,
-                                                             kAdjThreads, 0);
+KernelShape adjoint_shape(int index) {
+  return KernelShape{32, 2 * kAdjShapes[index].pairs, kAdjBJ, 0};
 }
 
-cudaError_t launch_adjoint(const AdjointArgs& a, int32_t num_tiles, bool per_pair_mass,
+cudaError_t adjoint_blocks_per_sm(int index, bool per_pair_mass, int* blocks) {
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      blocks, kAdjShapes[index].kernel[per_pair_mass], 32, 0);
+}
+
+cudaError_t launch_adjoint(int index, bool per_pair_mass, const AdjointArgs& a, int grid,
                            cudaStream_t stream) {
-  const dim3 grid(num_tiles, a.num_splits);
-  if (per_pair_mass)
-    adjoint_partial_kernel<true><<<grid, kAdjThreads, 0, stream>>>(a);
-  else
-    adjoint_partial_kernel<false><<<grid, kAdjThreads, 0, stream>>>(a);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  adjoint_combine_kernel<<<dim3(num_tiles, kAdjBI / kCombineThreads), kCombineThreads, 0,
-                           stream>>>(a);
-  return cudaGetLastError();
+  return launch_dependent(kAdjShapes[index].kernel[per_pair_mass], dim3(grid), 32, 0, stream, a);
+}
+
+cudaError_t launch_adjoint_add(const AdjointArgs& a, int tiles, int bi, cudaStream_t stream) {
+  if (static_cast<int64_t>(tiles) * bi < kManyParticles)
+    return launch_dependent(adjoint_add_kernel<32, 8>, add_grid<32>(tiles, bi), 256, 0, stream, a,
+                            bi);
+  return launch_dependent(adjoint_add_kernel<64, 2>, add_grid<64>(tiles, bi), 128, 0, stream, a, bi);
 }
 
 cudaError_t launch_unpack_vec3(const float* in, int64_t n, const int64_t* map, float4* out,

@@ -105,20 +105,25 @@ struct AdjointArgs {
   float4* lam_x_out;      // [n_pad] lam_x = lam_x' + dt * G * J^T mu, mu = lam_v' + dt lam_x'
   float4* lam_v_out;      // [n_pad] lam_v = damping * mu
   const SystemDesc* sys;
-  const int32_t* tile_sys;  // [tiles] system of each i-tile
-  const int32_t* tile_idx;  // [tiles] i-tile index within its system
-  float4* partial;          // [num_splits][n_pad] per-chunk partial sums
-  int64_t n_pad;
-  int32_t num_splits;       // j-chunks per i-tile
+  const SymSegment* segs;  // work list, i-tiles, row scratch and parts: as in SymArgs
+  const SymTile* tiles;
+  float* rows;
+  int64_t plane;
+  float4* carry;
+  float4* partials;
+  int32_t tile0, tile1;
   float eps2;
   float dt;
   float damping;
   int32_t mask_self;
 };
-cudaError_t launch_adjoint(const AdjointArgs& a, int32_t num_tiles, bool per_pair_mass,
+int num_adjoint_shapes();
+KernelShape adjoint_shape(int index);  // threads, i-particles per thread, j-tile, 0 stages
+cudaError_t adjoint_blocks_per_sm(int index, bool per_pair_mass, int* blocks);
+cudaError_t launch_adjoint(int index, bool per_pair_mass, const AdjointArgs& a, int grid,
                            cudaStream_t stream);
-int adjoint_tile();  // i-particles per adjoint CTA
-cudaError_t adjoint_blocks_per_sm(bool per_pair_mass, int* blocks);
+// Add the rows and parts of the band's i-tiles and write lam_x_out and lam_v_out.
+cudaError_t launch_adjoint_add(const AdjointArgs& a, int tiles, int bi, cudaStream_t stream);
 // n x 3 interleaved (user order) <-> padded float4.
 cudaError_t launch_unpack_vec3(const float* in, int64_t n, const int64_t* map, float4* out,
                                cudaStream_t stream);

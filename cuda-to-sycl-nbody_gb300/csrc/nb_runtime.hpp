@@ -52,11 +52,8 @@ struct AdjointState {
   float4* mu = nullptr;
   float4* tmp = nullptr;
   float4* vel = nullptr;            // velocities of the recomputed segment
-  int32_t* tile_sys = nullptr;
-  int32_t* tile_idx = nullptr;
-  int32_t num_tiles = 0;
-  int32_t num_splits = 1;
-  float4* partial = nullptr;        // [num_splits][n_pad]
+  int shape = 0;                    // of the pair kernel
+  WorkListDev wl;                   // its list (the scratch is the simulation's)
   bool valid = false;
 };
 
@@ -115,6 +112,7 @@ struct nb_sim {
   cudaGraph_t graph[2] = {nullptr, nullptr};        // indexed by starting buffer
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
   int32_t graph_iters = 0;
+  std::vector<void*> retired;  // outgrown scratch whose address the graphs still hold
 
   nbg::DiagScratch diag{};
   double* diag_out_d = nullptr;
@@ -192,6 +190,9 @@ int force_pass(nb_sim* s, float4* accel_out, int per_system);
 int check_error_word(nb_sim* s);
 int ensure_staging(nb_sim* s);
 int ensure_accel(nb_sim* s);
+// Upload a symmetric plan for i-tiles of bi particles and make its scratch: rows, and
+// `rec` float4 records per slot and i-particle.
+int upload_symmetric(nb_sim* s, const SymPlanHost& h, int bi, int rec, WorkListDev* out);
 // Launch the force kernel with arguments `a` over work list `w`.
 int launch_with(nb_sim* s, ForceArgs a, const WorkListDev& w);
 

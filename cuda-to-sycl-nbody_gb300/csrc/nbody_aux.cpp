@@ -27,15 +27,35 @@ void release_aux(nb_sim* s) {
   dev_free(a.mu);
   dev_free(a.tmp);
   dev_free(a.vel);
-  dev_free(a.tile_sys);
-  dev_free(a.tile_idx);
-  dev_free(a.partial);
+  free_worklist(a.wl);
   a = AdjointState{};
 }
 
 }  // namespace nbg
 
 namespace {
+
+// The pair kernel's shape, and its largest grid.  The shapes' rates are measured at
+// N = 65,536 (1.73, 1.83 and 2.30 ms per backward step); the blocks per CTA, where two
+// neighbouring shapes meet (us per backward step with the larger / the smaller
+// i-tiles): 16,384 133 / 131 and 65,536 1,730 / 1,830 for 768 against 256 particles;
+// 4,690 30.6 / 28.7 and 16,384 131 / 159 for 256 against 64.
+int adjoint_shape_for(const nb_sim* s, int* grid) {
+  static constexpr double kRates[][2] = {{1.0, 6.0}, {0.945, 1.7}, {0.751, 0.0}};
+  constexpr int kCount = sizeof(kRates) / sizeof(kRates[0]);
+  SymCandidate c[kCount];
+  for (int k = 0; k < kCount; ++k) {
+    int per_sm = 0;
+    if (adjoint_blocks_per_sm(k, s->per_pair_mass, &per_sm) != cudaSuccess || per_sm < 1)
+      per_sm = 1;
+    c[k] = SymCandidate{adjoint_shape(k), kRates[k][0], kRates[k][1], per_sm * s->sms};
+  }
+  const int shape =
+      choose_symmetric(s->sys_h.data(), 0, static_cast<int32_t>(s->sys_h.size()), c, kCount,
+                       kAdjDiagCost, kAdjPairCost);
+  *grid = c[shape].max_grid;
+  return shape;
+}
 
 int ensure_adjoint_buffers(nb_sim* s, int32_t ncp, int32_t every) {
   AdjointState& a = s->adj;
@@ -63,28 +83,14 @@ int ensure_adjoint_buffers(nb_sim* s, int32_t ncp, int32_t every) {
     NB_TRY(dev_alloc(&a.mu, np));
     NB_TRY(dev_alloc(&a.tmp, np));
   }
-  if (!a.tile_sys) {
-    std::vector<int32_t> ts, ti;
-    const int bi = adjoint_tile();
-    for (int32_t k = 0; k < static_cast<int32_t>(s->sys_h.size()); ++k)
-      for (int32_t t = 0; t < (s->sys_h[k].n + bi - 1) / bi; ++t) {
-        ts.push_back(k);
-        ti.push_back(t);
-      }
-    a.num_tiles = static_cast<int32_t>(ts.size());
-    // j-chunks per i-tile: one full wave of resident CTAs (i-tiles x chunks = SMs x
-    // resident CTAs per SM, rounded up), the chunk sums reduced in order afterwards.
-    int per_sm = 1;
-    if (adjoint_blocks_per_sm(s->per_pair_mass, &per_sm) != cudaSuccess || per_sm < 1) per_sm = 1;
-    const int32_t target = per_sm * s->sms;
-    a.num_splits = std::max(1, std::min(64, (target + a.num_tiles - 1) / a.num_tiles));
-    NB_TRY(dev_alloc(&a.partial, static_cast<size_t>(a.num_splits) * np));
-    NB_TRY(dev_alloc(&a.tile_sys, ts.size()));
-    NB_TRY(dev_alloc(&a.tile_idx, ti.size()));
-    NB_CUDA(cudaMemcpy(a.tile_sys, ts.data(), ts.size() * sizeof(int32_t),
-                       cudaMemcpyHostToDevice));
-    NB_CUDA(cudaMemcpy(a.tile_idx, ti.data(), ti.size() * sizeof(int32_t),
-                       cudaMemcpyHostToDevice));
+  if (a.wl.bands.empty()) {
+    int grid = 0;
+    a.shape = adjoint_shape_for(s, &grid);
+    const KernelShape sh = adjoint_shape(a.shape);
+    const SymPlanHost h =
+        plan_symmetric(s->sys_h.data(), 0, static_cast<int32_t>(s->sys_h.size()), sh.bi(), sh.bj,
+                       grid, kSymScratchBytes / kSymRowBytes, kAdjDiagCost, kAdjPairCost);
+    NB_TRY(upload_symmetric(s, h, sh.bi(), 1, &a.wl));
   }
   return NB_OK;
 }
@@ -240,16 +246,22 @@ static int adjoint_backward_stream(nb_sim* s, const float* gx_T, const float* gv
       aa.lam_x_out = a.tmp;
       aa.lam_v_out = a.mu;  // second buffer pair: (tmp, mu) <- (lam_x, lam_v)
       aa.sys = s->sys_d;
-      aa.tile_sys = a.tile_sys;
-      aa.tile_idx = a.tile_idx;
-      aa.partial = a.partial;
-      aa.n_pad = s->n_pad;
-      aa.num_splits = a.num_splits;
+      aa.tiles = a.wl.sym_tiles;
+      aa.rows = s->rows_d;
+      aa.plane = a.wl.row_values;
+      aa.carry = s->carry_d;
+      aa.partials = s->partials_d;
       aa.eps2 = s->params.dist_eps;
       aa.dt = dt;
       aa.damping = s->params.damping;
       aa.mask_self = s->mask_self;
-      NB_CUDA(launch_adjoint(aa, a.num_tiles, s->per_pair_mass, s->stream));
+      for (const SymBand& b : a.wl.bands) {
+        aa.segs = a.wl.sym_segs + b.seg0;
+        aa.tile0 = b.tile0;
+        aa.tile1 = b.tile1;
+        NB_CUDA(launch_adjoint(a.shape, s->per_pair_mass, aa, b.grid, s->stream));
+        NB_CUDA(launch_adjoint_add(aa, b.end - b.tile0, adjoint_shape(a.shape).bi(), s->stream));
+      }
       std::swap(a.lam_x, a.tmp);
       std::swap(a.lam_v, a.mu);
     }

@@ -167,9 +167,8 @@ static int upload_state(nb_sim* s, const float* const arrays[7], bool with_mass)
   return NB_OK;
 }
 
-// Captured graphs bake in the work lists' and the scratch's device addresses:
-// whenever either is replaced, the graphs go too (nb_sim_graph_launch then reports
-// that none is captured).
+// Captured graphs bake in the work lists' device addresses: whenever they are replaced,
+// the graphs go too (nb_sim_graph_launch then reports that none is captured).
 static void drop_graphs(nb_sim* s) {
   for (int b = 0; b < 2; ++b) {
     if (s->gexec[b]) cudaGraphExecDestroy(s->gexec[b]);
@@ -178,6 +177,8 @@ static void drop_graphs(nb_sim* s) {
     s->graph[b] = nullptr;
   }
   s->graph_iters = 0;
+  for (void* p : s->retired) cudaFree(p);
+  s->retired.clear();
 }
 
 // Config indices: the tuned kernel's shapes, then the symmetric kernel's.
@@ -191,34 +192,37 @@ static KernelShape shape_of(int cfg) {
 }
 
 // Replace *p by a larger buffer; the current one stays (and serves the current work
-// list) when the allocation fails.
+// list) when the allocation fails, and until the graphs that hold its address go.
 template <class T>
-static int grow(T** p, size_t* cap, size_t need) {
+static int grow(nb_sim* s, T** p, size_t* cap, size_t need) {
   if (need <= *cap) return NB_OK;
   T* q = nullptr;
   NB_TRY(dev_alloc(&q, need));
-  dev_free(*p);
+  if (*p && s->graph_iters > 0)
+    s->retired.push_back(*p);
+  else
+    dev_free(*p);
   *p = q;
   *cap = need;
   return NB_OK;
 }
 
-static int ensure_scratch(nb_sim* s, const WorkListDev& w) {
-  const KernelShape sh = shape_of(w.cfg);
-  // Partial sums: (hi, lo) records for the compensated tuned kernel, one record
-  // otherwise (the reference-order kernel's hand-over holds one float4 per particle).
-  const size_t rec = (w.cfg >= 0 && s->params.accumulator == NB_ACC_COMPENSATED) ? 2 : 1;
-  const size_t need = static_cast<size_t>(w.slots) * sh.bi() * rec;
-  const size_t rows = 3 * static_cast<size_t>(w.row_values);
-  if (need > s->partials_cap || static_cast<size_t>(w.nfix) > s->counters_cap ||
-      rows > s->rows_cap)
-    drop_graphs(s);
-  NB_TRY(grow(&s->rows_d, &s->rows_cap, rows));
-  NB_TRY(grow(&s->partials_d, &s->partials_cap, need));
+// Records per slot and i-particle of config `cfg`: (hi, lo) for the compensated tuned
+// and symmetric kernels, one otherwise (the reference-order kernel's hand-over holds one
+// float4 per particle).
+static int part_records(const nb_sim* s, int cfg) {
+  return cfg >= 0 && s->params.accumulator == NB_ACC_COMPENSATED ? 2 : 1;
+}
+
+static int ensure_scratch(nb_sim* s, const WorkListDev& w, int bi, int rec) {
+  const size_t need = static_cast<size_t>(w.slots) * bi * rec;
+  NB_TRY(grow(s, &s->rows_d, &s->rows_cap, 3 * static_cast<size_t>(w.row_values)));
+  NB_TRY(grow(s, &s->partials_d, &s->partials_cap, need));
   if (w.bands.size() > 1 && !s->carry_d)
     NB_TRY(dev_alloc(&s->carry_d, 2 * static_cast<size_t>(s->n_pad)));
   if (static_cast<size_t>(w.nfix) > s->counters_cap) {
-    NB_TRY(grow(&s->counters_d, &s->counters_cap, static_cast<size_t>(w.nfix)));
+    drop_graphs(s);  // they expect their counters at zero
+    NB_TRY(grow(s, &s->counters_d, &s->counters_cap, static_cast<size_t>(w.nfix)));
     NB_CUDA(cudaMemsetAsync(s->counters_d, 0, w.nfix * sizeof(int32_t), s->stream));
   }
   return NB_OK;
@@ -266,7 +270,7 @@ static int upload_worklist(nb_sim* s, const WorkListHost& h, int cfg, WorkListDe
     free_worklist(w);
     return cuda_error(e, "upload work list");
   }
-  st = ensure_scratch(s, w);
+  st = ensure_scratch(s, w, shape_of(cfg).bi(), part_records(s, cfg));
   if (st != NB_OK) {
     free_worklist(w);
     return st;
@@ -289,13 +293,8 @@ static int plan_tuned(nb_sim* s, int cfg, int32_t first, int32_t count, int grid
   return NB_OK;
 }
 
-// Plan systems [first, first + count) for symmetric-kernel config `cfg`.
-static int plan_sym(nb_sim* s, int cfg, int32_t first, int32_t count, WorkListDev* out) {
-  const KernelShape sh = shape_of(cfg);
-  const SymPlanHost h = plan_symmetric(s->sys_h.data(), first, count, sh.bi(), sh.bj,
-                                       max_grid_for(s, cfg), kSymScratchBytes / kSymRowBytes);
+int upload_symmetric(nb_sim* s, const SymPlanHost& h, int bi, int rec, WorkListDev* out) {
   WorkListDev w;
-  w.cfg = cfg;
   w.grid = h.bands[0].grid;
   w.nseg = static_cast<int32_t>(h.segs.size());
   w.slots = h.slots;
@@ -305,7 +304,7 @@ static int plan_sym(nb_sim* s, int cfg, int32_t first, int32_t count, WorkListDe
   const std::vector<SymSegment> segs = link_segments(h);
   int st = dev_alloc(&w.sym_segs, segs.size());
   if (st == NB_OK) st = dev_alloc(&w.sym_tiles, h.tiles.size());
-  if (st == NB_OK) st = ensure_scratch(s, w);
+  if (st == NB_OK) st = ensure_scratch(s, w, bi, rec);
   if (st != NB_OK) {
     free_worklist(w);
     return st;
@@ -321,6 +320,16 @@ static int plan_sym(nb_sim* s, int cfg, int32_t first, int32_t count, WorkListDe
     return cuda_error(e, "upload work list");
   }
   *out = w;
+  return NB_OK;
+}
+
+// Plan systems [first, first + count) for symmetric-kernel config `cfg`.
+static int plan_sym(nb_sim* s, int cfg, int32_t first, int32_t count, WorkListDev* out) {
+  const KernelShape sh = shape_of(cfg);
+  const SymPlanHost h = plan_symmetric(s->sys_h.data(), first, count, sh.bi(), sh.bj,
+                                       max_grid_for(s, cfg), kSymScratchBytes / kSymRowBytes);
+  NB_TRY(upload_symmetric(s, h, sh.bi(), part_records(s, cfg), out));
+  out->cfg = cfg;
   return NB_OK;
 }
 
@@ -517,43 +526,22 @@ static bool sharded(const nb_sim* s) {
   return s->sys_h[0].shard_first != 0 || s->sys_h[0].shard_count != 0;
 }
 
-// Default symmetric-kernel config for systems [first, first + count).  Larger i-tiles
-// run their pairs at a higher rate but leave more of them on the diagonal and in a
-// system's last tile, and make fewer blocks to balance.  So: the shape with the lowest
-// charge over rate among those with enough blocks per CTA.  Rates are measured at
-// N = 1,048,576 (229.9, 251.8, 267.2 and 373.1 ms per step, where all are balanced and
-// nearly nothing is diagonal); the blocks, at the sizes of single systems where two
-// neighbouring shapes meet (thin disks, us per step with the larger / the smaller
-// i-tiles): 36,000 319 / 315 and 50,000 587 / 598 for 4,096 against 512 particles;
-// 12,800 55.2 / 50.7 and 25,600 167.4 / 172.5 for 512 against 256; 4,096 14.7 / 14.0
-// and 8,192 25.7 / 30.3 for 256 against 64.
+// Default symmetric-kernel config for systems [first, first + count).  The shapes' rates
+// are measured at N = 1,048,576 (229.9, 251.8, 267.2 and 373.1 ms per step, where all
+// are balanced and nearly nothing is diagonal); the blocks per CTA, at the sizes of
+// single systems where two neighbouring shapes meet (thin disks, us per step with the
+// larger / the smaller i-tiles): 36,000 319 / 315 and 50,000 587 / 598 for 4,096 against
+// 512 particles; 12,800 55.2 / 50.7 and 25,600 167.4 / 172.5 for 512 against 256; 4,096
+// 14.7 / 14.0 and 8,192 25.7 / 30.3 for 256 against 64.
 static int default_symmetric_for(nb_sim* s, int32_t first, int32_t count) {
-  static const struct {
-    double rate, blocks_per_cta;
-  } kShapes[] = {{1.0, 12.0}, {0.913, 7.0}, {0.86, 0.8}, {0.617, 0.0}};
-  const int shapes = num_symmetric_shapes();
-  int best = shapes - 1;
-  double best_time = DBL_MAX;
-  for (int k = 0; k < shapes; ++k) {
-    const KernelShape sh = symmetric_shape(k);
-    double charge = 0, blocks = 0;
-    for (int32_t q = first; q < first + count; ++q) {
-      const double npad = s->sys_h[q].npad, bi = sh.bi();
-      const double tiles = (s->sys_h[q].n + sh.bi() - 1) / sh.bi();
-      const double last = npad - (tiles - 1) * bi;                // columns of the last i-tile
-      const double cols = tiles * npad - bi * tiles * (tiles - 1) / 2;
-      const double diag = (tiles - 1) * bi + last;
-      charge += bi * (kSymDiagCost * diag + kSymPairCost * (cols - diag));
-      blocks += cols / sh.bj;
-    }
-    const double time = charge / kShapes[k].rate;
-    if (time < best_time &&
-        blocks >= kShapes[k].blocks_per_cta * max_grid_for(s, num_force_configs() + k)) {
-      best = k;
-      best_time = time;
-    }
-  }
-  return num_force_configs() + best;
+  static constexpr double kRates[][2] = {{1.0, 12.0}, {0.913, 7.0}, {0.86, 0.8}, {0.617, 0.0}};
+  constexpr int kCount = sizeof(kRates) / sizeof(kRates[0]);
+  SymCandidate c[kCount];
+  for (int k = 0; k < kCount; ++k)
+    c[k] = SymCandidate{symmetric_shape(k), kRates[k][0], kRates[k][1],
+                        max_grid_for(s, num_force_configs() + k)};
+  return num_force_configs() + choose_symmetric(s->sys_h.data(), first, count, c, kCount,
+                                                kSymDiagCost, kSymPairCost);
 }
 
 // Default kernel shape of systems [first, first + count), judged alone: a symmetric one,
@@ -883,10 +871,7 @@ int nb_sim_destroy(nb_sim* s) {
   if (!s) return NB_OK;
   DeviceGuard dg_(s->device);
   if (s->stream) cudaStreamSynchronize(s->stream);
-  for (int b = 0; b < 2; ++b) {
-    if (s->gexec[b]) cudaGraphExecDestroy(s->gexec[b]);
-    if (s->graph[b]) cudaGraphDestroy(s->graph[b]);
-  }
+  drop_graphs(s);
   free_worklist(s->wl);
   free_worklist(s->inject_wl);
   for (auto& w : s->wl_sys) free_worklist(w);

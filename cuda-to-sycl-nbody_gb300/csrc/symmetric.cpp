@@ -2,6 +2,7 @@
 #include "symmetric.hpp"
 
 #include <algorithm>
+#include <cfloat>
 
 namespace nbg {
 
@@ -29,7 +30,8 @@ struct TileCharge {
 }  // namespace
 
 SymPlanHost plan_symmetric(const SystemDesc* sys, int32_t first, int32_t count, int32_t bi,
-                           int32_t bj, int32_t max_grid, int64_t max_row_values) {
+                           int32_t bj, int32_t max_grid, int64_t max_row_values,
+                           int diag_cost, int pair_cost) {
   SymPlanHost plan;
   // The i-tiles, their rows and the bands they fall into.
   plan.sys_tile0.assign(first + count + 1, 0);
@@ -61,8 +63,8 @@ SymPlanHost plan_symmetric(const SystemDesc* sys, int32_t first, int32_t count, 
     c.t0 = t.itile * (bi / bj);
     c.t1 = (d.npad + bj - 1) / bj;
     c.td = std::min(c.t1, c.t0 + bi / bj);
-    c.diag = static_cast<int64_t>(bj) * kSymDiagCost;
-    c.pair = static_cast<int64_t>(bj) * kSymPairCost;
+    c.diag = static_cast<int64_t>(bj) * diag_cost;
+    c.pair = static_cast<int64_t>(bj) * pair_cost;
     return c;
   };
   for (SymBand& b : plan.bands) {
@@ -117,6 +119,32 @@ SymPlanHost plan_symmetric(const SystemDesc* sys, int32_t first, int32_t count, 
     plan.slots = std::max(plan.slots, static_cast<int32_t>(plan.segs.size()) - b.seg0);
   }
   return plan;
+}
+
+int choose_symmetric(const SystemDesc* sys, int32_t first, int32_t count, const SymCandidate* c,
+                     int count_c, int diag_cost, int pair_cost) {
+  int best = count_c - 1;
+  double best_time = DBL_MAX;
+  for (int k = 0; k < count_c; ++k) {
+    const KernelShape& sh = c[k].shape;
+    double charge = 0, blocks = 0;
+    for (int32_t q = first; q < first + count; ++q) {
+      const double npad = sys[q].npad, bi = sh.bi();
+      const double tiles = (sys[q].n + sh.bi() - 1) / sh.bi();
+      const double last = npad - (tiles - 1) * bi;  // columns of the last i-tile
+      const double cols = tiles * npad - bi * tiles * (tiles - 1) / 2;
+      const double diag = (tiles - 1) * bi + last;
+      charge += bi * (diag_cost * diag + pair_cost * (cols - diag));
+      blocks += cols / sh.bj;
+    }
+    const double time = charge / c[k].rate;
+    if (time < best_time &&
+        (k + 1 == count_c || blocks >= c[k].blocks_per_cta * c[k].max_grid)) {
+      best = k;
+      best_time = time;
+    }
+  }
+  return best;
 }
 
 std::vector<SymSegment> link_segments(const SymPlanHost& plan) {

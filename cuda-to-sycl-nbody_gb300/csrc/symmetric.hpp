@@ -26,6 +26,9 @@ namespace nbg {
 // Lane operations per pair on the FMA pipe (symmetric_kernel.cuh): one side, both sides.
 constexpr int kSymDiagCost = 11;
 constexpr int kSymPairCost = 14;
+// The same of the adjoint (adjoint_kernel.cu).
+constexpr int kAdjDiagCost = 22;
+constexpr int kAdjPairCost = 25;
 constexpr int64_t kSymRowBytes = 3 * sizeof(float);  // scratch per row value
 constexpr int64_t kSymScratchBytes = int64_t{1} << 29;
 
@@ -83,8 +86,26 @@ std::vector<SymSegment> link_segments(const SymPlanHost& plan);
 
 // Plan systems [first, first + count) (whole systems, no shards) for i-tiles of bi and
 // j-tiles of bj particles (bi % bj == 0) on at most max_grid CTAs, with at most
-// max_row_values row values per band (one i-tile at least).
+// max_row_values row values per band (one i-tile at least); diag_cost and pair_cost: the
+// charges per particle of a diagonal and of another j-tile.
 SymPlanHost plan_symmetric(const SystemDesc* sys, int32_t first, int32_t count, int32_t bi,
-                           int32_t bj, int32_t max_grid, int64_t max_row_values);
+                           int32_t bj, int32_t max_grid, int64_t max_row_values,
+                           int diag_cost = kSymDiagCost, int pair_cost = kSymPairCost);
+
+// A shape to choose from: its relative rate where it is balanced, the blocks per CTA
+// from which it is, and its largest grid.
+struct SymCandidate {
+  KernelShape shape;
+  double rate;
+  double blocks_per_cta;
+  int max_grid;
+};
+
+// Index of the best of `count_c` shapes for systems [first, first + count): the lowest
+// charge over rate among those with enough blocks per CTA (the last always counts).
+// Larger i-tiles run their pairs at a higher rate but leave more of them on the diagonal
+// and in a system's last tile, and make fewer blocks to balance.
+int choose_symmetric(const SystemDesc* sys, int32_t first, int32_t count, const SymCandidate* c,
+                     int count_c, int diag_cost, int pair_cost);
 
 }  // namespace nbg

@@ -1,160 +1,42 @@
-// The adding pass of the symmetric force step (symmetric_kernel.cuh): a particle's
-// force is the sum over its i-tile's parts (the CTAs that shared it) minus the rows of
-// the i-tiles before its own, in a fixed order (compensated or plain), and then the
-// integrate epilogue.  With several bands the running sum is carried from band to band.
-//
-// What bounds it: load latency (a particle of a 4,096-particle system has up to 130
-// terms of 12 to 32 bytes, a few MB in all, from L2), not bandwidth.  So a CTA is 32
-// particles by 8 groups, each group adding a contiguous range of the terms, eight loads
-// in flight, and the groups' sums are added in order.
+// The adding pass of the symmetric force step, with the integrate epilogue.
 #include <cuda_runtime.h>
 
 #include "nb_device.cuh"
 #include "nb_kernels.hpp"
-#include "symmetric.hpp"
+#include "symmetric_add.cuh"
 
 namespace nbg {
 namespace {
 
-constexpr int kAddBatch = 8;
-// From here on two groups (of 64 particles) fill the GPU.
-constexpr int64_t kManyParticles = 1 << 17;
-
-template <bool kComp>
-struct Sum3 {
-  float s[3] = {0.f, 0.f, 0.f}, c[3] = {0.f, 0.f, 0.f};
-  __device__ __forceinline__ void add(int k, float t) {
-    if (kComp) {
-      const float y = t - c[k], u = s[k] + y;
-      c[k] = (u - s[k]) - y;
-      s[k] = u;
-    } else {
-      s[k] += t;
-    }
+struct EarlyForce {
+  const ForceArgs& f;
+  SystemDesc sd;
+  float x, y, z;
+  __device__ void lists(int sys) { sd = f.sys[sys]; }
+  __device__ void state(int64_t g) {
+    x = f.pos[pair_index(g, 0)];
+    y = f.pos[pair_index(g, 1)];
+    z = f.pos[pair_index(g, 2)];
   }
 };
 
-// blockIdx.x: i-tile tile0 + x of the band's systems; blockIdx.y: 32 of its particles.
-template <int kAddLanes, int kAddGroups, bool kComp>
-__global__ void __launch_bounds__(kAddLanes * kAddGroups) symmetric_add_kernel(const SymArgs a,
-                                                                               int bi) {
-  __shared__ float group_sum[kAddGroups][6][kAddLanes];
-  const int t = a.tile0 + blockIdx.x;
-  const SymTile tile = a.tiles[t];
-  const int sys0 = t - tile.itile;  // the system's first i-tile
-  const int64_t row_first = a.tiles[max(sys0, a.tile0)].row;
-  const SystemDesc sd = a.f.sys[tile.sys];
-  pdl_trigger();
-  pdl_wait();
-  const int lane = threadIdx.x % kAddLanes, group = threadIdx.x / kAddLanes;
-  const int idx = blockIdx.y * kAddLanes + lane;
-  const int j = tile.itile * bi + idx;
-  if (j - lane >= tile.n) return;
-  const bool real = j < tile.n;
-  const int64_t g = tile.offset + j;
-  const int i0 = max(0, a.tile0 - sys0);  // the band's first i-tile in the system
-  const bool mine = t < a.tile1;          // the particle's i-tile is in the band
-  const int nrows = (mine ? tile.itile : a.tile1 - sys0) - i0;
-  const int nparts = mine ? tile.nslots : 0;
+template <int kLanes, int kGroups, bool kComp>
+__global__ void __launch_bounds__(kLanes * kGroups) symmetric_add_kernel(const SymArgs a, int bi) {
+  const AddTerms t{a.tiles, a.rows, a.plane, a.carry, a.f.partials, a.tile0, a.tile1};
+  EarlyForce e{a.f, {}, 0.f, 0.f, 0.f};
+  AddResult r;
+  if (add_terms<kLanes, kGroups, kComp>(t, bi, e, r))
+    finish_particle(a.f, e.sd, r.g, r.x, r.y, r.z, e.x, e.y, e.z);
+}
 
-  float xi = 0.f, yi = 0.f, zi = 0.f;  // asked for now, used at the end
-  if (group == 0 && real) {
-    xi = a.f.pos[pair_index(g, 0)];
-    yi = a.f.pos[pair_index(g, 1)];
-    zi = a.f.pos[pair_index(g, 2)];
-  }
-
-  Sum3<kComp> sum;
-  float q[3] = {0.f, 0.f, 0.f};  // low words of the parts
-  // The group's rows.  The row of each i-tile is bi values shorter than the one before.
-  const int k1 = real ? nrows * (group + 1) / kAddGroups : 0;
-  int k = nrows * group / kAddGroups;
-  const int64_t npad = (tile.n + kPadQuantum - 1) & -kPadQuantum;
-  int64_t step = npad - static_cast<int64_t>(i0 + 2 + k) * bi;  // from row k to row k + 1
-  const float* row = a.rows + (row_first + j + k * (npad - static_cast<int64_t>(i0 + 2) * bi) -
-                               bi * (static_cast<int64_t>(k) * (k - 1) / 2));
-  for (; k < k1; k += kAddBatch) {
-    float v[kAddBatch][3];
-#pragma unroll
-    for (int u = 0; u < kAddBatch; ++u) {
-      const bool in = k + u < k1;
-      v[u][0] = in ? -row[0] : 0.f;
-      v[u][1] = in ? -row[a.plane] : 0.f;
-      v[u][2] = in ? -row[2 * a.plane] : 0.f;
-      row += step;
-      step -= bi;
-    }
-#pragma unroll
-    for (int u = 0; u < kAddBatch; ++u)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) sum.add(c, v[u][c]);
-  }
-  // The group's parts.
-  constexpr int kRec = kComp ? 2 : 1;
-  const int p1 = real ? nparts * (group + 1) / kAddGroups : 0;
-  int p = nparts * group / kAddGroups;
-  const float4* part =
-      a.f.partials + (static_cast<int64_t>(tile.slot0 + p) * bi + idx) * kRec;
-  for (; p < p1; p += kAddBatch / 2) {
-    float4 h[kAddBatch / 2], l[kAddBatch / 2];
-#pragma unroll
-    for (int u = 0; u < kAddBatch / 2; ++u) {
-      const bool in = p + u < p1;
-      h[u] = in ? part[0] : make_float4(0.f, 0.f, 0.f, 0.f);
-      if (kComp) l[u] = in ? part[1] : make_float4(0.f, 0.f, 0.f, 0.f);
-      part += static_cast<int64_t>(bi) * kRec;
-    }
-#pragma unroll
-    for (int u = 0; u < kAddBatch / 2; ++u) {
-      sum.add(0, h[u].x);
-      sum.add(1, h[u].y);
-      sum.add(2, h[u].z);
-      if (kComp) q[0] += l[u].x, q[1] += l[u].y, q[2] += l[u].z;
-    }
-  }
-  // Group sums in order, each as its sum and what is still to be added to it.
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    group_sum[group][c][lane] = sum.s[c];
-    group_sum[group][3 + c][lane] = kComp ? q[c] - sum.c[c] : 0.f;
-  }
-  __syncthreads();
-  if (group > 0 || !real) return;
-  Sum3<kComp> all;
-  float low[3] = {0.f, 0.f, 0.f};
-  if (sys0 < a.tile0) {  // earlier bands
-    const float4 s = a.carry[2 * g], l = a.carry[2 * g + 1];
-    all.s[0] = s.x, all.s[1] = s.y, all.s[2] = s.z;
-    low[0] = l.x, low[1] = l.y, low[2] = l.z;
-  }
-#pragma unroll
-  for (int u = 0; u < kAddGroups; ++u)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      all.add(c, group_sum[u][c][lane]);
-      if (kComp) low[c] += group_sum[u][3 + c][lane];
-    }
-  if (kComp)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) low[c] -= all.c[c];
-  if (!mine) {  // later bands add the rest
-    a.carry[2 * g] = make_float4(all.s[0], all.s[1], all.s[2], 0.f);
-    a.carry[2 * g + 1] = make_float4(low[0], low[1], low[2], 0.f);
-    return;
-  }
-  finish_particle(a.f, sd, g, all.s[0] + low[0], all.s[1] + low[1], all.s[2] + low[2],
-                  xi, yi, zi);
+template <int kLanes, int kGroups>
+cudaError_t add_one(bool compensated, const SymArgs& a, int tiles, int bi, cudaStream_t stream) {
+  return launch_dependent(compensated ? symmetric_add_kernel<kLanes, kGroups, true>
+                                      : symmetric_add_kernel<kLanes, kGroups, false>,
+                          add_grid<kLanes>(tiles, bi), kLanes * kGroups, 0, stream, a, bi);
 }
 
 }  // namespace
-
-template <int kLanes, int kGroups>
-static cudaError_t add_one(bool compensated, const SymArgs& a, int tiles, int bi,
-                           cudaStream_t stream) {
-  return launch_dependent(compensated ? symmetric_add_kernel<kLanes, kGroups, true>
-                                      : symmetric_add_kernel<kLanes, kGroups, false>,
-                          dim3(tiles, bi / kLanes), kLanes * kGroups, 0, stream, a, bi);
-}
 
 cudaError_t launch_symmetric_add(bool compensated, const SymArgs& a, int tiles, int bi,
                                  cudaStream_t stream) {
