@@ -1,10 +1,13 @@
 // FP64 diagnostics on the GPU: kinetic and potential energy, linear and angular
-// momentum, and FP64 accelerations of selected rows.  Pair arithmetic and all
-// reductions are double precision; reductions use fixed-order trees and
-// per-block partials summed in block order, so results are deterministic.
+// momentum, and FP64 accelerations of selected rows.  Sums are double precision, and
+// so is the pair arithmetic, except the potential's of large systems, whose terms are
+// sums of two floats; reductions use fixed-order trees over per-block partials, so
+// results are deterministic.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <vector>
 
 #include "nb_internal.hpp"
 #include "nb_kernels.hpp"
@@ -29,17 +32,31 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   return r;
 }
 
+// Whether a value lies where the split potential below neither overflows nor loses low
+// words to underflow (NaN does not).
+__device__ __forceinline__ bool splittable(float x, float y, float z, float m) {
+  return fabsf(x) <= 1e6f && fabsf(y) <= 1e6f && fabsf(z) <= 1e6f &&
+         (m == 0.f || (fabsf(m) >= 1e-12f && fabsf(m) <= 1e12f));
+}
+
 // Per-particle moments over the padded range [first, last): padding has zero
-// mass and velocity, so it contributes nothing.
-__global__ void moments_kernel(const float* __restrict__ pos, const float4* __restrict__ vel,
-                               int64_t first, int64_t last, double* __restrict__ partial) {
+// mass and velocity, so it contributes nothing.  Sets *wide where a particle is not
+// splittable.
+__global__ void __launch_bounds__(kDiagThreads) moments_kernel(
+    const float* __restrict__ pos, const float4* __restrict__ vel, int64_t first, int64_t last,
+    double* __restrict__ partial, int* __restrict__ wide) {
   __shared__ double sh[kDiagThreads];
   double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  bool far = false;
   for (int64_t g = first + blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; g < last;
        g += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const double m = pos[pair_index(g, 3)];
+    const float xf = pos[pair_index(g, 0)], yf = pos[pair_index(g, 1)], zf = pos[pair_index(g, 2)];
+    const float mf = pos[pair_index(g, 3)];
+    if (xf == kFarAway && mf == 0.f) continue;  // padding
+    far = far || !splittable(xf, yf, zf, mf);
+    const double m = mf;
     if (m == 0.0) continue;
-    const double x = pos[pair_index(g, 0)], y = pos[pair_index(g, 1)], z = pos[pair_index(g, 2)];
+    const double x = xf, y = yf, z = zf;
     const float4 v = vel[g];
     const double vx = v.x, vy = v.y, vz = v.z;
     acc[0] += 0.5 * m * (vx * vx + vy * vy + vz * vz);
@@ -51,61 +68,312 @@ __global__ void moments_kernel(const float* __restrict__ pos, const float4* __re
     acc[7] += m * (x * vy - y * vx);
     acc[8] += m;
   }
+  if (far) atomicOr(wide, 1);
   for (int k = 0; k < 9; ++k) {
     const double s = block_sum(acc[k], sh);
     if (threadIdx.x == 0) partial[blockIdx.x * kDiagVals + k] = s;
   }
 }
 
-// Potential: block b handles i-tile tiles[b] = (system, tile) and all j > i of
-// that system.  Writes -G * sum_i m_i sum_{j>i} m_j / sqrt(r^2 + eps) to partial.
-__global__ void potential_kernel(const float* __restrict__ pos, const SystemDesc* __restrict__ sys,
-                                 const int2* __restrict__ tiles, float eps2, double G,
-                                 double* __restrict__ partial) {
-  __shared__ double sh[kDiagThreads];
-  __shared__ float4 tj[kDiagThreads];
+// ---- potential, pairs in two floats -------------------------------------------------
+// The potential needs N^2 / 2 inverse square roots in double precision, about 30 FP64
+// operations per pair on a pipe of 2 lanes per SM (FP32: 128; a third-order step from the FP32 root is no faster
+// than rsqrt: its conversions run on that pipe too).  Here a pair's term is a
+// sum of two floats (packed FP32x2, two j-particles per register pair): the coordinate
+// differences are exact (TwoSum), the squared distance and the root carry 47 bits or
+// more (two Newton steps on the MUFU rsqrt, residuals by fused multiply-add), and 128
+// terms at a time are added error-free before they go to FP64.  About 90 FP32 lane
+// operations per pair.  Errors of single terms (below 1e-14) average out over a
+// system's pairs, and the sums are no further from exact ones than the FP64 kernel's,
+// whose threads add thousands of terms one after another (RMS over disks and spheres,
+// equal and own masses, FP64 / split: 1.6e-16 / 1.2e-16 at N = 6,000, 2.0e-16 / 1.6e-16
+// at 10,011, 5.6e-16 / 2.2e-16 at 65,536).  N = 65,536: 103.5 ms before, 7.6 now.
+// Systems below kSplitMin particles, softenings below kSplitEps and values out of the
+// split's range keep the FP64 kernel; an i-tile whose particles are nearly at one place,
+// where all terms are rounded alike and nothing averages out, is summed in FP64 too.
+constexpr int kSplitMin = 4096;  // below, FP64's sums are the more exact ones
+constexpr float kSplitEps = 1e-12f;
+constexpr int kSplitThreads = 256;
+constexpr int kSplitR = 1;                          // i-particles per thread
+constexpr int kSplitBI = kSplitThreads * kSplitR;   // i-tile and j-tile
+constexpr int kSplitFlush = 64;                     // j-pairs between two sums into FP64
+
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, neg2(b)); }
+
+// a + b = s + e exactly (Knuth's TwoSum).
+__device__ __forceinline__ float2 two_sum(float2 a, float2 b, float2& e) {
+  const float2 s = __fadd2_rn(a, b);
+  const float2 t = sub2(s, a);
+  e = __fadd2_rn(sub2(a, sub2(s, t)), sub2(b, t));
+  return s;
+}
+
+// One squared difference: a - b = h + l exactly, its square as p + q + l^2.
+__device__ __forceinline__ void square_diff(float2 a, float2 nb, float2& p, float2& q, float2& l) {
+  const float2 h = two_sum(a, nb, l);
+  p = __fmul2_rn(h, h);
+  q = __ffma2_rn(h, h, neg2(p));
+  q = __ffma2_rn(__fadd2_rn(h, h), l, q);
+}
+
+// 1 - (h + l) y^2, for y near the inverse square root of h + l.
+__device__ __forceinline__ float2 root_residual(float2 h, float2 l, float2 y) {
+  const float2 p = __fmul2_rn(h, y);
+  const float2 pe = __ffma2_rn(h, y, neg2(p));
+  const float2 ny = neg2(y);
+  float2 e = __ffma2_rn(p, ny, make_float2(1.f, 1.f));
+  e = __ffma2_rn(pe, ny, e);
+  return __ffma2_rn(__fmul2_rn(l, y), ny, e);
+}
+
+// j-pairs [p0, p1) of the shared tile against the thread's i-particles, added to
+// (s, l, k): the sum is s + l - k / 2.
+// kMask: leave out j == i and j >= cnt.
+template <bool kMass, bool kMask>
+__device__ __forceinline__ void split_pairs(const float4* tile, int p0, int p1, int cnt,
+                                            const float2 (&nx)[kSplitR],
+                                            const float2 (&ny)[kSplitR],
+                                            const float2 (&nz)[kSplitR], float2 e2, int self,
+                                            float2 (&s)[kSplitR], float2 (&l)[kSplitR],
+                                            float2 (&k)[kSplitR]) {
+#pragma unroll 2
+  for (int p = p0; p < p1; ++p) {
+    const float4 A = tile[2 * p], B = tile[2 * p + 1];
+#pragma unroll
+    for (int r = 0; r < kSplitR; ++r) {
+      float2 px, qx, lx, py, qy, ly, pz, qz, lz, a, b, c;
+      square_diff(make_float2(A.x, A.y), nx[r], px, qx, lx);
+      square_diff(make_float2(A.z, A.w), ny[r], py, qy, ly);
+      square_diff(make_float2(B.x, B.y), nz[r], pz, qz, lz);
+      // What the differences' low words add to the square, at most 2^-48 of it: never
+      // negative, so rounding it away would shift every term the same way (1e-16).
+      const float2 ll = __ffma2_rn(lz, lz, __ffma2_rn(ly, ly, __fmul2_rn(lx, lx)));
+      float2 h = two_sum(px, py, a);
+      h = two_sum(h, pz, b);
+      h = two_sum(h, e2, c);
+      const float2 low = __fadd2_rn(__fadd2_rn(__fadd2_rn(a, b), c),
+                                    __fadd2_rn(__fadd2_rn(qx, qy), qz));
+      const float2 H = __fadd2_rn(h, low);
+      const float2 L = sub2(low, sub2(H, h));
+      float2 y = make_float2(rsqrtf(H.x), rsqrtf(H.y));
+      // y + y e (1/2 + 3/8 e) rounded to one float, then what is left of it.  (Without
+      // its 3/8 e^2 the second step would be off by 4e-16 on average, always to one side.)
+      const float2 c3 = make_float2(0.375f, 0.375f), c1 = make_float2(0.5f, 0.5f);
+      float2 e = root_residual(H, L, y);
+      y = __ffma2_rn(y, __fmul2_rn(e, __ffma2_rn(c3, e, c1)), y);
+      e = root_residual(H, L, y);
+      float2 w = __fmul2_rn(y, __fmul2_rn(e, __ffma2_rn(c3, e, c1)));
+      float2 v = __fmul2_rn(__fmul2_rn(__fmul2_rn(y, y), y), ll);
+      if (kMass) {
+        const float2 m = make_float2(B.z, B.w);
+        v = __fmul2_rn(m, v);
+        const float2 my = __fmul2_rn(m, y);
+        w = __ffma2_rn(m, w, __ffma2_rn(m, y, neg2(my)));
+        y = my;
+      }
+      if (kMask) {
+        if (2 * p == self + r * kSplitThreads || 2 * p >= cnt) y.x = w.x = v.x = 0.f;
+        if (2 * p + 1 == self + r * kSplitThreads || 2 * p + 1 >= cnt) y.y = w.y = v.y = 0.f;
+      }
+      float2 t;
+      s[r] = two_sum(s[r], y, t);
+      l[r] = __fadd2_rn(l[r], __fadd2_rn(t, w));
+      k[r] = __fadd2_rn(k[r], v);
+    }
+  }
+}
+
+// Whether the block's particles nearly coincide: within 2^-10 of their coordinates in
+// every component, or within 2^-20 softening lengths.
+__device__ __forceinline__ bool nearly_coincident(float x, float y, float z, float eps2) {
+  __shared__ float ext[kSplitThreads / 32][6];
+  float v[6] = {x, y, z, -x, -y, -z};
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    for (int d = 16; d > 0; d >>= 1) v[c] = fmaxf(v[c], __shfl_xor_sync(0xffffffffu, v[c], d));
+    if (threadIdx.x % 32 == 0) ext[threadIdx.x / 32][c] = v[c];
+  }
+  __syncthreads();
+  float extent2 = 0.f;
+  bool near = true;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    float hi = ext[0][c], lo = -ext[0][c + 3];
+    for (int w = 1; w < kSplitThreads / 32; ++w) {
+      hi = fmaxf(hi, ext[w][c]);
+      lo = fminf(lo, -ext[w][c + 3]);
+    }
+    near = near && hi - lo <= 0x1p-10f * fmaxf(fabsf(hi), fabsf(lo));
+    extent2 = fmaf(hi - lo, hi - lo, extent2);
+  }
+  return near || extent2 <= 0x1p-40f * eps2;
+}
+
+// One i-particle's sum over j in [j0, j1) of its system, j > i, in FP64.
+__device__ __noinline__ double fp64_row(const float* __restrict__ pos, int64_t offset, int li,
+                                        int j0, int j1, double eps2) {
+  const int64_t gi = offset + li;
+  const double xi = pos[pair_index(gi, 0)], yi = pos[pair_index(gi, 1)],
+               zi = pos[pair_index(gi, 2)];
+  double sum = 0.0;
+  for (int j = max(j0, li + 1); j < j1; ++j) {
+    const int64_t g = offset + j;
+    const double dx = pos[pair_index(g, 0)] - xi, dy = pos[pair_index(g, 1)] - yi,
+                 dz = pos[pair_index(g, 2)] - zi;
+    const double d2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
+    sum = fma(static_cast<double>(pos[pair_index(g, 3)]), rsqrt(d2), sum);
+  }
+  return sum;
+}
+
+// blockIdx.x: i-tile tiles[x] = (system, tile); blockIdx.y: one of gridDim.y spans of the
+// j-tiles from it to the end of the system.  Each pair of different tiles is met once;
+// the i-tile itself over all ordered pairs, at half weight.  Writes its part of
+// -G sum_i m_i sum_j m_j / sqrt(r^2 + eps), zero where the FP64 kernel does the system.
+template <bool kMass>
+__global__ void __launch_bounds__(kSplitThreads) potential_split_kernel(
+    const float* __restrict__ pos, const SystemDesc* __restrict__ sys,
+    const int2* __restrict__ tiles, const int* __restrict__ wide, float eps2, double G,
+    double* __restrict__ partial) {
+  __shared__ __align__(16) float4 tile[kSplitBI];
+  __shared__ double sh[kSplitThreads];
   const int2 tl = tiles[blockIdx.x];
   const SystemDesc sd = sys[tl.x];
-  const int li = tl.y * kDiagThreads + threadIdx.x;
+  const int tid = threadIdx.x;
+  const int njt = (sd.n + kSplitBI - 1) / kSplitBI - tl.y;
+  const int t0 = tl.y + static_cast<int>(static_cast<int64_t>(njt) * blockIdx.y / gridDim.y);
+  const int t1 = tl.y + static_cast<int>(static_cast<int64_t>(njt) * (blockIdx.y + 1) / gridDim.y);
+  double* out = partial + static_cast<int64_t>(blockIdx.y) * gridDim.x + blockIdx.x;
+  if (*wide || sd.n < kSplitMin || t0 == t1) {
+    if (tid == 0) *out = 0.0;
+    return;
+  }
+  const float4* recs = reinterpret_cast<const float4*>(pos + 4 * sd.offset);
+  const float2 e2 = make_float2(eps2, eps2);
+  float2 nx[kSplitR], ny[kSplitR], nz[kSplitR];
+  double acc[kSplitR], mi[kSplitR];
+#pragma unroll
+  for (int r = 0; r < kSplitR; ++r) {
+    const int li = tl.y * kSplitBI + r * kSplitThreads + tid;
+    const int64_t g = sd.offset + min(li, sd.n - 1);
+    const float x = pos[pair_index(g, 0)], y = pos[pair_index(g, 1)], z = pos[pair_index(g, 2)];
+    nx[r] = make_float2(-x, -x);
+    ny[r] = make_float2(-y, -y);
+    nz[r] = make_float2(-z, -z);
+    mi[r] = li < sd.n ? static_cast<double>(pos[pair_index(g, 3)]) : 0.0;
+    acc[r] = 0.0;
+  }
+  static_assert(kSplitR == 1, "the block's particles are its threads'");
+  if (nearly_coincident(-nx[0].x, -ny[0].x, -nz[0].x, eps2)) {
+    const int li = tl.y * kSplitBI + tid;
+    const double v = li < sd.n ? fp64_row(pos, sd.offset, li, t0 * kSplitBI,
+                                          min(sd.n, t1 * kSplitBI), eps2)
+                               : 0.0;
+    const double total = block_sum(-G * mi[0] * v, sh);
+    if (tid == 0) *out = total;
+    return;
+  }
+  for (int t = t0; t < t1; ++t) {
+    const int cnt = min(kSplitBI, sd.n - t * kSplitBI);
+    const int npairs = (cnt + 1) / 2;
+    __syncthreads();
+    for (int k = tid; k < 2 * npairs; k += kSplitThreads)
+      tile[k] = recs[static_cast<int64_t>(t) * kSplitBI + k];
+    __syncthreads();
+    const bool diag = t == tl.y;
+    for (int p = 0; p < npairs; p += kSplitFlush) {
+      float2 s[kSplitR], l[kSplitR], k[kSplitR];
+#pragma unroll
+      for (int r = 0; r < kSplitR; ++r) s[r] = l[r] = k[r] = make_float2(0.f, 0.f);
+      const int p1 = min(npairs, p + kSplitFlush);
+      if (diag || cnt < kSplitBI)
+        split_pairs<kMass, true>(tile, p, p1, cnt, nx, ny, nz, e2,
+                                 diag ? tid : -2 * kSplitBI, s, l, k);
+      else
+        split_pairs<kMass, false>(tile, p, p1, cnt, nx, ny, nz, e2, 0, s, l, k);
+#pragma unroll
+      for (int r = 0; r < kSplitR; ++r)
+        acc[r] += (static_cast<double>(s[r].x) + static_cast<double>(s[r].y)) +
+                  (static_cast<double>(l[r].x) + static_cast<double>(l[r].y) -
+                   0.5 * static_cast<double>(k[r].x + k[r].y));
+    }
+    if (diag)
+#pragma unroll
+      for (int r = 0; r < kSplitR; ++r) acc[r] *= 0.5;
+  }
+  double v = 0.0;
+#pragma unroll
+  for (int r = 0; r < kSplitR; ++r) v += mi[r] * acc[r];
+  if (!kMass) v *= static_cast<double>(pos[pair_index(sd.offset, 3)]);  // the common m_j
+  const double total = block_sum(-G * v, sh);
+  if (tid == 0) *out = total;
+}
+
+// ---- potential, FP64 pairs ----------------------------------------------------------
+// blockIdx.x: i-tile tiles[x] = (system, tile); blockIdx.y: one of gridDim.y spans of the
+// j-tiles from it to the end of the system (a small system has few i-tiles: one CTA each
+// left 3,000 particles at 3.6 ms).  Writes its part of -G * sum_i m_i sum_{j>i} m_j /
+// sqrt(r^2 + eps), zero where the split kernel does the system (`split`: it is launched).
+constexpr int kPotThreads = 128;
+
+__global__ void __launch_bounds__(kPotThreads) potential_kernel(
+    const float* __restrict__ pos, const SystemDesc* __restrict__ sys,
+    const int2* __restrict__ tiles, const int* __restrict__ wide, bool split, float eps2, double G,
+    double* __restrict__ partial) {
+  __shared__ double sh[kPotThreads];
+  __shared__ double tj[4][kPotThreads];
+  const int2 tl = tiles[blockIdx.x];
+  const SystemDesc sd = sys[tl.x];
+  const int njt = (sd.n + kPotThreads - 1) / kPotThreads - tl.y;
+  const int t0 = tl.y + static_cast<int>(static_cast<int64_t>(njt) * blockIdx.y / gridDim.y);
+  const int t1 = tl.y + static_cast<int>(static_cast<int64_t>(njt) * (blockIdx.y + 1) / gridDim.y);
+  double* out = partial + static_cast<int64_t>(blockIdx.y) * gridDim.x + blockIdx.x;
+  if (t0 == t1 || (split && !*wide && sd.n >= kSplitMin)) {
+    if (threadIdx.x == 0) *out = 0.0;
+    return;
+  }
+  const int li = tl.y * kPotThreads + threadIdx.x;
   const bool valid = li < sd.n;
   const int64_t gi = sd.offset + (valid ? li : 0);
   const double xi = pos[pair_index(gi, 0)], yi = pos[pair_index(gi, 1)],
                zi = pos[pair_index(gi, 2)], mi = pos[pair_index(gi, 3)];
+  const double e2 = eps2;
   double sum = 0.0;
-  for (int j0 = tl.y * kDiagThreads; j0 < sd.n; j0 += kDiagThreads) {
-    const int lj = j0 + threadIdx.x;
-    if (lj < sd.n) {
-      const int64_t gj = sd.offset + lj;
-      tj[threadIdx.x] = make_float4(pos[pair_index(gj, 0)], pos[pair_index(gj, 1)],
-                                    pos[pair_index(gj, 2)], pos[pair_index(gj, 3)]);
-    } else {
-      tj[threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int t = t0; t < t1; ++t) {
+    const int j0 = t * kPotThreads;
+    const int cnt = min(kPotThreads, sd.n - j0);
+    __syncthreads();
+    if (static_cast<int>(threadIdx.x) < cnt) {
+      const int64_t gj = sd.offset + j0 + threadIdx.x;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tj[c][threadIdx.x] = pos[pair_index(gj, c)];
     }
     __syncthreads();
-    const int cnt = min(kDiagThreads, sd.n - j0);
-    if (valid) {
-      for (int k = 0; k < cnt; ++k) {
-        if (j0 + k <= li) continue;
-        const float4 q = tj[k];
-        const double dx = q.x - xi, dy = q.y - yi, dz = q.z - zi;
-        const double d2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, static_cast<double>(eps2))));
-        sum = fma(static_cast<double>(q.w), rsqrt(d2), sum);
-      }
+    if (!valid) continue;
+    for (int k = t == tl.y ? static_cast<int>(threadIdx.x) + 1 : 0; k < cnt; ++k) {
+      const double dx = tj[0][k] - xi, dy = tj[1][k] - yi, dz = tj[2][k] - zi;
+      const double d2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, e2)));
+      sum = fma(tj[3][k], rsqrt(d2), sum);
     }
-    __syncthreads();
   }
   const double s = block_sum(valid ? -G * mi * sum : 0.0, sh);
-  if (threadIdx.x == 0) partial[blockIdx.x] = s;
+  if (threadIdx.x == 0) *out = s;
 }
 
-// Sum `count` partial records of `stride` doubles, column by column in index order.
-__global__ void reduce_partials_kernel(const double* __restrict__ partial, int count, int stride,
-                                       int ncols, double* __restrict__ out) {
-  const int c = threadIdx.x;
-  if (c >= ncols) return;
+// out[0]: the sum of the potential's parts; out[1 + c]: column c of the moments.  One
+// CTA each; a thread adds a stride of the parts in order, then a fixed tree.
+__global__ void __launch_bounds__(kDiagThreads) reduce_partials_kernel(
+    const double* __restrict__ moments, int mblocks, const double* __restrict__ potential,
+    int64_t parts, double* __restrict__ out) {
+  __shared__ double sh[kDiagThreads];
+  const int c = static_cast<int>(blockIdx.x) - 1;
+  const double* src = c < 0 ? potential : moments + c;
+  const int64_t count = c < 0 ? parts : mblocks, stride = c < 0 ? 1 : kDiagVals;
   double s = 0.0;
-  for (int b = 0; b < count; ++b) s += partial[static_cast<int64_t>(b) * stride + c];
-  out[c] = s;
+  for (int64_t b = threadIdx.x; b < count; b += kDiagThreads) s += src[b * stride];
+  s = block_sum(s, sh);
+  if (threadIdx.x == 0) out[blockIdx.x] = s;
 }
 
 // FP64 acceleration of row r: G * sum_{j != i} m_j (x_j - x_i) / (|.|^2 + eps)^(3/2).
@@ -144,44 +412,73 @@ __global__ void fp64_rows_kernel(const float* __restrict__ pos, const SystemDesc
 
 cudaError_t launch_diagnostics(const float* pos, const float4* vel, const SystemDesc* sys_d,
                                const SystemDesc* sys_h, int32_t first_sys, int32_t num_sys,
-                               float eps2, float G, bool, double* out10, DiagScratch& scratch,
-                               cudaStream_t stream) {
-  // Moments.
+                               float eps2, float G, bool per_pair_mass, int sms, double* out10,
+                               DiagScratch& scratch, cudaStream_t stream) {
   const int64_t first = sys_h[first_sys].offset;
   const int64_t last = sys_h[first_sys + num_sys - 1].offset + sys_h[first_sys + num_sys - 1].npad;
-  const int mblocks = 1024;
-  cudaError_t e = cudaSuccess;
-  // Potential tiles.
-  int64_t ntiles = 0;
-  for (int32_t s = first_sys; s < first_sys + num_sys; ++s)
-    ntiles += (sys_h[s].n + kDiagThreads - 1) / kDiagThreads;
-  const int64_t need = static_cast<int64_t>(mblocks) * kDiagVals + ntiles + 2 * ntiles + 16;
-  if (scratch.max_blocks < need) {
-    if (scratch.partial) cudaFree(scratch.partial);
-    scratch.partial = nullptr;
-    scratch.max_blocks = 0;
-    e = cudaMalloc(&scratch.partial, need * sizeof(double));
+  const int mblocks = static_cast<int>(
+      std::min<int64_t>(1024, (last - first + kDiagThreads - 1) / kDiagThreads));
+  // i-tiles of the FP64 kernel, and of the split one over the systems large enough.
+  if (scratch.first_sys != first_sys || scratch.num_sys != num_sys || !scratch.partial) {
+    std::vector<int2> tiles;
+    auto list = [&](int bi, int min_n) {
+      const size_t n0 = tiles.size();
+      for (int32_t s = first_sys; s < first_sys + num_sys; ++s)
+        for (int t = 0; sys_h[s].n >= min_n && t < (sys_h[s].n + bi - 1) / bi; ++t)
+          tiles.push_back(make_int2(s, t));
+      return static_cast<int64_t>(tiles.size() - n0);
+    };
+    const int64_t nfp64 = list(kPotThreads, 1);
+    const int64_t nsplit = list(kSplitBI, kSplitMin);
+    // Spans per i-tile: enough CTAs per SM that the triangle's uneven shares even out.
+    auto spans_of = [&](int64_t tiles_n, int per_sm) {
+      return static_cast<int32_t>(
+          std::max<int64_t>(1, std::min<int64_t>(64, per_sm * sms / std::max<int64_t>(1, tiles_n))));
+    };
+    scratch.spans = spans_of(nsplit, 64);
+    scratch.fp64_spans = spans_of(nfp64, 16);
+    const int64_t parts = nfp64 * scratch.fp64_spans + nsplit * scratch.spans;
+    const int64_t need = static_cast<int64_t>(mblocks) * kDiagVals + parts + nfp64 + nsplit + 1;
+    scratch.num_sys = 0;
+    if (scratch.cap < need) {
+      if (scratch.partial) cudaFree(scratch.partial);
+      scratch.partial = nullptr;
+      scratch.cap = 0;
+      const cudaError_t e = cudaMalloc(&scratch.partial, need * sizeof(double));
+      if (e != cudaSuccess) return e;
+      scratch.cap = need;
+    }
+    scratch.nfp64 = nfp64;
+    scratch.nsplit = nsplit;
+    // The list is pageable: the copy has read it before it returns.
+    const cudaError_t e =
+        cudaMemcpyAsync(scratch.partial + mblocks * kDiagVals + parts, tiles.data(),
+                        tiles.size() * sizeof(int2), cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return e;
-    scratch.max_blocks = static_cast<int32_t>(need);
+    scratch.first_sys = first_sys;
+    scratch.num_sys = num_sys;
   }
+  const int64_t fp64_parts = scratch.nfp64 * scratch.fp64_spans;
+  const int64_t parts = fp64_parts + scratch.nsplit * scratch.spans;
   double* mom_part = scratch.partial;
-  double* pot_part = scratch.partial + static_cast<int64_t>(mblocks) * kDiagVals;
-  int2* tiles_d = reinterpret_cast<int2*>(pot_part + ntiles);
-  int2* tiles_h = nullptr;
-  e = cudaMallocHost(&tiles_h, ntiles * sizeof(int2));
+  double* pot_part = mom_part + static_cast<int64_t>(mblocks) * kDiagVals;
+  const int2* tiles = reinterpret_cast<const int2*>(pot_part + parts);
+  int* wide = reinterpret_cast<int*>(pot_part + parts + scratch.nfp64 + scratch.nsplit);
+  const bool split = scratch.nsplit > 0 && eps2 >= kSplitEps;
+  cudaError_t e = cudaMemsetAsync(wide, 0, sizeof(int), stream);
   if (e != cudaSuccess) return e;
-  int64_t k = 0;
-  for (int32_t s = first_sys; s < first_sys + num_sys; ++s)
-    for (int t = 0; t < (sys_h[s].n + kDiagThreads - 1) / kDiagThreads; ++t) tiles_h[k++] = {s, t};
-  e = cudaMemcpyAsync(tiles_d, tiles_h, ntiles * sizeof(int2), cudaMemcpyHostToDevice, stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-  cudaFreeHost(tiles_h);
-  if (e != cudaSuccess) return e;
-  moments_kernel<<<mblocks, kDiagThreads, 0, stream>>>(pos, vel, first, last, mom_part);
-  potential_kernel<<<static_cast<unsigned>(ntiles), kDiagThreads, 0, stream>>>(pos, sys_d, tiles_d,
-                                                                             eps2, G, pot_part);
-  reduce_partials_kernel<<<1, 32, 0, stream>>>(mom_part, mblocks, kDiagVals, 9, out10 + 1);
-  reduce_partials_kernel<<<1, 32, 0, stream>>>(pot_part, static_cast<int>(ntiles), 1, 1, out10);
+  moments_kernel<<<mblocks, kDiagThreads, 0, stream>>>(pos, vel, first, last, mom_part, wide);
+  potential_kernel<<<dim3(static_cast<unsigned>(scratch.nfp64), scratch.fp64_spans), kPotThreads, 0,
+                     stream>>>(
+      pos, sys_d, tiles, wide, split, eps2, G, pot_part);
+  if (split) {
+    const dim3 grid(static_cast<unsigned>(scratch.nsplit), scratch.spans);
+    auto kernel = per_pair_mass ? potential_split_kernel<true> : potential_split_kernel<false>;
+    kernel<<<grid, kSplitThreads, 0, stream>>>(pos, sys_d, tiles + scratch.nfp64, wide, eps2, G,
+                                               pot_part + fp64_parts);
+  }
+  reduce_partials_kernel<<<10, kDiagThreads, 0, stream>>>(mom_part, mblocks, pot_part,
+                                                          split ? parts : fp64_parts, out10);
   return cudaGetLastError();
 }
 

@@ -86,12 +86,15 @@ cudaError_t launch_fill_padding(float* pos, float4* vel, int64_t n_pad_total, cu
 
 // ---- FP64 diagnostics (diag_kernels.cu) ---------------------------------------------
 struct DiagScratch {
-  double* partial;   // [max_blocks][10]
-  int32_t max_blocks;
+  double* partial = nullptr;  // moments, potential parts, tile lists, range flag
+  int64_t cap = 0;            // doubles
+  int32_t first_sys = 0, num_sys = 0;  // the systems the tile lists are for
+  int64_t nfp64 = 0, nsplit = 0;       // tiles of the FP64 and of the split kernel
+  int32_t spans = 1, fp64_spans = 1;   // parts their j-tiles are cut into
 };
 cudaError_t launch_diagnostics(const float* pos, const float4* vel, const SystemDesc* sys_d,
                                const SystemDesc* sys_h, int32_t first_sys, int32_t num_sys,
-                               float eps2, float G, bool per_pair_mass, double* out10,
+                               float eps2, float G, bool per_pair_mass, int sms, double* out10,
                                DiagScratch& scratch, cudaStream_t stream);
 cudaError_t launch_fp64_rows(const float* pos, const SystemDesc* sys_d, const int64_t* rows_dev,
                              const int32_t* row_sys_dev, int64_t count, float eps2, float G,

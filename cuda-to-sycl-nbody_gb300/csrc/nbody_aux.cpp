@@ -108,8 +108,8 @@ int nb_sim_diagnostics(nb_sim* s, int32_t system, nb_diagnostics* out) {
   const int32_t first = system < 0 ? 0 : system;
   const int32_t count = system < 0 ? nsys : 1;
   NB_CUDA(launch_diagnostics(s->pos_d[s->cur], s->vel_d, s->sys_d, s->sys_h.data(), first, count,
-                             s->params.dist_eps, s->params.G, s->per_pair_mass, s->diag_out_d,
-                             s->diag, s->stream));
+                             s->params.dist_eps, s->params.G, s->per_pair_mass, s->sms,
+                             s->diag_out_d, s->diag, s->stream));
   double h[10];
   NB_CUDA(cudaMemcpyAsync(h, s->diag_out_d, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
   NB_CUDA(cudaStreamSynchronize(s->stream));
