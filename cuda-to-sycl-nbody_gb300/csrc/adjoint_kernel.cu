@@ -152,7 +152,6 @@ __global__ void __launch_bounds__(32, 8) adjoint_pair_kernel(const AdjointArgs a
   const int lane = threadIdx.x;
   const float2 e2 = make_float2(a.eps2, a.eps2);
   const float2 zero = make_float2(0.f, 0.f);
-  pdl_trigger();
   SymSegment sg = a.segs[blockIdx.x];
   pdl_wait();
   for (int next = blockIdx.x; next >= 0;) {
@@ -231,6 +230,7 @@ __global__ void __launch_bounds__(32, 8) adjoint_pair_kernel(const AdjointArgs a
         folded = true;
       }
     }
+    if (next < 0) pdl_trigger();
     float4* part = a.partials + static_cast<int64_t>(sg.slot) * BI;
 #pragma unroll
     for (int r = 0; r < P; ++r) {

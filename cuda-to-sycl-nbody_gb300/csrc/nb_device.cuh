@@ -10,7 +10,11 @@ namespace nbg {
 // Programmatic dependent launch: a kernel launched with launch_dependent may start
 // while its predecessor in the stream still runs.  pdl_wait returns when the
 // predecessor has finished and its writes are visible; pdl_trigger lets the successor
-// start (once every CTA has called it or left).
+// start (once every CTA has called it or left).  Kernels trigger near their end: a
+// successor whose CTAs become resident earlier finds free places only on the SMs that
+// have little or no work, and its CTAs crowd there (reference order, 16,384 particles on
+// 128 CTAs: 192 us per step triggered at the start, 153 near the end; symmetric, 2,048
+// particles: 8.5 and 7.4).
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

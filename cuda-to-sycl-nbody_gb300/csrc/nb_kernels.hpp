@@ -54,14 +54,17 @@ cudaError_t launch_predicated(const ForceArgs& a, const SystemDesc& sd, int32_t 
 // (ForceArgs segs / seg_begin / fix) of reference_order_shape(index) tiles; split
 // i-tiles hand their running sums over through `partials` and `counters`.  `dup` is
 // the duplicated j-layout of a.pos (2 float4 per padded particle) written by
-// launch_reference_order_dup.  The launch is cooperative: grid <= blocks per SM x SMs.
+// launch_reference_order_dup, for the shapes that need it.  With split i-tiles the
+// launch is cooperative: grid <= blocks per SM x SMs.
 int reference_order_num_shapes();
 KernelShape reference_order_shape(int index);  // threads, i-particles per thread, j-tile, stages
 cudaError_t reference_order_blocks_per_sm(int index, bool predicated, int* blocks);
 cudaError_t launch_reference_order_dup(const float* pos, int64_t n_pad_total, float4* dup,
                                        cudaStream_t stream);
 cudaError_t launch_reference_order(int index, bool predicated, const ForceArgs& a,
-                                   const float4* dup, int grid, cudaStream_t stream);
+                                   const float4* dup, int grid, bool split,
+                                   cudaStream_t stream);
+bool reference_order_needs_dup(int index);
 
 // ---- measured FP32 throughput (peak_probe.cu) ----------------------------------------
 // Time `repeats` launches (after one warm-up) of an FFMA2 loop over sms x blocks_per_sm

@@ -469,7 +469,7 @@ int launch_with(nb_sim* s, ForceArgs a, const WorkListDev& list) {
   if (w.cfg < 0) {
     // Sequential order: the duplicated layout of a.pos must have been written.
     NB_CUDA(launch_reference_order(-1 - w.cfg, s->params.calc_method == NB_PREDICATED, a,
-                                   s->ro_dup_d, w.grid, s->stream));
+                                   s->ro_dup_d, w.grid, w.split > 0, s->stream));
     return NB_OK;
   }
   NB_CUDA(launch_force(w.cfg, s->params.accumulator == NB_ACC_COMPENSATED, s->per_pair_mass,
@@ -487,10 +487,15 @@ int force_pass(nb_sim* s, float4* accel_out, int per_system) {
       NB_CUDA(launch_predicated(a, s->sys_h[k], k, s->stream));
   } else if (sequential_order_mode(s)) {
     if (s->per_pair_mass) return set_error(NB_ERR_INVALID_ARGUMENT, kReferenceOrderMassError);
-    NB_TRY(ensure_reference_order_dup(s));
-    NB_CUDA(launch_reference_order_dup(a.pos, s->n_pad, s->ro_dup_d, s->stream));
+    if (per_system) NB_TRY(build_per_system_worklists(s, per_system));
+    bool dup = !per_system && reference_order_needs_dup(-1 - s->ro_wl.cfg);
+    if (per_system)
+      for (const auto& w : s->wl_sys) dup = dup || reference_order_needs_dup(-1 - w.cfg);
+    if (dup) {
+      NB_TRY(ensure_reference_order_dup(s));
+      NB_CUDA(launch_reference_order_dup(a.pos, s->n_pad, s->ro_dup_d, s->stream));
+    }
     if (per_system) {
-      NB_TRY(build_per_system_worklists(s, per_system));
       for (const auto& w : s->wl_sys) NB_TRY(launch_with(s, a, w));
     } else {
       NB_TRY(launch_with(s, a, s->ro_wl));
@@ -596,15 +601,30 @@ static int64_t reference_order_tiles(const nb_sim* s, int shape, int32_t first, 
   return tiles;
 }
 
-// Grid of the reference-order kernel: one CTA per i-tile while every CTA fits
-// on the GPU at once, else the occupancy limit on every SM with the stream-K work
-// list.  A CTA's share is then at least one whole i-tile, so a hand-over chain is
-// never longer than two parts (a particle's sum is sequential: a longer chain
-// would only run its parts one after another).
+// Grid of the reference-order kernel, at most one CTA per i-tile: a CTA's share is then
+// at least one whole i-tile, so a hand-over chain is never longer than two parts (a
+// particle's sum is sequential: a longer chain would only run its parts one after
+// another).  The last shape's CTAs are one warp per scheduler, and an SM takes 18.75,
+// 32.4, 48.4, ... cycles per j-particle for one, two, three, ... of them (N = 19,456,
+// 38,912, 58,368, where that many i-tiles fill it): where i-tiles are left over, fewer
+// CTAs that share them can be faster than one more on some SMs (25,600: 152 CTAs 316 us
+// per step, 200 414).  The others: one CTA per i-tile while all fit on the GPU.
 static int reference_order_grid(nb_sim* s, int shape, int32_t first, int32_t count) {
   const int64_t tiles = reference_order_tiles(s, shape, first, count);
-  return static_cast<int>(std::max<int64_t>(
-      1, std::min<int64_t>(tiles, max_grid_for(s, -1 - shape))));
+  const int64_t most = std::max<int64_t>(1, std::min<int64_t>(tiles, max_grid_for(s, -1 - shape)));
+  if (shape + 1 != reference_order_num_shapes()) return static_cast<int>(most);
+  int64_t best = most;
+  double best_time = DBL_MAX;
+  for (int64_t k = 1; (k - 1) * s->sms < most; ++k) {
+    const int64_t grid = std::min<int64_t>(k * s->sms, most);
+    const double cycles = k == 1 ? 18.75 : k == 2 ? 32.4 : 16.13 * static_cast<double>(k);
+    const double time = cycles * std::max(1.0, static_cast<double>(tiles) / grid);
+    if (time < best_time) {
+      best_time = time;
+      best = grid;
+    }
+  }
+  return static_cast<int>(best);
 }
 
 // Default reference-order shape: the largest i-tiles that still fill the GPU --
@@ -720,7 +740,8 @@ static int create_impl(const nb_params* p, uint32_t num_systems, const uint32_t*
   if (sequential_order_mode(s)) {
     s->ro_shape = default_reference_order_for(s, 0, static_cast<int32_t>(s->sys_h.size()));
     if ((st = build_reference_order_worklist(s, s->ro_shape)) != NB_OK) return fail(st);
-    if ((st = ensure_reference_order_dup(s)) != NB_OK) return fail(st);
+    if (reference_order_needs_dup(s->ro_shape) && (st = ensure_reference_order_dup(s)) != NB_OK)
+      return fail(st);
   }
   if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) return fail(cuda_error(e, "create"));
   *out = s;

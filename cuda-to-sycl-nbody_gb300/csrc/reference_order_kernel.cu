@@ -32,6 +32,9 @@
 //     mbarrier or on a predecessor -- is bounded (2 s of %globaltimer); on
 //     timeout the CTA sets bit 0 of the error word, drains its own copies and
 //     exits.
+//   * Small systems take two j-particles, not two i-particles, in the packed registers
+//     (reference_order_jpair_kernel): roots on the packed pipe, and each thread's one
+//     particle adds its terms one by one.
 //   * Only the n real particles of a system are summed (no padding terms), as in
 //     the reference.
 #include <cuda_runtime.h>
@@ -386,16 +389,264 @@ __global__ void __launch_bounds__(THREADS, MINB) reference_order_kernel(
   }
 }
 
+// ---- two j-particles per packed register pair ------------------------------------------
+// One j-pair against the thread's R i-particles: the differences, the softened square
+// and the root of both pairs on the packed pipe, then each running sum takes its two
+// terms one after the other.  live1: the pair's second particle exists.
+template <bool kDiag, bool kPred>
+__device__ __forceinline__ void roj_step(const float4 A, const float4 B, float2 e2, float2 nx,
+                                         float2 ny, float2 nz, float3& f, int j, bool live1,
+                                         int li) {
+  const float2 rx = __fadd2_rn(make_float2(A.x, A.y), nx);
+  const float2 ry = __fadd2_rn(make_float2(A.z, A.w), ny);
+  const float2 rz = __fadd2_rn(make_float2(B.x, B.y), nz);
+  float2 d2 = __fmul2_rn(ry, ry);
+  d2 = __ffma2_rn(rx, rx, d2);
+  d2 = __ffma2_rn(rz, rz, d2);
+  d2 = __fadd2_rn(d2, e2);
+  float2 t = __fmul2_rn(d2, d2);
+  t = __fmul2_rn(t, d2);
+  const float2 inv = make_float2(rsqrtf(t.x), rsqrtf(t.y));
+  if (kPred) {
+    const float m0 = kDiag && j == li ? 1.f : 0.f, m1 = kDiag && j + 1 == li ? 1.f : 0.f;
+    const float2 px = __fmul2_rn(rx, inv), py = __fmul2_rn(ry, inv), pz = __fmul2_rn(rz, inv);
+    f.x = __fmaf_rn(px.x, m0, f.x);
+    f.y = __fmaf_rn(py.x, m0, f.y);
+    f.z = __fmaf_rn(pz.x, m0, f.z);
+    if (!kDiag || live1) {
+      f.x = __fmaf_rn(px.y, m1, f.x);
+      f.y = __fmaf_rn(py.y, m1, f.y);
+      f.z = __fmaf_rn(pz.y, m1, f.z);
+    }
+    return;
+  }
+  if (!kDiag || j != li) {
+    f.x = __fmaf_rn(rx.x, inv.x, f.x);
+    f.y = __fmaf_rn(ry.x, inv.x, f.y);
+    f.z = __fmaf_rn(rz.x, inv.x, f.z);
+  }
+  if (!kDiag || (live1 && j + 1 != li)) {
+    f.x = __fmaf_rn(rx.y, inv.y, f.x);
+    f.y = __fmaf_rn(ry.y, inv.y, f.y);
+    f.z = __fmaf_rn(rz.y, inv.y, f.z);
+  }
+}
+
+// U j-pairs' differences and roots.
+template <int U>
+struct RojBlock {
+  float2 rx[U], ry[U], rz[U], inv[U];
+  __device__ __forceinline__ void roots(const float4* __restrict__ tile, float2 nx, float2 ny,
+                                        float2 nz, float2 e2) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float4 A = tile[2 * u], B = tile[2 * u + 1];
+      rx[u] = __fadd2_rn(make_float2(A.x, A.y), nx);
+      ry[u] = __fadd2_rn(make_float2(A.z, A.w), ny);
+      rz[u] = __fadd2_rn(make_float2(B.x, B.y), nz);
+      float2 d2 = __fmul2_rn(ry[u], ry[u]);
+      d2 = __ffma2_rn(rx[u], rx[u], d2);
+      d2 = __ffma2_rn(rz[u], rz[u], d2);
+      d2 = __fadd2_rn(d2, e2);
+      float2 t = __fmul2_rn(d2, d2);
+      t = __fmul2_rn(t, d2);
+      inv[u] = make_float2(rsqrtf(t.x), rsqrtf(t.y));
+    }
+  }
+  __device__ __forceinline__ void add(float3& f) const {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      f.x = __fmaf_rn(rx[u].x, inv[u].x, f.x);
+      f.y = __fmaf_rn(ry[u].x, inv[u].x, f.y);
+      f.z = __fmaf_rn(rz[u].x, inv[u].x, f.z);
+      f.x = __fmaf_rn(rx[u].y, inv[u].y, f.x);
+      f.y = __fmaf_rn(ry[u].y, inv[u].y, f.y);
+      f.z = __fmaf_rn(rz[u].y, inv[u].y, f.z);
+    }
+  }
+};
+
+// j = j0 .. j0 + count - 1 of the staged tile, in order.  Without masks, blocks of U
+// j-pairs are pipelined: the next block's roots are independent of the sums the current
+// one is added to, which hides part of a lone warp's latencies (12,800 particles: 135 ->
+// 127 us per step).
+template <bool kDiag, bool kPred, int U>
+__device__ __forceinline__ void roj_tile(const float4* __restrict__ tile, int count, int j0,
+                                         float2 e2, float2 nx, float2 ny, float2 nz, float3& f,
+                                         int li) {
+  const int pairs = count >> 1;
+  int p = 0;
+  if constexpr (!kDiag && !kPred) {
+    if (pairs >= 2 * U) {
+      RojBlock<U> b0, b1;
+      b0.roots(tile, nx, ny, nz, e2);
+#pragma unroll 1
+      for (; p + 4 * U <= pairs; p += 2 * U) {
+        b1.roots(tile + 2 * (p + U), nx, ny, nz, e2);
+        b0.add(f);
+        b0.roots(tile + 2 * (p + 2 * U), nx, ny, nz, e2);
+        b1.add(f);
+      }
+      b1.roots(tile + 2 * (p + U), nx, ny, nz, e2);
+      b0.add(f);
+      b1.add(f);
+      p += 2 * U;
+    }
+  } else {
+#pragma unroll 1
+    for (; p + U <= pairs; p += U) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        roj_step<kDiag, kPred>(tile[2 * (p + u)], tile[2 * (p + u) + 1], e2, nx, ny, nz, f,
+                               j0 + 2 * (p + u), true, li);
+    }
+  }
+#pragma unroll 1
+  for (; 2 * p < count; ++p)  // what is left, and an odd system's last particle
+    roj_step<true, kPred>(tile[2 * p], tile[2 * p + 1], e2, nx, ny, nz, f, j0 + 2 * p,
+                          2 * p + 1 < count, li);
+}
+
+// The work list, the ring and the hand-overs are reference_order_kernel's; an i-tile is
+// one particle per thread, and j-tiles come from the positions themselves.
+template <int THREADS, int BJ, int U, bool kPred>
+__global__ void __launch_bounds__(THREADS, 1) reference_order_jpair_kernel(const ForceArgs a) {
+  constexpr int BI = THREADS;
+  static_assert(BI % kPadQuantum == 0, "i-tiles must hold whole padding quanta");
+  extern __shared__ __align__(128) float4 ring_smem[];  // [kRoStages][BJ]
+  auto ring = [&](uint32_t slot) { return ring_smem + slot * BJ; };
+  __shared__ __align__(8) uint64_t full_bar[kRoStages];
+  __shared__ int s_bail;
+  const int tid = threadIdx.x;
+  const int seg_lo = a.seg_begin[blockIdx.x];
+  const int seg_hi = a.seg_begin[blockIdx.x + 1];
+  if (tid == 0) {
+#pragma unroll
+    for (int s = 0; s < kRoStages; ++s) ro_mbar_init(&full_bar[s], 1);
+    ro_fence_mbar_init();
+    s_bail = 0;
+  }
+  __syncthreads();
+  pdl_wait();
+  if (seg_lo >= seg_hi) return;
+  int p_seg = seg_hi - 1;
+  int p_jt = a.segs[p_seg].jt0;
+  uint32_t issued = 0;
+  auto produce = [&]() {
+    if (p_seg < seg_lo) return;
+    const Segment& sg = a.segs[p_seg];
+    const SystemDesc& sd = a.sys[sg.sys];
+    const int count = min(BJ, sd.n - p_jt * BJ);
+    const int64_t first = sd.offset + static_cast<int64_t>(p_jt) * BJ;
+    const uint32_t slot = issued % kRoStages;
+    const uint32_t bytes = static_cast<uint32_t>((count + 1) / 2) * 32u;  // whole pair records
+    if (!(a.inject == kInjectSkipFirstTile && issued == 0)) {
+      ro_fence_proxy_async();
+      ro_arrive_expect_tx(&full_bar[slot], bytes);
+      ro_bulk_g2s(ring(slot), a.pos + 4 * first, bytes, &full_bar[slot]);
+    }
+    ++issued;
+    if (++p_jt >= sg.jt1) {
+      --p_seg;
+      if (p_seg >= seg_lo) p_jt = a.segs[p_seg].jt0;
+    }
+  };
+  if (tid == 0) {
+#pragma unroll
+    for (int k = 0; k < kRoStages - 1; ++k) produce();
+  }
+  const float2 e2 = make_float2(a.eps2, a.eps2);
+  uint32_t consumed = 0;
+  auto bail = [&]() {
+    if (tid == 0) {
+      atomicOr(a.err, 1);
+      for (uint32_t k = consumed; k < issued; ++k)
+        (void)ro_wait(&full_bar[k % kRoStages], (k / kRoStages) & 1u);
+    }
+  };
+  for (int sgi = seg_hi - 1; sgi >= seg_lo; --sgi) {
+    const Segment sg = a.segs[sgi];
+    const SystemDesc sd = a.sys[sg.sys];
+    const int ibase = sd.shard_first + sg.itile * BI;
+    const int iend = shard_end(sd);
+    const bool split = sg.fix >= 0;
+    const Fixup fx = split ? a.fix[sg.fix] : Fixup{1, 0};
+    float4* slots = a.partials + static_cast<int64_t>(fx.slot0) * BI;
+    const int li = ibase + tid;
+    const int64_t g = sd.offset + min(li, sd.n - 1);
+    const float x = a.pos[pair_index(g, 0)], y = a.pos[pair_index(g, 1)],
+                z = a.pos[pair_index(g, 2)];
+    const float2 nx = make_float2(-x, -x), ny = make_float2(-y, -y), nz = make_float2(-z, -z);
+    float3 f = make_float3(0.f, 0.f, 0.f);
+    if (split && sg.part > 0) {
+      if (tid == 0 && !ro_wait_counter(&a.counters[sg.fix], sg.part)) s_bail = 1;
+      __syncthreads();
+      if (s_bail) {
+        bail();
+        return;
+      }
+      const float4* in = slots + static_cast<int64_t>(sg.part - 1) * BI;
+      const float4 u = __ldcg(&in[tid]);
+      f = make_float3(u.x, u.y, u.z);
+    }
+    bool timed_out = false;
+    for (int jt = sg.jt0; jt < sg.jt1; ++jt, ++consumed) {
+      if (tid == 0) produce();
+      const uint32_t slot = consumed % kRoStages;
+      if (!ro_wait(&full_bar[slot], (consumed / kRoStages) & 1u)) timed_out = true;
+      const int j0 = jt * BJ;
+      const int count = min(BJ, sd.n - j0);
+      // The warp's own particles within the tile take the masked loop; before and after
+      // them nothing is left out.
+      const int own0 = min(max(ibase + (tid & ~31) - j0, 0), count);
+      const int own1 = min(max(ibase + (tid & ~31) + 32 - j0, 0), count);
+      if (!timed_out) {
+#pragma unroll 1
+        for (int part = 0; part < 3; ++part) {
+          const int from = part == 0 ? 0 : part == 1 ? own0 : own1;
+          const int to = part == 0 ? own0 : part == 1 ? own1 : count;
+          if (from >= to) continue;
+          const float4* at = ring(slot) + from;
+          if (part == 1)
+            roj_tile<true, kPred, 4>(at, to - from, j0 + from, e2, nx, ny, nz, f, li);
+          else
+            roj_tile<false, kPred, U>(at, to - from, j0 + from, e2, nx, ny, nz, f, li);
+        }
+      }
+      if (__syncthreads_or(timed_out)) {
+        bail();
+        return;
+      }
+    }
+    if (split && sg.part < fx.nparts - 1) {
+      float4* out = slots + static_cast<int64_t>(sg.part) * BI;
+      __stcg(&out[tid], make_float4(f.x, f.y, f.z, 0.f));
+      __threadfence();
+      __syncthreads();
+      if (tid == 0 && a.inject != kInjectWithholdHandOver) atomicAdd(&a.counters[sg.fix], 1);
+      continue;
+    }
+    if (sgi == seg_lo) pdl_trigger();
+    if (split && tid == 0) a.counters[sg.fix] = 0;
+    if (li < iend) finish_particle(a, sd, sd.offset + li, f.x, f.y, f.z, x, y, z);
+  }
+}
+
 struct RoShapeEntry {
   int threads;
-  int pairs;
+  int r;  // i-particles per thread
   int bj;
   void (*kernel[2])(const ForceArgs, const float4*);  // [BRANCH, PREDICATED]
+  void (*jpair[2])(const ForceArgs);
+  int stage_bytes() const { return bj * (jpair[0] ? 16 : 32); }
 };
 
 #define RO_SHAPE(T, P, BJ, U, B)                                                   \
-  {T, P, BJ, {reference_order_kernel<T, P, BJ, U, B, false>,                       \
-              reference_order_kernel<T, P, BJ, U, B, true>}}
+  {T, 2 * P, BJ, {reference_order_kernel<T, P, BJ, U, B, false>,                   \
+                  reference_order_kernel<T, P, BJ, U, B, true>}, {nullptr, nullptr}}
+#define RO_JPAIR(T, BJ, U)                                                            \
+  {T, 1, BJ, {nullptr, nullptr}, {reference_order_jpair_kernel<T, BJ, U, false>,      \
+                                  reference_order_jpair_kernel<T, BJ, U, true>}}
 // Largest i-tiles first; the default for a system is the first shape whose i-tiles
 // give every SM two CTAs (one where only one fits), else the last.  Measured
 // (thin disk, ms per step; every variant gave the same bits):
@@ -410,20 +661,26 @@ struct RoShapeEntry {
 //     number of independent j-steps a thread has in flight: one i-pair per thread,
 //     32 j-steps per unrolled block (128 registers).  At 196,608: 256 x 1 x 1024
 //     14.2 ms (384 x 2 16.4, 128 x 2 x 256 with 4 j-steps 17.7); at 131,072:
-//     128 x 1 x 1024 6.61 (64 x 1 x 1024 6.98, 384 x 2 10.9); at 65,536:
-//     64 x 1 x 1024 1.76 (128 x 2 x 256 2.25); at 25,600: 0.418 (64 x 1 x 256 with
-//     4 j-steps 0.605); at 2,048: 0.045 (0.057).  2048-particle j-tiles (one CTA
-//     per SM) halve the rate of the 64-thread shape.
+//     128 x 1 x 1024 6.61 (384 x 2 10.9).  2048-particle j-tiles (one CTA per SM)
+//     halve the rate of small shapes.
+//   * Below 77,824 even those leave schedulers idle: one particle per thread has twice
+//     the warps, and with two j-particles in the packed registers no more issue slots
+//     per pair (the j-pair form above).  us per step, against 64 threads with an i-pair
+//     each: 333 particles 6.2 (16.4), 2,048 21.1 (47.1), 12,800 119 (217), 25,600 316
+//     (420), 65,536 1,766 (1,766); 77,824 2,482 (128 x 1 x 1024 2,338).  Larger systems
+//     too are faster with i-pairs: 25.0 against 24.6 ms at 262,144, 400 against 391 at 1M
+//     for the best of eleven j-pair shapes.  Four lanes per particle, exchanging roots
+//     by shuffles, are bound by the shuffles: 12,800 230 us.
 const RoShapeEntry kRoShapes[] = {
     RO_SHAPE(384, 2, 1024, 4, 1),
     RO_SHAPE(256, 1, 1024, 32, 1),
     RO_SHAPE(128, 1, 1024, 32, 1),
-    RO_SHAPE(64, 1, 1024, 32, 1),
+    RO_JPAIR(128, 512, 16),
 };
 constexpr int kNumRoShapes = sizeof(kRoShapes) / sizeof(kRoShapes[0]);
 
 size_t ro_smem_bytes(const RoShapeEntry& e) {
-  return static_cast<size_t>(kRoStages) * e.bj * 32;
+  return static_cast<size_t>(kRoStages) * e.stage_bytes();
 }
 
 // Rings of 48 KB or more opt in to the larger dynamic shared memory, once per
@@ -438,7 +695,9 @@ cudaError_t ro_smem_opt_in(int index) {
   const uint64_t bit = dev >= 0 && dev < 64 ? uint64_t{1} << dev : 0;
   if (bit != 0 && (opted[index].load(std::memory_order_acquire) & bit) != 0) return cudaSuccess;
   for (int v = 0; v < 2 && err == cudaSuccess; ++v)
-    err = cudaFuncSetAttribute(e.kernel[v], cudaFuncAttributeMaxDynamicSharedMemorySize,
+    err = cudaFuncSetAttribute(e.jpair[v] ? reinterpret_cast<const void*>(e.jpair[v])
+                                          : reinterpret_cast<const void*>(e.kernel[v]),
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(ro_smem_bytes(e)));
   if (err == cudaSuccess && bit != 0) opted[index].fetch_or(bit, std::memory_order_release);
   return err;
@@ -450,15 +709,17 @@ int reference_order_num_shapes() { return kNumRoShapes; }
 
 KernelShape reference_order_shape(int index) {
   const RoShapeEntry& e = kRoShapes[index];
-  return KernelShape{e.threads, 2 * e.pairs, e.bj, kRoStages};
+  return KernelShape{e.threads, e.r, e.bj, kRoStages};
 }
 
 cudaError_t reference_order_blocks_per_sm(int index, bool predicated, int* blocks) {
   const RoShapeEntry& e = kRoShapes[index];
   const cudaError_t err = ro_smem_opt_in(index);
   if (err != cudaSuccess) return err;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, e.kernel[predicated], e.threads,
-                                                       ro_smem_bytes(e));
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      blocks, e.jpair[predicated] ? reinterpret_cast<const void*>(e.jpair[predicated])
+                                  : reinterpret_cast<const void*>(e.kernel[predicated]),
+      e.threads, ro_smem_bytes(e));
 }
 
 cudaError_t launch_reference_order_dup(const float* pos, int64_t n_pad_total, float4* dup,
@@ -471,11 +732,16 @@ cudaError_t launch_reference_order_dup(const float* pos, int64_t n_pad_total, fl
   return cudaGetLastError();
 }
 
+bool reference_order_needs_dup(int index) { return kRoShapes[index].jpair[0] == nullptr; }
+
 cudaError_t launch_reference_order(int index, bool predicated, const ForceArgs& a,
-                                   const float4* dup, int grid, cudaStream_t stream) {
+                                   const float4* dup, int grid, bool split, cudaStream_t stream) {
   const RoShapeEntry& e = kRoShapes[index];
   const cudaError_t err = ro_smem_opt_in(index);
   if (err != cudaSuccess) return err;
+  if (!split && e.jpair[predicated])  // no CTA waits for another
+    return launch_dependent(e.jpair[predicated], dim3(grid), e.threads, ro_smem_bytes(e), stream,
+                            a);
   // Cooperative: every CTA is resident, so a CTA waiting for its predecessor's
   // hand-over always waits on a running CTA.
   cudaLaunchAttribute attr[1];
@@ -488,6 +754,7 @@ cudaError_t launch_reference_order(int index, bool predicated, const ForceArgs& 
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (e.jpair[predicated]) return cudaLaunchKernelEx(&cfg, e.jpair[predicated], a);
   return cudaLaunchKernelEx(&cfg, e.kernel[predicated], a, dup);
 }
 

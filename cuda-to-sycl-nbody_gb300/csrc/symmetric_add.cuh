@@ -68,7 +68,6 @@ __device__ __forceinline__ bool add_terms(const AddTerms& a, int bi, Early& earl
   const int sys0 = t - tile.itile;  // the system's first i-tile
   const int64_t row_first = a.tiles[max(sys0, a.tile0)].row;
   early.lists(tile.sys);
-  pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x % kAddLanes, group = threadIdx.x / kAddLanes;
   const int idx = blockIdx.y * kAddLanes + lane;
@@ -131,6 +130,7 @@ __device__ __forceinline__ bool add_terms(const AddTerms& a, int bi, Early& earl
       if (kComp) q[0] += l[u].x, q[1] += l[u].y, q[2] += l[u].z;
     }
   }
+  pdl_trigger();
   // Group sums in order, each as its sum and what is still to be added to it.
 #pragma unroll
   for (int c = 0; c < 3; ++c) {

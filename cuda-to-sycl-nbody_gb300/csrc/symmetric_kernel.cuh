@@ -183,7 +183,6 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) symmetric_kernel(const SymArg
   int par = 0;  // buffer of the next j-tile's j-side sums
 
   // The lists are older than the predecessor's launch; the state is not.
-  pdl_trigger();
   SymSegment sg = a.segs[blockIdx.x];
   pdl_wait();
   for (int next = blockIdx.x; next >= 0;) {
@@ -285,6 +284,7 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) symmetric_kernel(const SymArg
       }
     }
 
+    if (next < 0) pdl_trigger();
     // The segment's i-side sums: (hi, lo) records, or the plain sums.
     constexpr int kRec = kComp ? 2 : 1;
     float4* part = a.f.partials + static_cast<int64_t>(sg.slot) * BI * kRec;
