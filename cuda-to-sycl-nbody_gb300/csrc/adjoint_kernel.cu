@@ -154,9 +154,9 @@ __global__ void __launch_bounds__(32, 8) adjoint_pair_kernel(const AdjointArgs a
   const float2 zero = make_float2(0.f, 0.f);
   SymSegment sg = a.segs[blockIdx.x];
   pdl_wait();
-  for (int next = blockIdx.x; next >= 0;) {
-    if (next != static_cast<int>(blockIdx.x)) sg = a.segs[next];
-    next = sg.next;
+  for (bool more = true; more;) {
+    const int next = sg.next;
+    more = next > 0;
     const int ibase = sg.itile * BI;
     const float* pos = a.pos + 4 * sg.offset;
     AdjI<P> q;
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(32, 8) adjoint_pair_kernel(const AdjointArgs a
         folded = true;
       }
     }
-    if (next < 0) pdl_trigger();
+    if (!more) pdl_trigger();
     float4* part = a.partials + static_cast<int64_t>(sg.slot) * BI;
 #pragma unroll
     for (int r = 0; r < P; ++r) {
@@ -240,6 +240,7 @@ __global__ void __launch_bounds__(32, 8) adjoint_pair_kernel(const AdjointArgs a
       part[64 * r + lane] = make_float4(sx.x, sy.x, sz.x, 0.f);
       part[64 * r + 32 + lane] = make_float4(sx.y, sy.y, sz.y, 0.f);
     }
+    if (more) sg = a.segs[next - 1];
   }
 }
 

@@ -28,7 +28,7 @@ struct SymArgs {
   const SymTile* tiles;      // every i-tile
   float* rows;               // [3][plane] j-side sums
   int64_t plane;
-  float4* carry;             // [n_pad][2] running sums between bands
+  float4* carry;             // running sums between bands, [n_pad] (compensated: [n_pad][2])
   int32_t tile0, tile1;      // the band's i-tiles
 };
 int num_symmetric_shapes();
@@ -36,6 +36,10 @@ KernelShape symmetric_shape(int index);  // threads, i-particles per thread, j-t
 cudaError_t symmetric_blocks_per_sm(int index, bool compensated, bool per_pair_mass, int* blocks);
 cudaError_t launch_symmetric(int index, bool compensated, bool per_pair_mass, const SymArgs& a,
                              int grid, cudaStream_t stream);
+// The same over positions in the caller's layout, a float4 (x, y, z, m) per particle
+// (plain sums, per-particle masses; accelerations only).
+cudaError_t symmetric_xyzm_blocks_per_sm(int index, int* blocks);
+cudaError_t launch_symmetric_xyzm(int index, const SymArgs& a, int grid, cudaStream_t stream);
 // Add the rows and parts of the band's i-tiles and integrate; `tiles` i-tiles from a.tile0.
 cudaError_t launch_symmetric_add(bool compensated, const SymArgs& a, int tiles, int bi,
                                  cudaStream_t stream);

@@ -8,16 +8,16 @@
 // their own input and output buffers; the library allocates nothing on the
 // device and, on success, nothing on the host.
 //
-// The work the force kernel needs beyond its input and output -- the work list,
-// the partial sums of i-tiles whose j-range is split between CTAs, the arrival
-// counters, a copy of the positions in the kernel's pair layout, and the error
-// word -- lives in one file-scope device array, kScratchBytes (13 MiB) long.
-// Every GPU that loads this module keeps that array until the process exits.
-// All calls share it and it keeps the last call's contents: each call clears
-// what must start at zero (the counters and the error word).  Two calls whose
-// work overlapped on the GPU would race on it, so each call holds a process-wide
-// lock from its first copy until its stream has drained: the calls of one
-// process run one after another, whatever streams and threads they come from.
+// The work the symmetric force kernel needs beyond its input and output -- the work
+// list, the partial sums and the rows of j-side sums -- lives in one file-scope device
+// array, kScratchBytes (13 MiB) long; larger systems run in bands of i-tiles that take
+// turns in it (20,000 particles 223 us per call with the tuned kernel and its list
+// uploaded on every call, 154 now).  Every GPU that loads this module keeps that array until the process
+// exits.  All calls share it and it keeps the last call's contents: the work list stays
+// for the next call of the same size, checked by a tag that is read back with every
+// call.  Two calls whose work overlapped on the GPU would race on it, so each call holds
+// a process-wide lock until its stream has drained: the calls of one process run one
+// after another, whatever streams and threads they come from.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -30,42 +30,76 @@
 #include "nb_kernels.hpp"
 #include "nb_runtime.hpp"
 #include "nbody_gb300.h"
-#include "worklist.hpp"
+#include "symmetric_plan.hpp"
 
 namespace nbg {
 
 namespace {
 
-constexpr int kNaConfig = 0;                  // kernel shape: 128 threads x 4 i, 256-particle j-tiles
-constexpr int kNaBI = 512;                    // i-particles per CTA of that shape
-constexpr int kNaBJ = 256;                    // j-particles per tile of that shape
 constexpr int64_t kNaMaxParticles = 1 << 18;  // 262,144
-constexpr int kNaMaxItiles = static_cast<int>(kNaMaxParticles / kNaBI);
-// Persistent CTAs: the occupancy limit of the shape (two per SM on GB300), capped
-// at four per SM of a 152-SM part; a smaller grid only balances less finely.
-constexpr int kNaMaxGrid = 608;
-// Bounds of a plan over at most kNaMaxItiles i-tiles on at most kNaMaxGrid CTAs
-// (worklist.hpp): every CTA boundary inside an i-tile adds one segment, each
-// segment of a split i-tile takes one partial-sum slot, and an i-tile is split
-// only by a CTA boundary.
-constexpr int kNaMaxSegments = kNaMaxItiles + kNaMaxGrid - 1;
-constexpr int kNaMaxSlots = kNaMaxSegments;
-constexpr int kNaMaxFixups = kNaMaxItiles < kNaMaxGrid - 1 ? kNaMaxItiles : kNaMaxGrid - 1;
 constexpr int kNaMaxDevices = 64;
-static_assert(kNaMaxParticles % kNaBI == 0, "whole i-tiles at the maximum size");
+constexpr size_t kScratchBytes = 13u << 20;
 
-constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }
+// Candidate shapes by index of the symmetric kernel (i-tiles of 4,096, 256 and 64
+// particles), largest first, and choose_symmetric's rates for them.  512-particle
+// i-tiles would need 10 MB for the parts and as much for the rows at their sizes.
+constexpr int kNaShapes[] = {0, 2, 3};
+constexpr double kNaRates[][2] = {{1.0, 6.0}, {0.86, 0.8}, {0.617, 0.0}};
+constexpr int kNaCount = 3;
 
-constexpr size_t kOffSys = 0;
-constexpr size_t kOffErr = 256;
-constexpr size_t kOffCounters = 512;
-constexpr size_t kOffFix = align256(kOffCounters + sizeof(int32_t) * kNaMaxFixups);
-constexpr size_t kOffBegin = align256(kOffFix + sizeof(Fixup) * kNaMaxFixups);
-constexpr size_t kOffSegs = align256(kOffBegin + sizeof(int32_t) * (kNaMaxGrid + 1));
-constexpr size_t kOffPos = align256(kOffSegs + sizeof(Segment) * kNaMaxSegments);
-constexpr size_t kOffPartials = align256(kOffPos + 16 * kNaMaxParticles);
-constexpr size_t kScratchBytes = align256(kOffPartials + sizeof(float4) * kNaBI * kNaMaxSlots);
-static_assert(kScratchBytes <= (13u << 20), "no-allocation scratch is stated as 13 MiB");
+// A table of fixed size with the vector operations the planner uses; what does not fit
+// is dropped and remembered.
+template <class T, int N>
+struct FixedTable {
+  T data[N];
+  int n = 0;
+  bool full = false;
+  void push_back(const T& v) {
+    if (n < N)
+      data[n++] = v;
+    else
+      full = true;
+  }
+  void assign(size_t count, const T& v) {
+    n = 0;
+    for (size_t k = 0; k < count; ++k) push_back(v);
+  }
+  void erase(T* from, T* to) {
+    (void)to;  // the planner erases the tail
+    n = static_cast<int>(from - data);
+  }
+  size_t size() const { return n; }
+  bool empty() const { return n == 0; }
+  T& operator[](size_t i) { return data[i]; }
+  const T& operator[](size_t i) const { return data[i]; }
+  T& back() { return data[n - 1]; }
+  T* begin() { return data; }
+  T* end() { return data + n; }
+  const T* begin() const { return data; }
+  const T* end() const { return data + n; }
+};
+
+// Bounds: at most 64 i-tiles of 4,096 particles, each a band of its own on up to 152
+// CTAs; the smaller shapes are chosen for at most about 128 i-tiles, in a few bands on
+// at most kNaMaxGrid CTAs.  A plan that passes them is refused for the next shape.
+constexpr int kNaMaxGrid = 2432;
+constexpr int kNaMaxTiles = 512;
+constexpr int kNaMaxSegments = 10240;
+constexpr int kNaMaxBands = 64;
+
+struct FixedPlan {
+  FixedTable<SymSegment, kNaMaxSegments> segs;
+  FixedTable<int32_t, kNaMaxSegments + kNaMaxBands + 1> seg_begin;
+  FixedTable<SymTile, kNaMaxTiles> tiles;
+  FixedTable<int32_t, 2> sys_tile0;
+  FixedTable<SymBand, kNaMaxBands> bands;
+  int64_t row_values = 0;
+  int32_t slots = 0;
+  int32_t split_tiles = 0;
+  bool fits() const {
+    return !segs.full && !seg_begin.full && !tiles.full && !bands.full;
+  }
+};
 
 }  // namespace
 
@@ -75,98 +109,130 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 namespace {
 
-// Input float4 (x, y, z, m) -> pair layout in the scratch, padding far away.
-__global__ void na_to_pair_layout(const float4* __restrict__ in, int64_t n, int64_t npad,
-                                  float* __restrict__ pos) {
-  for (int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; g < npad;
-       g += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const float4 v = g < n ? in[g] : make_float4(kFarAway, kFarAway, kFarAway, 0.f);
-    pos[pair_index(g, 0)] = v.x;
-    pos[pair_index(g, 1)] = v.y;
-    pos[pair_index(g, 2)] = v.z;
-    pos[pair_index(g, 3)] = v.w;
-  }
-}
+constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }
+
+// Where the current plan's parts lie in the scratch; `copy`: of the caller's positions,
+// 0 where they are read in place.
+struct Layout {
+  size_t sys = 256, segs = 512, tiles = 0, partials = 0, rows = 0, copy = 0;  // the tag is at 0
+};
 
 struct DeviceSetup {
   bool ready = false;
   unsigned char* scratch = nullptr;  // device address of g_noalloc_scratch
-  int grid = 0;
+  int grid[kNaCount] = {};           // largest grid of each shape
+  // The plan in the scratch: for `n` particles, `tag` at its start; n = 0: none.
+  uint64_t n = 0;
+  uint32_t tag = 0;
+  float G = 0.f;
+  bool copied = false;
+  int shape = 0;
+  int64_t plane = 0;
+  int nbands = 0;
+  SymBand bands[kNaMaxBands];
+  Layout at;
 };
 
-std::mutex g_na_mutex;                       // guards the host-side tables below
+std::mutex g_na_mutex;            // guards the host-side tables below
 DeviceSetup g_na_setup[kNaMaxDevices];
-Segment g_na_segs[kNaMaxSegments];           // host plan, uploaded every call
-int32_t g_na_begin[kNaMaxGrid + 1];
-Fixup g_na_fix[kNaMaxFixups];
+FixedPlan g_na_plan;
+FixedTable<SymSegment, kNaMaxSegments> g_na_linked;
+uint32_t g_na_tag = 0;
 
-// The fixed host tables as the planner's output (worklist.hpp); refuses to grow.
-struct FixedTables {
-  int64_t grid = 0;
-  int64_t nseg = 0;
-  int64_t nfix = 0;
-  bool set_grid(int64_t g) {
-    grid = g;
-    return g >= 1 && g <= kNaMaxGrid;
-  }
-  bool add_segment(const Segment& sg) {
-    if (nseg >= kNaMaxSegments) return false;
-    g_na_segs[nseg++] = sg;
-    return true;
-  }
-  Segment& segment(int64_t i) { return g_na_segs[i]; }
-  int64_t num_segments() const { return nseg; }
-  void set_begin(int64_t cta, int64_t first) { g_na_begin[cta] = static_cast<int32_t>(first); }
-  bool add_fixup(const Fixup& f) {
-    if (nfix >= kNaMaxFixups) return false;
-    g_na_fix[nfix++] = f;
-    return true;
-  }
-  int64_t num_fixups() const { return nfix; }
-};
-
-// Once per device, with that device current: the scratch's device address and
-// the persistent grid size.
-int na_setup(int dev, DeviceSetup* out) {
+// Once per device, with that device current: the scratch's device address and the
+// shapes' grids.
+int na_setup(int dev) {
   DeviceSetup& d = g_na_setup[dev];
-  if (!d.ready) {
-    int sms = 0;
-    cudaDeviceProp prop;
-    NB_TRY(check_device(&sms, &prop));
-    void* p = nullptr;
-    const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-    if (e != cudaSuccess) return cuda_error(e, "cudaGetSymbolAddress(no-allocation scratch)");
+  if (d.ready) return NB_OK;
+  int sms = 0;
+  cudaDeviceProp prop;
+  NB_TRY(check_device(&sms, &prop));
+  void* p = nullptr;
+  const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+  if (e != cudaSuccess) return cuda_error(e, "cudaGetSymbolAddress(no-allocation scratch)");
+  for (int k = 0; k < kNaCount; ++k) {
     int blocks = 0;
-    NB_CUDA(force_blocks_per_sm(kNaConfig, false, true, false, &blocks));
-    const KernelShape sh = force_config_shape(kNaConfig);
-    if (sh.bi() != kNaBI || sh.bj != kNaBJ)
-      return set_error(NB_ERR_STATE, "no-allocation kernel shape mismatch");
-    d.scratch = static_cast<unsigned char*>(p);
-    d.grid = blocks * sms < kNaMaxGrid ? blocks * sms : kNaMaxGrid;
-    if (d.grid < 1) d.grid = 1;
-    d.ready = true;
+    NB_CUDA(symmetric_xyzm_blocks_per_sm(kNaShapes[k], &blocks));
+    d.grid[k] = std::max(1, std::min(blocks * sms, kNaMaxGrid));
   }
-  *out = d;
+  d.scratch = static_cast<unsigned char*>(p);
+  d.ready = true;
   return NB_OK;
 }
 
-// The force kernel's stream-K plan (plan_work_into, the rule of every other
-// launch) for one system, written into the fixed host tables.  The kernel runs
-// every register slot here (no live-slot variant), so the plan is unweighted.  The bounds above
-// make it fit for every n <= kNaMaxParticles and grid <= kNaMaxGrid; false if not.
-bool na_plan(int32_t n, int32_t npad, int32_t grid_max, int32_t* grid, int32_t* nseg,
-             int32_t* nfix, int32_t* nslots) {
+// Plan shape k for the system: as large bands as the scratch holds, on the shape's
+// full grid, or a smaller one where even one i-tile's row and parts are too much.  False
+// if it does not fit.
+bool na_plan(const SystemDesc& sd, const DeviceSetup& d, int k, bool copied, Layout* at) {
+  const KernelShape sh = symmetric_shape(kNaShapes[k]);
+  const int64_t tiles = (sd.n + sh.bi() - 1) / sh.bi();
+  if (tiles > kNaMaxTiles) return false;
+  const int64_t part = static_cast<int64_t>(sh.bi()) * sizeof(float4);  // bytes of one slot
+  const int64_t longest = std::max<int64_t>(0, sd.npad - sh.bi());      // values of the first row
+  const int64_t copy = copied ? static_cast<int64_t>(sd.n) * 16 : 0;
+  int64_t grid = d.grid[k];
+  for (int64_t per = tiles; grid >= 1;) {
+    // A plan of `per` i-tiles per band: its row values at most, and whether the parts and
+    // the rows of the largest band fit beside its tables.
+    const int64_t values = std::max<int64_t>(1, per * longest);
+    g_na_plan = FixedPlan{};
+    plan_symmetric_into(&sd, 0, 1, sh.bi(), sh.bj, static_cast<int32_t>(grid), values, per,
+                        kSymDiagCost, kSymPairCost, g_na_plan);
+    if (g_na_plan.fits()) {
+      at->tiles = align256(at->segs + g_na_plan.segs.size() * sizeof(SymSegment));
+      at->partials = align256(at->tiles + g_na_plan.tiles.size() * sizeof(SymTile));
+      at->rows = align256(at->partials + g_na_plan.slots * static_cast<size_t>(part));
+      const size_t end =
+          align256(at->rows + 3 * sizeof(float) * static_cast<size_t>(g_na_plan.row_values));
+      at->copy = copied ? end : 0;
+      if (end + static_cast<size_t>(copy) <= kScratchBytes) {
+        g_na_linked.n = static_cast<int>(g_na_plan.segs.size());
+        link_segments_into(g_na_plan, g_na_linked);
+        return true;
+      }
+    }
+    if (per > 1)
+      per = (per + 1) / 2;
+    else
+      grid -= 8;
+  }
+  return false;
+}
+
+// Plan n particles and put the plan into the scratch.
+int na_upload(DeviceSetup& d, uint64_t n, float G, bool copied, cudaStream_t st) {
+  d.n = 0;  // nothing until all of it is there
   SystemDesc sd{};
-  sd.n = n;
-  sd.npad = npad;
-  FixedTables out;
-  int32_t split = 0;
-  if (!plan_work_into(&sd, 0, 1, kNaBI, kNaBJ, grid_max, out, nslots, &split)) return false;
-  if (*nslots > kNaMaxSlots) return false;
-  *grid = static_cast<int32_t>(out.grid);
-  *nseg = static_cast<int32_t>(out.nseg);
-  *nfix = static_cast<int32_t>(out.nfix);
-  return true;
+  sd.offset = 0;
+  sd.n = static_cast<int32_t>(n);
+  sd.npad = (sd.n + kPadQuantum - 1) / kPadQuantum * kPadQuantum;
+  sd.gscale = G;  // per-pair masses: each pair term carries m_j
+  SymCandidate c[kNaCount];
+  for (int k = 0; k < kNaCount; ++k)
+    c[k] = SymCandidate{symmetric_shape(kNaShapes[k]), kNaRates[k][0], kNaRates[k][1], d.grid[k]};
+  int k = choose_symmetric(&sd, 0, 1, c, kNaCount, kSymDiagCost, kSymPairCost);
+  Layout at;
+  if (!na_plan(sd, d, k, copied, &at) && !na_plan(sd, d, k = 0, copied, &at))
+    return set_error(NB_ERR_INVALID_ARGUMENT, "work list exceeds the no-allocation scratch");
+  unsigned char* base = d.scratch;
+  const uint32_t tag = ++g_na_tag;
+  // Host sources are pageable: each copy has read them before it returns.
+  NB_CUDA(cudaMemcpyAsync(base + at.segs, g_na_linked.data, g_na_linked.n * sizeof(SymSegment),
+                          cudaMemcpyHostToDevice, st));
+  NB_CUDA(cudaMemcpyAsync(base + at.tiles, g_na_plan.tiles.data,
+                          g_na_plan.tiles.size() * sizeof(SymTile), cudaMemcpyHostToDevice, st));
+  NB_CUDA(cudaMemcpyAsync(base + at.sys, &sd, sizeof(sd), cudaMemcpyHostToDevice, st));
+  NB_CUDA(cudaMemcpyAsync(base, &tag, sizeof(tag), cudaMemcpyHostToDevice, st));
+  d.tag = tag;
+  d.G = G;
+  d.copied = copied;
+  d.shape = kNaShapes[k];
+  d.plane = g_na_plan.row_values;
+  d.nbands = static_cast<int>(g_na_plan.bands.size());
+  for (int b = 0; b < d.nbands; ++b) d.bands[b] = g_na_plan.bands[b];
+  d.at = at;
+  d.n = n;
+  return NB_OK;
 }
 
 }  // namespace
@@ -195,64 +261,52 @@ extern "C" int nb_accelerations_noalloc(const float* pos_xyzm_device, uint64_t n
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 
   std::lock_guard<std::mutex> lock(g_na_mutex);
-  DeviceSetup d;
-  NB_TRY(na_setup(dev, &d));
-  const int32_t ni = static_cast<int32_t>(n);
-  const int32_t npad = (ni + kPadQuantum - 1) / kPadQuantum * kPadQuantum;
-  int32_t grid = 0, nseg = 0, nfix = 0, nslots = 0;
-  if (!na_plan(ni, npad, d.grid, &grid, &nseg, &nfix, &nslots))
-    return set_error(NB_ERR_INVALID_ARGUMENT, "work list exceeds the no-allocation scratch");
-
-  SystemDesc sd{};
-  sd.offset = 0;
-  sd.n = ni;
-  sd.npad = npad;
-  sd.gscale = G;  // per-pair masses: each pair term carries m_j
-  sd.mass = 0.f;
-  sd.equal_mass = 0;
-  unsigned char* base = d.scratch;
-  // Host sources are pageable: each copy has read them before it returns.
-  NB_CUDA(cudaMemcpyAsync(base + kOffSys, &sd, sizeof(sd), cudaMemcpyHostToDevice, st));
-  NB_CUDA(cudaMemcpyAsync(base + kOffSegs, g_na_segs, sizeof(Segment) * nseg,
-                          cudaMemcpyHostToDevice, st));
-  NB_CUDA(cudaMemcpyAsync(base + kOffBegin, g_na_begin, sizeof(int32_t) * (grid + 1),
-                          cudaMemcpyHostToDevice, st));
-  if (nfix > 0)
-    NB_CUDA(cudaMemcpyAsync(base + kOffFix, g_na_fix, sizeof(Fixup) * nfix,
-                            cudaMemcpyHostToDevice, st));
-  // What must start at zero: the arrival counters and the error word.
-  NB_CUDA(cudaMemsetAsync(base + kOffCounters, 0, sizeof(int32_t) * kNaMaxFixups, st));
-  NB_CUDA(cudaMemsetAsync(base + kOffErr, 0, sizeof(int32_t), st));
-  float* pos = reinterpret_cast<float*>(base + kOffPos);
-  na_to_pair_layout<<<(npad + 255) / 256, 256, 0, st>>>(
-      reinterpret_cast<const float4*>(pos_xyzm_device), static_cast<int64_t>(n), npad, pos);
-  NB_CUDA(cudaGetLastError());
-
-  ForceArgs a{};
-  a.pos = pos;
-  a.pos_next = nullptr;
-  a.vel = nullptr;
-  a.accel_out = reinterpret_cast<float4*>(accel_xyzw_device);
-  a.sys = reinterpret_cast<const SystemDesc*>(base + kOffSys);
-  a.segs = reinterpret_cast<const Segment*>(base + kOffSegs);
-  a.seg_begin = reinterpret_cast<const int32_t*>(base + kOffBegin);
-  a.fix = reinterpret_cast<const Fixup*>(base + kOffFix);
-  a.partials = reinterpret_cast<float4*>(base + kOffPartials);
-  a.counters = reinterpret_cast<int32_t*>(base + kOffCounters);
-  a.err = reinterpret_cast<int32_t*>(base + kOffErr);
-  a.eps2 = dist_eps;
-  a.dt = 0.f;
-  a.damping = 0.f;
-  {
+  NB_TRY(na_setup(dev));
+  DeviceSetup& d = g_na_setup[dev];
+  // A caller may pass one buffer for both: bands would read positions that earlier bands
+  // have replaced, so overlapping buffers are copied first.
+  const uintptr_t in = reinterpret_cast<uintptr_t>(pos_xyzm_device);
+  const uintptr_t out = reinterpret_cast<uintptr_t>(accel_xyzw_device);
+  const bool copied = in < out + 16 * n && out < in + 16 * n;
+  // Twice where the scratch does not hold the plan any more (a device reset).
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    if (d.n != n || d.G != G || d.copied != copied) NB_TRY(na_upload(d, n, G, copied, st));
+    unsigned char* base = d.scratch;
+    SymArgs a{};
+    a.f.pos = pos_xyzm_device;
+    if (copied) {
+      NB_CUDA(cudaMemcpyAsync(base + d.at.copy, pos_xyzm_device, 16 * n, cudaMemcpyDeviceToDevice,
+                              st));
+      a.f.pos = reinterpret_cast<const float*>(base + d.at.copy);
+    }
+    a.f.accel_out = reinterpret_cast<float4*>(accel_xyzw_device);
+    a.f.sys = reinterpret_cast<const SystemDesc*>(base + d.at.sys);
+    a.f.partials = reinterpret_cast<float4*>(base + d.at.partials);
+    a.f.eps2 = dist_eps;
     const float e3 = dist_eps * dist_eps * dist_eps;
-    a.mask_self = (e3 >= FLT_MIN) ? 0 : 1;
+    a.f.mask_self = (e3 >= FLT_MIN) ? 0 : 1;
+    a.tiles = reinterpret_cast<const SymTile*>(base + d.at.tiles);
+    a.rows = reinterpret_cast<float*>(base + d.at.rows);
+    a.plane = d.plane;
+    a.carry = a.f.accel_out;  // a particle's place is free until its last band
+    const int bi = symmetric_shape(d.shape).bi();
+    for (int b = 0; b < d.nbands; ++b) {
+      const SymBand& band = d.bands[b];
+      a.segs = reinterpret_cast<const SymSegment*>(base + d.at.segs) + band.seg0;
+      a.tile0 = band.tile0;
+      a.tile1 = band.tile1;
+      NB_CUDA(launch_symmetric_xyzm(d.shape, a, band.grid, st));
+      NB_CUDA(launch_symmetric_add(false, a, band.end - band.tile0, bi, st));
+    }
+    uint32_t tag = 0;
+    NB_CUDA(cudaMemcpyAsync(&tag, base, sizeof(tag), cudaMemcpyDeviceToHost, st));
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {
+      d.n = 0;
+      return cuda_error(e, "cudaStreamSynchronize");
+    }
+    if (tag == d.tag) return NB_OK;
+    d.n = 0;
   }
-  a.inject = 0;
-  NB_CUDA(launch_force(kNaConfig, false, true, false, a, grid, st));
-  int32_t err = 0;
-  NB_CUDA(cudaMemcpyAsync(&err, base + kOffErr, sizeof(err), cudaMemcpyDeviceToHost, st));
-  NB_CUDA(cudaStreamSynchronize(st));
-  if (err != 0)
-    return set_error(NB_ERR_DEVICE_TIMEOUT, "a bounded device-side wait timed out");
-  return NB_OK;
+  return set_error(NB_ERR_STATE, "the no-allocation scratch was overwritten");
 }

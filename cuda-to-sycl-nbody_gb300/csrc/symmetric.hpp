@@ -44,7 +44,7 @@ struct SymSegment {
   int64_t offset;  // first particle of the system, and its particles
   int32_t n;
   int32_t slot;
-  int32_t next;    // the CTA's next segment, -1 for none; CTA k starts with segment k
+  int32_t next;    // 1 + the CTA's next segment, 0 for none; CTA k starts with segment k
   int32_t pad_;
 };
 
@@ -81,7 +81,7 @@ struct SymPlanHost {
 };
 
 // The segments in the order the kernel wants them: per band, the first of every CTA and
-// then the others, linked by `next` (relative to the band's seg0).
+// then the others, linked by `next` (counted from the band's seg0).
 std::vector<SymSegment> link_segments(const SymPlanHost& plan);
 
 // Plan systems [first, first + count) (whole systems, no shards) for i-tiles of bi and

@@ -14,6 +14,7 @@ struct EarlyForce {
   float x, y, z;
   __device__ void lists(int sys) { sd = f.sys[sys]; }
   __device__ void state(int64_t g) {
+    if (f.accel_out != nullptr) return;
     x = f.pos[pair_index(g, 0)];
     y = f.pos[pair_index(g, 1)];
     z = f.pos[pair_index(g, 2)];

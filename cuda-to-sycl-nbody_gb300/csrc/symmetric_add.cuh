@@ -29,7 +29,7 @@ struct AddTerms {
   const SymTile* tiles;
   const float* rows;
   int64_t plane;
-  float4* carry;
+  float4* carry;  // running sums, with their low words if compensated
   const float4* partials;
   int tile0, tile1;
 };
@@ -142,9 +142,12 @@ __device__ __forceinline__ bool add_terms(const AddTerms& a, int bi, Early& earl
   Sum3<kComp> all;
   float low[3] = {0.f, 0.f, 0.f};
   if (sys0 < a.tile0) {  // earlier bands
-    const float4 s = a.carry[2 * g], l = a.carry[2 * g + 1];
+    const float4 s = a.carry[kRec * g];
     all.s[0] = s.x, all.s[1] = s.y, all.s[2] = s.z;
-    low[0] = l.x, low[1] = l.y, low[2] = l.z;
+    if (kComp) {
+      const float4 l = a.carry[kRec * g + 1];
+      low[0] = l.x, low[1] = l.y, low[2] = l.z;
+    }
   }
 #pragma unroll
   for (int u = 0; u < kAddGroups; ++u)
@@ -157,8 +160,8 @@ __device__ __forceinline__ bool add_terms(const AddTerms& a, int bi, Early& earl
 #pragma unroll
     for (int c = 0; c < 3; ++c) low[c] -= all.c[c];
   if (!mine) {  // later bands add the rest
-    a.carry[2 * g] = make_float4(all.s[0], all.s[1], all.s[2], 0.f);
-    a.carry[2 * g + 1] = make_float4(low[0], low[1], low[2], 0.f);
+    a.carry[kRec * g] = make_float4(all.s[0], all.s[1], all.s[2], 0.f);
+    if (kComp) a.carry[kRec * g + 1] = make_float4(low[0], low[1], low[2], 0.f);
     return false;
   }
   out = AddResult{g, all.s[0] + low[0], all.s[1] + low[1], all.s[2] + low[2]};

@@ -164,7 +164,8 @@ __device__ __forceinline__ void sym_chunk(SymI<P>& q, const float2* mi, float x,
 }  // namespace
 
 // NW warps, P i-pairs per thread (i-tiles of 64 P NW particles).
-template <int NW, int P, int U, bool kComp, bool kMass>
+// kXyzm: positions are a float4 (x, y, z, m) per particle, and no padding follows them.
+template <int NW, int P, int U, bool kComp, bool kMass, bool kXyzm>
 __global__ void __launch_bounds__(NW * 32, 8 / NW) symmetric_kernel(const SymArgs a) {
   constexpr int T = NW * 32;
   constexpr int BI = T * 2 * P;
@@ -185,11 +186,19 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) symmetric_kernel(const SymArg
   // The lists are older than the predecessor's launch; the state is not.
   SymSegment sg = a.segs[blockIdx.x];
   pdl_wait();
-  for (int next = blockIdx.x; next >= 0;) {
-    if (next != static_cast<int>(blockIdx.x)) sg = a.segs[next];
+  // Where the next segment is loaded makes no difference to what runs, but ptxas
+  // schedules the pair loop differently (N = 1,048,576: 8 warps 229 ms at the top of the
+  // loop, 239 at its end; one warp 252 and 244).
+  constexpr bool kTop = NW == 8;
+  for (int next = blockIdx.x + 1; next > 0;) {
+    if (kTop && next != static_cast<int>(blockIdx.x) + 1) sg = a.segs[next - 1];
     next = sg.next;
     const int ibase = sg.itile * BI;
     const float* pos = a.f.pos + 4 * sg.offset;  // offsets are even: whole pair records
+
+    auto at = [](int i, int c) -> int64_t {
+      return kXyzm ? 4 * static_cast<int64_t>(i) + c : pair_index(i, c);
+    };
 
     SymI<P> q;
     float2 mi[P];
@@ -202,7 +211,7 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) symmetric_kernel(const SymArg
         const bool real = li < sg.n;
 #pragma unroll
         for (int c = 0; c < 4; ++c)
-          v[h][c] = real ? pos[pair_index(li, c)] : (c < 3 ? kFarAway : 0.f);
+          v[h][c] = real ? pos[at(li, c)] : (c < 3 ? kFarAway : 0.f);
       }
       q.nx[r] = make_float2(-v[0][0], -v[1][0]);
       q.ny[r] = make_float2(-v[0][1], -v[1][1]);
@@ -212,15 +221,15 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) symmetric_kernel(const SymArg
     }
 
     // The lane's j-particle of the next chunk, loaded one chunk ahead.
-    const int jend = min((sg.n + kPadQuantum - 1) & -kPadQuantum, sg.jt1 * BJ);
+    const int jend = min(kXyzm ? sg.n : (sg.n + kPadQuantum - 1) & -kPadQuantum, sg.jt1 * BJ);
     float nx = kFarAway, ny = kFarAway, nz = kFarAway, nm = 0.f;
     auto fetch = [&](int j0) {
       const int j = j0 + lane;
       const bool in = j < jend;
-      nx = in ? pos[pair_index(j, 0)] : kFarAway;
-      ny = in ? pos[pair_index(j, 1)] : kFarAway;
-      nz = in ? pos[pair_index(j, 2)] : kFarAway;
-      if (kMass) nm = in ? pos[pair_index(j, 3)] : 0.f;
+      nx = in ? pos[at(j, 0)] : kFarAway;
+      ny = in ? pos[at(j, 1)] : kFarAway;
+      nz = in ? pos[at(j, 2)] : kFarAway;
+      if (kMass) nm = in ? pos[at(j, 3)] : 0.f;
     };
     fetch(sg.jt0 * BJ);
 
@@ -284,7 +293,7 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) symmetric_kernel(const SymArg
       }
     }
 
-    if (next < 0) pdl_trigger();
+    if (next <= 0) pdl_trigger();
     // The segment's i-side sums: (hi, lo) records, or the plain sums.
     constexpr int kRec = kComp ? 2 : 1;
     float4* part = a.f.partials + static_cast<int64_t>(sg.slot) * BI * kRec;
@@ -304,6 +313,7 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) symmetric_kernel(const SymArg
         part[i1 * kRec + 1] = make_float4(-cx.y, -cy.y, -cz.y, 0.f);
       }
     }
+    if (!kTop && next > 0) sg = a.segs[next - 1];
   }
 }
 

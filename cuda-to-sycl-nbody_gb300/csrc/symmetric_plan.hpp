@@ -1,0 +1,144 @@
+// The planner behind symmetric.hpp, writing to tables that grow (plan_symmetric) or to
+// fixed ones (nb_accelerations_noalloc) by one rule.
+//
+// Plan has the members of SymPlanHost; its tables provide the std::vector operations
+// used here, and fixed ones drop what does not fit (their owner checks).
+#pragma once
+
+#include <algorithm>
+#include <cstdint>
+
+#include "symmetric.hpp"
+
+namespace nbg {
+
+// Charges of one i-tile's units: the j-tiles from t0 (diagonal) over td (behind the
+// i-tile) to t1, each bj particles of the diagonal or the pair cost.
+struct SymTileCharge {
+  int32_t t0, td, t1;
+  int64_t diag, pair;
+  int64_t upto(int32_t t) const {
+    const int64_t d = std::min(t, td) - t0, p = std::max(0, t - td);
+    return d * diag + p * pair;
+  }
+  // Smallest t in [t0, t1] with upto(t) >= c.
+  int32_t reach(int64_t c) const {
+    if (c <= 0) return t0;
+    const int64_t whole = upto(td);
+    const int64_t t = c <= whole ? t0 + (c + diag - 1) / diag
+                                 : td + (c - whole + pair - 1) / pair;
+    return static_cast<int32_t>(std::min<int64_t>(t, t1));
+  }
+};
+
+template <class Plan>
+void plan_symmetric_into(const SystemDesc* sys, int32_t first, int32_t count, int32_t bi,
+                         int32_t bj, int32_t max_grid, int64_t max_row_values,
+                         int64_t max_band_tiles, int diag_cost, int pair_cost, Plan& plan) {
+  // The i-tiles, their rows and the bands they fall into.
+  plan.sys_tile0.assign(first + count + 1, 0);
+  int64_t values = 0;
+  for (int32_t s = first; s < first + count; ++s) {
+    plan.sys_tile0[s] = static_cast<int32_t>(plan.tiles.size());
+    const int32_t nit = (sys[s].n + bi - 1) / bi;
+    for (int32_t it = 0; it < nit; ++it) {
+      const int32_t t = static_cast<int32_t>(plan.tiles.size());
+      const int64_t behind = static_cast<int64_t>(it + 1) * bi;
+      const int64_t len = std::max<int64_t>(0, sys[s].npad - behind);
+      if (plan.bands.empty() || values + len > max_row_values ||
+          t - plan.bands.back().tile0 >= max_band_tiles) {
+        SymBand b;
+        b.tile0 = t;
+        plan.bands.push_back(b);
+        values = 0;
+      }
+      plan.tiles.push_back(SymTile{values - behind, sys[s].offset, sys[s].n, s, it, 0, 0, 0});
+      values += len;
+      plan.row_values = std::max(plan.row_values, values);
+      plan.bands.back().tile1 = t + 1;
+    }
+  }
+  plan.sys_tile0[first + count] = static_cast<int32_t>(plan.tiles.size());
+
+  auto charge_of = [&](const SymTile& t) {
+    const SystemDesc& d = sys[t.sys];
+    SymTileCharge c;
+    c.t0 = t.itile * (bi / bj);
+    c.t1 = (d.npad + bj - 1) / bj;
+    c.td = std::min(c.t1, c.t0 + bi / bj);
+    c.diag = static_cast<int64_t>(bj) * diag_cost;
+    c.pair = static_cast<int64_t>(bj) * pair_cost;
+    return c;
+  };
+  for (SymBand& b : plan.bands) {
+    b.end = plan.sys_tile0[plan.tiles[b.tile1 - 1].sys + 1];
+    int64_t total = 0, units = 0;
+    for (int32_t t = b.tile0; t < b.tile1; ++t) {
+      const SymTileCharge c = charge_of(plan.tiles[t]);
+      total += c.upto(c.t1);
+      units += c.t1 - c.t0;
+    }
+    b.grid = static_cast<int32_t>(std::max<int64_t>(1, std::min<int64_t>(max_grid, units)));
+    b.begin0 = static_cast<int32_t>(plan.seg_begin.size());
+    // CTA k takes the units whose starting charge is in [k, k + 1) * total / grid.
+    auto bound = [&](int64_t k) {
+      return static_cast<int64_t>((static_cast<__int128>(k) * total + b.grid - 1) / b.grid);
+    };
+    int64_t c0 = 0;
+    int32_t next_cta = 0, slot = 0;
+    b.seg0 = static_cast<int32_t>(plan.segs.size());
+    for (int32_t t = b.tile0; t < b.tile1; ++t) {
+      SymTile& tile = plan.tiles[t];
+      const SymTileCharge c = charge_of(tile);
+      tile.slot0 = slot;
+      int32_t jt = c.t0;
+      while (jt < c.t1) {
+        const int64_t at = c0 + c.upto(jt);
+        int64_t k = std::min<int64_t>(b.grid - 1,
+                                      static_cast<int64_t>(static_cast<__int128>(at) * b.grid / total));
+        int32_t end = c.t1;
+        if (k + 1 < b.grid) end = std::max(jt + 1, c.reach(bound(k + 1) - c0));
+        while (next_cta <= k) {
+          plan.seg_begin.push_back(static_cast<int32_t>(plan.segs.size()));
+          ++next_cta;
+        }
+        plan.segs.push_back(SymSegment{tile.sys, tile.itile, jt, end, tile.row,
+                                       sys[tile.sys].offset, sys[tile.sys].n, slot++, -1, 0});
+        jt = end;
+      }
+      tile.nslots = slot - tile.slot0;
+      if (tile.nslots > 1) ++plan.split_tiles;
+      c0 += c.upto(c.t1);
+    }
+    while (next_cta <= b.grid) {
+      plan.seg_begin.push_back(static_cast<int32_t>(plan.segs.size()));
+      ++next_cta;
+    }
+    // A CTA whose share holds no unit's start (a unit can charge more than a share)
+    // drops out.
+    const auto begin = plan.seg_begin.begin() + b.begin0;
+    plan.seg_begin.erase(std::unique(begin, plan.seg_begin.end()), plan.seg_begin.end());
+    b.grid = static_cast<int32_t>(plan.seg_begin.size()) - b.begin0 - 1;
+    plan.slots = std::max(plan.slots, static_cast<int32_t>(plan.segs.size()) - b.seg0);
+  }
+}
+
+// `out` holds plan.segs.size() segments.
+template <class Plan, class Out>
+void link_segments_into(const Plan& plan, Out& out) {
+  for (const SymBand& b : plan.bands) {
+    int32_t more = b.grid;  // the next free place behind the first segments
+    for (int32_t k = 0; k < b.grid; ++k) {
+      int32_t at = k;
+      for (int32_t q = plan.seg_begin[b.begin0 + k]; q < plan.seg_begin[b.begin0 + k + 1]; ++q) {
+        SymSegment sg = plan.segs[q];
+        const bool last = q + 1 == plan.seg_begin[b.begin0 + k + 1];
+        sg.next = last ? 0 : ++more;
+        out[b.seg0 + at] = sg;
+        at = sg.next - 1;
+      }
+    }
+  }
+}
+
+}  // namespace nbg

@@ -7,7 +7,7 @@
 namespace nbg {
 namespace {
 
-template <int NW, int P, int U, bool C, bool M>
+template <int NW, int P, int U, bool C, bool M, bool X>
 cudaError_t smem_opt_in() {
   static std::atomic<uint64_t> opted{0};  // once per device ordinal (>= 64: every call)
   int dev = 0;
@@ -15,41 +15,44 @@ cudaError_t smem_opt_in() {
   if (e != cudaSuccess) return e;
   const uint64_t bit = dev >= 0 && dev < 64 ? uint64_t{1} << dev : 0;
   if (bit != 0 && (opted.load(std::memory_order_acquire) & bit) != 0) return cudaSuccess;
-  e = cudaFuncSetAttribute(symmetric_kernel<NW, P, U, C, M>,
+  e = cudaFuncSetAttribute(symmetric_kernel<NW, P, U, C, M, X>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize,
                            symmetric_smem<NW, P, C>());
   if (e == cudaSuccess && bit != 0) opted.fetch_or(bit, std::memory_order_release);
   return e;
 }
 
-template <int NW, int P, int U, bool C, bool M>
+template <int NW, int P, int U, bool C, bool M, bool X>
 cudaError_t launch_one(const SymArgs& a, int grid, cudaStream_t st) {
-  const cudaError_t e = smem_opt_in<NW, P, U, C, M>();
+  const cudaError_t e = smem_opt_in<NW, P, U, C, M, X>();
   if (e != cudaSuccess) return e;
-  return launch_dependent(symmetric_kernel<NW, P, U, C, M>, dim3(grid), NW * 32,
+  return launch_dependent(symmetric_kernel<NW, P, U, C, M, X>, dim3(grid), NW * 32,
                           symmetric_smem<NW, P, C>(), st, a);
 }
 
-template <int NW, int P, int U, bool C, bool M>
+template <int NW, int P, int U, bool C, bool M, bool X>
 cudaError_t occ_one(int* blocks) {
-  const cudaError_t e = smem_opt_in<NW, P, U, C, M>();
+  const cudaError_t e = smem_opt_in<NW, P, U, C, M, X>();
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      blocks, symmetric_kernel<NW, P, U, C, M>, NW * 32, symmetric_smem<NW, P, C>());
+      blocks, symmetric_kernel<NW, P, U, C, M, X>, NW * 32, symmetric_smem<NW, P, C>());
 }
 
 struct SymEntry {
   int warps, pairs, bj;
   cudaError_t (*launch[2][2])(const SymArgs&, int, cudaStream_t);  // [compensated][mass]
   cudaError_t (*occ[2][2])(int*);
+  cudaError_t (*launch_xyzm)(const SymArgs&, int, cudaStream_t);   // plain, own masses
+  cudaError_t (*occ_xyzm)(int*);
 };
 
-#define NBG_SYM(NW, P, U)                                                                   \
-  {NW, P, kSymBJ<NW>,                                                                       \
-   {{launch_one<NW, P, U, false, false>, launch_one<NW, P, U, false, true>},                \
-    {launch_one<NW, P, U, true, false>, launch_one<NW, P, U, true, true>}},                 \
-   {{occ_one<NW, P, U, false, false>, occ_one<NW, P, U, false, true>},                      \
-    {occ_one<NW, P, U, true, false>, occ_one<NW, P, U, true, true>}}}
+#define NBG_SYM(NW, P, U)                                                                         \
+  {NW, P, kSymBJ<NW>,                                                                             \
+   {{launch_one<NW, P, U, false, false, false>, launch_one<NW, P, U, false, true, false>},        \
+    {launch_one<NW, P, U, true, false, false>, launch_one<NW, P, U, true, true, false>}},         \
+   {{occ_one<NW, P, U, false, false, false>, occ_one<NW, P, U, false, true, false>},              \
+    {occ_one<NW, P, U, true, false, false>, occ_one<NW, P, U, true, true, false>}},               \
+   launch_one<NW, P, U, false, true, true>, occ_one<NW, P, U, false, true, true>}
 
 const SymEntry kShapes[] = {NBG_SYM(8, 8, 2), NBG_SYM(1, 8, 2), NBG_SYM(1, 4, 4),
                             NBG_SYM(1, 1, 4)};
@@ -70,6 +73,14 @@ cudaError_t symmetric_blocks_per_sm(int index, bool compensated, bool per_pair_m
 cudaError_t launch_symmetric(int index, bool compensated, bool per_pair_mass, const SymArgs& a,
                              int grid, cudaStream_t stream) {
   return kShapes[index].launch[compensated][per_pair_mass](a, grid, stream);
+}
+
+cudaError_t symmetric_xyzm_blocks_per_sm(int index, int* blocks) {
+  return kShapes[index].occ_xyzm(blocks);
+}
+
+cudaError_t launch_symmetric_xyzm(int index, const SymArgs& a, int grid, cudaStream_t stream) {
+  return kShapes[index].launch_xyzm(a, grid, stream);
 }
 
 }  // namespace nbg
