@@ -12,12 +12,12 @@
 // list, the partial sums and the rows of j-side sums -- lives in one file-scope device
 // array, kScratchBytes (13 MiB) long; larger systems run in bands of i-tiles that take
 // turns in it (20,000 particles 223 us per call with the tuned kernel and its list
-// uploaded on every call, 154 now).  Every GPU that loads this module keeps that array until the process
-// exits.  All calls share it and it keeps the last call's contents: the work list stays
-// for the next call of the same size, checked by a tag that is read back with every
-// call.  Two calls whose work overlapped on the GPU would race on it, so each call holds
-// a process-wide lock until its stream has drained: the calls of one process run one
-// after another, whatever streams and threads they come from.
+// uploaded on every call, 154 now).  Every GPU that loads this module keeps that array
+// until the process exits.  All calls share it and it keeps the last call's contents:
+// the work list stays for the next call of the same size, checked by a tag that is read
+// back with every call.  Two calls whose work overlapped on the GPU would race on it, so
+// each call holds a process-wide lock until its stream has drained: the calls of one
+// process run one after another, whatever streams and threads they come from.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -60,8 +60,12 @@ struct FixedTable {
     else
       full = true;
   }
-  void assign(size_t count, const T& v) {
+  void clear() {
     n = 0;
+    full = false;
+  }
+  void assign(size_t count, const T& v) {
+    clear();
     for (size_t k = 0; k < count; ++k) push_back(v);
   }
   void erase(T* from, T* to) {
@@ -96,6 +100,15 @@ struct FixedPlan {
   int64_t row_values = 0;
   int32_t slots = 0;
   int32_t split_tiles = 0;
+  void clear() {
+    segs.clear();
+    seg_begin.clear();
+    tiles.clear();
+    sys_tile0.clear();
+    bands.clear();
+    row_values = 0;
+    slots = split_tiles = 0;
+  }
   bool fits() const {
     return !segs.full && !seg_begin.full && !tiles.full && !bands.full;
   }
@@ -175,7 +188,7 @@ bool na_plan(const SystemDesc& sd, const DeviceSetup& d, int k, bool copied, Lay
     // A plan of `per` i-tiles per band: its row values at most, and whether the parts and
     // the rows of the largest band fit beside its tables.
     const int64_t values = std::max<int64_t>(1, per * longest);
-    g_na_plan = FixedPlan{};
+    g_na_plan.clear();
     plan_symmetric_into(&sd, 0, 1, sh.bi(), sh.bj, static_cast<int32_t>(grid), values, per,
                         kSymDiagCost, kSymPairCost, g_na_plan);
     if (g_na_plan.fits()) {
