@@ -17,6 +17,7 @@ struct RenderUniforms {
   int32_t height;
   int32_t margin;        // HDR framebuffer margin (FBO_MARGIN)
   int32_t bw, bh;        // HDR framebuffer
+  int32_t pitch;         // its row in pixels, even (two pixels are one 16-byte reduction)
   int32_t ow, oh;        // blur targets (downscaled by 2)
   int32_t lw, lh;        // luminance target (half size)
   int32_t flare_n;       // flare texture is flare_n x flare_n
@@ -26,11 +27,12 @@ struct RenderUniforms {
   float weight[kRenderMaxTaps];
 };
 
+// Light is additive in two terms: a sprite's colour is (t, 0.4 (1 - t) + 0.2 t, 1) times
+// its alpha, so sums of alpha and of alpha t give all three channels (light_rgb).
 struct RenderBuffers {
-  float4* hdr = nullptr;     // bw x bh
-  float4* blur1 = nullptr;   // ow x oh
-  float4* blur2 = nullptr;   // ow x oh (bloom)
-  float* lum = nullptr;      // lw x lh
+  float2* hdr = nullptr;     // pitch x bh
+  float2* blur1 = nullptr;   // ow x oh
+  float2* blur2 = nullptr;   // ow x oh (bloom)
   double* block_sums = nullptr;
   float* mean = nullptr;
   float* flare = nullptr;    // flare_n x flare_n
@@ -40,6 +42,9 @@ struct RenderBuffers {
 cudaError_t launch_render(const float* pos, const float4* vel, int64_t n_pad,
                           const RenderUniforms& u, const RenderBuffers& b, float4* out,
                           cudaStream_t stream);
+
+// Partial luminance sums of a frame.
+int64_t render_luminance_parts(const RenderUniforms& u);
 
 // Host tables shared by the renderer and its tests.
 void render_gauss_tables(float sigma, int halfwidth, float* offsets, float* weights, int* taps);

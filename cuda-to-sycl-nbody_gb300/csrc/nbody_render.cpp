@@ -77,7 +77,6 @@ void release_render(RenderBuffers& b) {
   dev_free(b.hdr);
   dev_free(b.blur1);
   dev_free(b.blur2);
-  dev_free(b.lum);
   dev_free(b.block_sums);
   dev_free(b.mean);
   dev_free(b.flare);
@@ -166,6 +165,7 @@ int nb_sim_render(nb_sim* s, const float view[16], const float proj[16], int32_t
   u.margin = kMargin;
   u.bw = width + 2 * kMargin;
   u.bh = height + 2 * kMargin;
+  u.pitch = (u.bw + 1) & ~1;
   u.ow = u.bw / kBlurDownscale;
   u.oh = u.bh / kBlurDownscale;
   u.lw = u.bw / 2;
@@ -179,11 +179,10 @@ int nb_sim_render(nb_sim* s, const float view[16], const float proj[16], int32_t
   RenderBuffers& b = s->render;
   if (b.width != width || b.height != height) {
     release_render(b);
-    NB_TRY(dev_alloc(&b.hdr, static_cast<size_t>(u.bw) * u.bh));
+    NB_TRY(dev_alloc(&b.hdr, static_cast<size_t>(u.pitch) * u.bh));
     NB_TRY(dev_alloc(&b.blur1, static_cast<size_t>(u.ow) * u.oh));
     NB_TRY(dev_alloc(&b.blur2, static_cast<size_t>(u.ow) * u.oh));
-    NB_TRY(dev_alloc(&b.lum, static_cast<size_t>(u.lw) * u.lh));
-    NB_TRY(dev_alloc(&b.block_sums, static_cast<size_t>((u.lw + 15) / 16) * ((u.lh + 15) / 16)));
+    NB_TRY(dev_alloc(&b.block_sums, static_cast<size_t>(render_luminance_parts(u))));
     NB_TRY(dev_alloc(&b.mean, 1));
     NB_TRY(dev_alloc(&b.flare, kFlareSize * kFlareSize));
     std::vector<float> fl(kFlareSize * kFlareSize);

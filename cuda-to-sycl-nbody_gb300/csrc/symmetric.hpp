@@ -30,7 +30,7 @@ constexpr int kSymPairCost = 14;
 constexpr int kAdjDiagCost = 22;
 constexpr int kAdjPairCost = 25;
 constexpr int64_t kSymRowBytes = 3 * sizeof(float);  // scratch per row value
-constexpr int64_t kSymScratchBytes = int64_t{1} << 29;
+constexpr int64_t kSymScratchBytes = int64_t{1} << 28;
 
 // One entry of a CTA's list: i-tile `itile` of system `sys` against j-tiles [jt0, jt1).
 // The j-side sum of particle j goes to value row + j of each plane of the row scratch,
