@@ -64,6 +64,7 @@ __global__ void unpack_kernel(const float* __restrict__ soa, int64_t n,
 __global__ void pack_kernel(const float* __restrict__ pos, const float4* __restrict__ vel,
                             int64_t n, const int64_t* __restrict__ map,
                             float* __restrict__ soa) {
+  pdl_wait();
   for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < n;
        k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t g = map ? map[k] : k;
@@ -75,10 +76,12 @@ __global__ void pack_kernel(const float* __restrict__ pos, const float4* __restr
     soa[4 * n + k] = v.y;
     soa[5 * n + k] = v.z;
   }
+  pdl_trigger();
 }
 
 __global__ void pack_accel_kernel(const float4* __restrict__ acc, int64_t n,
                                   const int64_t* __restrict__ map, float* __restrict__ soa) {
+  pdl_wait();
   for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < n;
        k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t g = map ? map[k] : k;
@@ -87,11 +90,13 @@ __global__ void pack_accel_kernel(const float4* __restrict__ acc, int64_t n,
     soa[n + k] = a.y;
     soa[2 * n + k] = a.z;
   }
+  pdl_trigger();
 }
 
 __global__ void export_kernel(const float* __restrict__ pos, const float4* __restrict__ vel,
                               int64_t n, const int64_t* __restrict__ map,
                               float4* __restrict__ pos_out, float4* __restrict__ vel_out) {
+  pdl_wait();
   for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < n;
        k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t g = map ? map[k] : k;
@@ -99,6 +104,7 @@ __global__ void export_kernel(const float* __restrict__ pos, const float4* __res
                              pos[pair_index(g, 3)]);
     if (vel_out) vel_out[k] = vel[g];
   }
+  pdl_trigger();
 }
 
 __global__ void fill_padding_kernel(float* __restrict__ pos, float4* __restrict__ vel,
@@ -130,20 +136,20 @@ cudaError_t launch_unpack_state(const float* soa, int64_t n, const int64_t* map,
 
 cudaError_t launch_pack_state(const float* pos, const float4* vel, int64_t n, const int64_t* map,
                               float* soa, cudaStream_t stream) {
-  pack_kernel<<<blocks_for(n), kBlock, 0, stream>>>(pos, vel, n, map, soa);
-  return cudaGetLastError();
+  return launch_dependent(pack_kernel, dim3(blocks_for(n)), dim3(kBlock), 0, stream, pos, vel, n, map,
+                          soa);
 }
 
 cudaError_t launch_pack_accel(const float4* acc, int64_t n, const int64_t* map, float* soa,
                               cudaStream_t stream) {
-  pack_accel_kernel<<<blocks_for(n), kBlock, 0, stream>>>(acc, n, map, soa);
-  return cudaGetLastError();
+  return launch_dependent(pack_accel_kernel, dim3(blocks_for(n)), dim3(kBlock), 0, stream, acc, n,
+                          map, soa);
 }
 
 cudaError_t launch_export(const float* pos, const float4* vel, int64_t n, const int64_t* map,
                           float4* pos_out, float4* vel_out, cudaStream_t stream) {
-  export_kernel<<<blocks_for(n), kBlock, 0, stream>>>(pos, vel, n, map, pos_out, vel_out);
-  return cudaGetLastError();
+  return launch_dependent(export_kernel, dim3(blocks_for(n)), dim3(kBlock), 0, stream, pos, vel, n,
+                          map, pos_out, vel_out);
 }
 
 cudaError_t launch_fill_padding(float* pos, float4* vel, int64_t n_pad_total,
