@@ -107,6 +107,13 @@ __global__ void export_kernel(const float* __restrict__ pos, const float4* __res
   pdl_trigger();
 }
 
+// The error word into pinned host memory: a launch, where a copy of four bytes holds the
+// stream for a copy engine's latency.
+__global__ void read_error_kernel(const int32_t* __restrict__ err, int32_t* __restrict__ host) {
+  pdl_wait();
+  *host = *err;
+}
+
 __global__ void fill_padding_kernel(float* __restrict__ pos, float4* __restrict__ vel,
                                     int64_t n) {
   for (int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; g < n;
@@ -138,6 +145,10 @@ cudaError_t launch_pack_state(const float* pos, const float4* vel, int64_t n, co
                               float* soa, cudaStream_t stream) {
   return launch_dependent(pack_kernel, dim3(blocks_for(n)), dim3(kBlock), 0, stream, pos, vel, n, map,
                           soa);
+}
+
+cudaError_t launch_read_error(const int32_t* err, int32_t* host, cudaStream_t stream) {
+  return launch_dependent(read_error_kernel, dim3(1), dim3(1), 0, stream, err, host);
 }
 
 cudaError_t launch_pack_accel(const float4* acc, int64_t n, const int64_t* map, float* soa,

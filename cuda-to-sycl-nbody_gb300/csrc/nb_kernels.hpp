@@ -85,6 +85,8 @@ cudaError_t launch_unpack_state(const float* soa /*[7][n]: x y z vx vy vz m*/, i
                                 cudaStream_t stream);
 cudaError_t launch_pack_state(const float* pos, const float4* vel, int64_t n, const int64_t* map,
                               float* soa /*[6][n]*/, cudaStream_t stream);
+// The device error word into pinned host memory.
+cudaError_t launch_read_error(const int32_t* err, int32_t* host, cudaStream_t stream);
 cudaError_t launch_pack_accel(const float4* acc, int64_t n, const int64_t* map,
                               float* soa /*[3][n]*/, cudaStream_t stream);
 cudaError_t launch_export(const float* pos, const float4* vel, int64_t n, const int64_t* map,

@@ -80,6 +80,10 @@ struct nb_sim {
   float4* acc_d = nullptr;
   float* staging_d = nullptr;  // [7][n_real]
   int32_t* err_d = nullptr;
+  // Pinned host memory for what goes back to the host: the error word, and behind
+  // kPinnedHead bytes the state of small systems (allocated on first use).
+  unsigned char* pinned = nullptr;
+  size_t pinned_bytes = 0;
   bool per_pair_mass = false;
   int32_t mask_self = 0;
   int32_t inject = 0;  // one-shot failure-detection hook for the next force launch (kInject*)
@@ -187,7 +191,11 @@ constexpr int kPerSystemSimShape = 2;
 // One force evaluation over all systems: integrate into the other position
 // buffer and swap (accel_out == nullptr), or write accelerations.
 int force_pass(nb_sim* s, float4* accel_out, int per_system);
-int check_error_word(nb_sim* s);
+// The error word in two halves, so that one wait serves it and the results: enqueue its
+// read, and judge it once the stream has drained (clearing it if it is set).
+int read_error_word(nb_sim* s);
+int judge_error_word(nb_sim* s);
+int check_error_word(nb_sim* s);  // both, with the wait
 int ensure_staging(nb_sim* s);
 int ensure_accel(nb_sim* s);
 // Upload a symmetric plan for i-tiles of bi particles and make its scratch: rows, and
