@@ -18,7 +18,8 @@
 // per frame with a float4 per pixel and a thread per particle, 269 with a lane per pair
 // of pixels, 220 with the profile evaluated once per column and row (the splat is bound
 // by instructions then: 2 x 2 pixels per sector, a fifth fewer sectors, gain nothing),
-// 194 with the kernels as programmatic dependents and the blur's taps fixed.
+// 198 with the kernels as programmatic dependents and the blur's taps fixed, 185 with the
+// blur's taps as pairs from shared memory and a gamma of its own.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -158,31 +159,69 @@ __device__ __forceinline__ void add2(float2& acc, float2 v, float w) {
 // memory, with the widest tap's reach on both sides.
 constexpr int kBlurX = 256;
 
+// Columns of a CTA's line (even).
+__host__ __device__ constexpr int blur_cols(int reach) { return 2 * kBlurX + 2 * reach + 2; }
+
+// A tap pair of the blur, for a pixel whose own taps start at place p of shared memory:
+// the samples on both sides lie between places p + up, p + up + step and between p + down,
+// p + down + step, mirrored.
+struct TapPair {
+  int up, down;
+  float near, far;  // weights of the inner and the outer place
+};
+
+__device__ __forceinline__ void add_pair(float2& acc, const TapPair& t, float2 near0, float2 near1,
+                                         float2 far0, float2 far1) {
+  acc = __ffma2_rn(__fadd2_rn(near0, near1), make_float2(t.near, t.near), acc);
+  acc = __ffma2_rn(__fadd2_rn(far0, far1), make_float2(t.far, t.far), acc);
+}
+
 // kEven: the source is exactly twice as wide, so a tap lies at the same place between
-// two columns for every pixel.
+// two columns for every pixel: the CTA works its places and weights out once.  Two copies
+// of the line, one shifted by a column, make any two neighbouring columns one 16-byte
+// load.
 template <bool kEven>
 __global__ void __launch_bounds__(kBlurX) blur_x_kernel(const float2* __restrict__ hdr,
                                                         RenderUniforms u, int reach,
                                                         float2* __restrict__ dst,
                                                         double* __restrict__ block_sums) {
-  extern __shared__ float2 line[];
+  extern __shared__ __align__(16) float2 line[];
   __shared__ double sh[kBlurX / 32];
+  __shared__ TapPair taps[kRenderMaxTaps];
+  // Source columns of the CTA: u of its first pixel minus the reach, and so on.
+  const int c0 = 2 * static_cast<int>(blockIdx.x) * kBlurX - reach;
+  const int cols = blur_cols(reach);
+  if (kEven && threadIdx.x < u.taps) {
+    const int i = threadIdx.x;
+    const float at = 0.5f + u.offset[i] * u.size_x * u.bw;
+    const int k = static_cast<int>(at);
+    const float f = at - k;
+    const int odd = (reach + k) & 1;
+    taps[i] = TapPair{odd * (cols - 1) + reach + k, odd * (cols - 1) + reach - k,
+                      u.weight[i] * (1.f - f), u.weight[i] * f};
+  }
   pdl_wait();
   const int x = blockIdx.x * kBlurX + threadIdx.x, y = blockIdx.y;
   const float v = (y + 0.5f) / u.oh * u.bh - 0.5f;
   const float fv = floorf(v);
   const int y0 = min(max(static_cast<int>(fv), 0), u.bh - 1), y1 = min(y0 + 1, u.bh - 1);
   const float b = v - fv;
-  // Source columns of the CTA: u of its first pixel minus the reach, and so on.
-  const int c0 = 2 * static_cast<int>(blockIdx.x) * kBlurX - reach;
-  const int cols = 2 * kBlurX + 2 * reach + 2;
-  // Even and odd columns apart: a warp's samples of one tap are two columns apart.
-  const int half = (cols + 1) / 2;
+  // Not kEven: even and odd columns apart, as a warp's samples of one tap are two columns
+  // apart.
+  const int half = cols / 2;
   auto place = [half](int k) { return (k & 1) * half + (k >> 1); };
+  const float2 *row0 = hdr + static_cast<int64_t>(y0) * u.pitch,
+               *row1 = hdr + static_cast<int64_t>(y1) * u.pitch;
+#pragma unroll 3
   for (int k = threadIdx.x; k < cols; k += kBlurX) {
     const int c = min(max(c0 + k, 0), u.bw - 1);
-    line[place(k)] = lerp2(hdr[static_cast<int64_t>(y0) * u.pitch + c],
-                    hdr[static_cast<int64_t>(y1) * u.pitch + c], b);
+    const float2 l = lerp2(row0[c], row1[c], b);
+    if (kEven) {
+      line[k] = l;
+      if (k > 0) line[cols + k - 1] = l;
+    } else {
+      line[place(k)] = l;
+    }
   }
   __syncthreads();
   double lum = 0.0;
@@ -194,24 +233,29 @@ __global__ void __launch_bounds__(kBlurX) blur_x_kernel(const float2* __restrict
       const int k = static_cast<int>(fu) - c0;
       return lerp2(line[place(k)], line[place(k + 1)], uu - fu);
     };
-    const int k0 = 2 * x - c0;  // kEven: the pixel's centre is k0 + 1/2
-    const float2 c = kEven ? lerp2(line[place(k0)], line[place(k0 + 1)], 0.5f) : sample(s);
-    float2 acc = make_float2(c.x * u.weight[0], c.y * u.weight[0]);
+    float2 acc;
+    if (kEven) {
+      const float2* mine = line + 2 * threadIdx.x;  // the pixel lies between columns
+      const float2 l = mine[reach], r = mine[reach + 1];  // reach and reach + 1
+      const float w = 0.5f * u.weight[0];
+      acc = make_float2((l.x + r.x) * w, (l.y + r.y) * w);
 #pragma unroll 4
-    for (int i = 1; i < u.taps; ++i) {
-      if (kEven) {
-        const float at = 0.5f + u.offset[i] * u.size_x * u.bw;
-        const int k = static_cast<int>(at);
-        const float f = at - k;
-        const float2 p = line[place(k0 + k)], q = line[place(k0 + 1 - k)];
-        const float2 r = line[place(k0 + k + 1)], l = line[place(k0 - k)];
-        add2(acc, lerp2(make_float2(p.x + q.x, p.y + q.y), make_float2(r.x + l.x, r.y + l.y), f),
-             u.weight[i]);
-        continue;
+      for (int i = 1; i < u.taps; ++i) {
+        const TapPair t = taps[i];
+        const float4 p = *reinterpret_cast<const float4*>(mine + t.up);
+        const float4 q = *reinterpret_cast<const float4*>(mine + t.down);
+        add_pair(acc, t, make_float2(p.x, p.y), make_float2(q.z, q.w), make_float2(p.z, p.w),
+                 make_float2(q.x, q.y));
       }
-      const float dx = u.offset[i] * u.size_x;
-      const float2 p = sample(s + dx), q = sample(s - dx);
-      add2(acc, make_float2(p.x + q.x, p.y + q.y), u.weight[i]);
+    } else {
+      const float2 c = sample(s);
+      acc = make_float2(c.x * u.weight[0], c.y * u.weight[0]);
+#pragma unroll 4
+      for (int i = 1; i < u.taps; ++i) {
+        const float dx = u.offset[i] * u.size_x;
+        const float2 p = sample(s + dx), q = sample(s - dx);
+        add2(acc, make_float2(p.x + q.x, p.y + q.y), u.weight[i]);
+      }
     }
     dst[static_cast<int64_t>(y) * u.ow + x] = acc;
     const float2 h = hdr[static_cast<int64_t>(2 * y + 1) * u.pitch + 2 * x + 1];
@@ -247,11 +291,26 @@ __device__ void luminance_mean(const double* __restrict__ block_sums, int64_t co
   if (tid == 0) *mean = static_cast<float>(sh[0] * inv_pixels);
 }
 
-// Vertical pass, at the target's own size: columns stay, rows are interpolated.  The
+// Vertical pass, at the target's own size: columns stay, rows are interpolated.  A CTA is
+// 32 columns of kBlurRows rows, its source rows in shared memory; a thread has
+// kBlurRows / 8 of them, so that a tap's places and weights are read once for all.  The
 // grid's last row of CTAs takes the luminance's mean instead.
+constexpr int kBlurRows = 32;
+
 __global__ void __launch_bounds__(kMeanThreads) blur_y_kernel(
-    const float2* __restrict__ src, RenderUniforms u, const double* __restrict__ block_sums,
-    int64_t parts, float* __restrict__ mean, float2* __restrict__ dst) {
+    const float2* __restrict__ src, RenderUniforms u, int reach,
+    const double* __restrict__ block_sums, int64_t parts, float* __restrict__ mean,
+    float2* __restrict__ dst) {
+  extern __shared__ __align__(16) float2 tile[];
+  __shared__ TapPair taps[kRenderMaxTaps];
+  const int tid = threadIdx.y * 32 + threadIdx.x;
+  if (tid < u.taps) {
+    const float at = u.offset[tid] * u.size_y * u.oh;
+    const int k = static_cast<int>(at);
+    const float f = at - k;
+    taps[tid] = TapPair{(reach + k) * 32, (reach - k) * 32, u.weight[tid] * (1.f - f),
+                        u.weight[tid] * f};
+  }
   pdl_wait();
   pdl_trigger();
   if (blockIdx.y + 1 == gridDim.y) {
@@ -259,56 +318,95 @@ __global__ void __launch_bounds__(kMeanThreads) blur_y_kernel(
       luminance_mean(block_sums, parts, 1.0 / (static_cast<double>(u.lw) * u.lh), mean);
     return;
   }
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= u.ow || y >= u.oh) return;
-  auto row = [&](int k) {
-    return src[static_cast<int64_t>(min(max(y + k, 0), u.oh - 1)) * u.ow + x];
-  };
-  const float2 c = row(0);
-  float2 acc = make_float2(c.x * u.weight[0], c.y * u.weight[0]);
+  const int x = blockIdx.x * 32 + threadIdx.x, xc = min(x, u.ow - 1);
+  const int top = blockIdx.y * kBlurRows - reach;  // row of the tile's first
 #pragma unroll 4
-  for (int i = 1; i < u.taps; ++i) {
-    const float at = u.offset[i] * u.size_y * u.oh;
-    const int k = static_cast<int>(at);
-    const float f = at - k;
-    const float2 p = row(k), q = row(-k), r = row(k + 1), l = row(-k - 1);
-    add2(acc, lerp2(make_float2(p.x + q.x, p.y + q.y), make_float2(r.x + l.x, r.y + l.y), f),
-         u.weight[i]);
+  for (int k = threadIdx.y; k < kBlurRows + 2 * reach; k += 8)
+    tile[k * 32 + threadIdx.x] =
+        src[static_cast<int64_t>(min(max(top + k, 0), u.oh - 1)) * u.ow + xc];
+  __syncthreads();
+  constexpr int kMine = kBlurRows / 8;
+  const float2* mine = tile + tid;  // row r of the thread: 8 r rows further down
+  float2 acc[kMine];
+#pragma unroll
+  for (int r = 0; r < kMine; ++r) {
+    const float2 c = mine[(reach + 8 * r) * 32];
+    acc[r] = make_float2(c.x * u.weight[0], c.y * u.weight[0]);
   }
-  dst[static_cast<int64_t>(y) * u.ow + x] = acc;
+  for (int i = 1; i < u.taps; ++i) {
+    const TapPair t = taps[i];
+    const float2 *up = mine + t.up, *down = mine + t.down;
+#pragma unroll
+    for (int r = 0; r < kMine; ++r)
+      add_pair(acc[r], t, up[r * 256], down[r * 256], up[r * 256 + 32], down[r * 256 - 32]);
+  }
+#pragma unroll
+  for (int r = 0; r < kMine; ++r) {
+    const int y = blockIdx.y * kBlurRows + threadIdx.y + 8 * r;
+    if (x < u.ow && y < u.oh) dst[static_cast<int64_t>(y) * u.ow + x] = acc[r];
+  }
 }
 
-// tonemap.frag: HDR + bloom, exposure from the mean luminance, gamma 2.2.
-__global__ void tonemap_kernel(const float2* __restrict__ hdr, const float2* __restrict__ bloom,
-                               const float* __restrict__ mean, RenderUniforms u,
-                               float4* __restrict__ out) {
-  pdl_wait();
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= u.width || y >= u.height) return;
-  const int cx = x + u.margin, cy = y + u.margin;
-  const float2 c = hdr[static_cast<int64_t>(cy) * u.pitch + cx];
-  const float exposure = 1.f / fminf(fmaxf(*mean * 10.f, 0.2f), 1000.f);
+// r^(1/2.2) = r^(5/11) for r in [0, 1], where r is 0 or at least 2^-24 (one minus a
+// float): the hardware's logarithm and power of two, then one Newton step for y^11 = r^5,
+// whose rounding errors the step divides by 11.  Over every such r within 1.2 ulp
+// of the power in 64 bits; powf(r, 1.f / 2.2f) is within 4.1, and took most of the 375
+// instructions per pixel of the tonemap.
+__device__ __forceinline__ float gamma_22(float r) {
+  r *= 2048.f;  // scales the result by 32: all powers below are normal numbers
+  const float y = exp2f(__log2f(r) * (5.f / 11.f));
+  const float r2 = r * r, r5 = r2 * r2 * r;
+  const float y2 = y * y, y4 = y2 * y2, y8 = y4 * y4;
+  const float z = __fdividef(fmaf(-y8 * y2, y, r5), r5) * (1.f / 11.f);
+  return r == 0.f ? 0.f : fmaf(y, z, y) * (1.f / 32.f);
+}
+
+// tonemap.frag: HDR + bloom, exposure from the mean luminance, gamma 2.2.  Bound by
+// instructions, of which a thread shares the exposure and the columns' places over its
+// kToneRows rows.
+constexpr int kToneRows = 4;
+
+__global__ void __launch_bounds__(256) tonemap_kernel(const float2* __restrict__ hdr,
+                                                      const float2* __restrict__ bloom,
+                                                      const float* __restrict__ mean,
+                                                      RenderUniforms u, float4* __restrict__ out) {
+  const int x = blockIdx.x * 32 + threadIdx.x;
+  const int y0 = blockIdx.y * 8 * kToneRows + threadIdx.y;
+  if (x >= u.width) return;
+  const int cx = x + u.margin;
   const float uu = static_cast<float>(cx) / u.bw * u.ow - 0.5f;
-  const float vv = static_cast<float>(cy) / u.bh * u.oh - 0.5f;
-  const float fu = floorf(uu), fv = floorf(vv);
+  const float per_row = static_cast<float>(u.oh) / u.bh;
+  const float fu = floorf(uu), wu = uu - fu;
   const int x0 = min(max(static_cast<int>(fu), 0), u.ow - 1), x1 = min(x0 + 1, u.ow - 1);
-  const int y0 = min(max(static_cast<int>(fv), 0), u.oh - 1), y1 = min(y0 + 1, u.oh - 1);
-  const float2* r0 = bloom + static_cast<int64_t>(y0) * u.ow;
-  const float2* r1 = bloom + static_cast<int64_t>(y1) * u.ow;
-  const float2 b = lerp2(lerp2(r0[x0], r0[x1], uu - fu), lerp2(r1[x0], r1[x1], uu - fu), vv - fv);
-  const float3 l = light_rgb(c.x + b.x, c.y + b.y);
-  const float r = 1.f - expf(-l.x * exposure);
-  const float g = 1.f - expf(-l.y * exposure);
-  const float bl = 1.f - expf(-l.z * exposure);
-  out[static_cast<int64_t>(y) * u.width + x] =
-      make_float4(powf(r, 1.f / 2.2f), powf(g, 1.f / 2.2f), powf(bl, 1.f / 2.2f), 1.f);
+  pdl_wait();
+  const float exposure = 1.f / fminf(fmaxf(*mean * 10.f, 0.2f), 1000.f);
+#pragma unroll
+  for (int k = 0; k < kToneRows; ++k) {
+    const int y = y0 + 8 * k;
+    if (y >= u.height) return;
+    const int cy = y + u.margin;
+    const float2 c = hdr[static_cast<int64_t>(cy) * u.pitch + cx];
+    const float vv = cy * per_row - 0.5f;
+    const float fv = floorf(vv);
+    const int r0 = min(max(static_cast<int>(fv), 0), u.oh - 1), r1 = min(r0 + 1, u.oh - 1);
+    const float2 *b0 = bloom + static_cast<int64_t>(r0) * u.ow,
+                 *b1 = bloom + static_cast<int64_t>(r1) * u.ow;
+    const float2 b = lerp2(lerp2(b0[x0], b0[x1], wu), lerp2(b1[x0], b1[x1], wu), vv - fv);
+    const float3 l = light_rgb(c.x + b.x, c.y + b.y);
+    out[static_cast<int64_t>(y) * u.width + x] =
+        make_float4(gamma_22(1.f - expf(-l.x * exposure)), gamma_22(1.f - expf(-l.y * exposure)),
+                    gamma_22(1.f - expf(-l.z * exposure)), 1.f);
+  }
 }
 
 // Source columns between a target pixel's centre and its widest tap, rounded up.
 int blur_reach(const RenderUniforms& u) {
   return static_cast<int>(u.offset[u.taps - 1] * u.size_x * u.bw) + 3;
+}
+
+// Rows between a pixel and its widest tap, rounded up.
+int blur_y_reach(const RenderUniforms& u) {
+  return static_cast<int>(u.offset[u.taps - 1] * u.size_y * u.oh) + 2;
 }
 
 }  // namespace
@@ -335,15 +433,28 @@ cudaError_t launch_render(const float* pos, const float4* vel, int64_t n_pad,
   const int reach = blur_reach(u);
   const dim3 gx((u.ow + kBlurX - 1) / kBlurX, u.oh);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  e = launch_dependent(u.bw == 2 * u.ow ? blur_x_kernel<true> : blur_x_kernel<false>, gx, dim3(kBlurX), sizeof(float2) * (2 * kBlurX + 2 * reach + 4),
-                       stream, b.hdr, u, reach, b.blur1, b.block_sums);
+  const bool even = u.bw == 2 * u.ow;
+  e = launch_dependent(even ? blur_x_kernel<true> : blur_x_kernel<false>, gx, dim3(kBlurX),
+                       sizeof(float2) * blur_cols(reach) * (even ? 2 : 1), stream, b.hdr, u, reach,
+                       b.blur1, b.block_sums);
   if (e != cudaSuccess) return e;
   const dim3 blk(32, 8);
-  e = launch_dependent(blur_y_kernel, dim3((u.ow + 31) / 32, (u.oh + 7) / 8 + 1), blk, 0, stream,
-                       b.blur1, u, b.block_sums, render_luminance_parts(u), b.mean, b.blur2);
+  // Images lower than about 60 rows: taps so far apart that the rows need more shared
+  // memory than a kernel has by default (104 KB at 16 rows).
+  const int reach_y = blur_y_reach(u);
+  const int smem_y = static_cast<int>(sizeof(float2)) * 32 * (kBlurRows + 2 * reach_y);
+  if (smem_y > 48 * 1024 &&
+      (e = cudaFuncSetAttribute(blur_y_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                smem_y)) != cudaSuccess)
+    return e;
+  e = launch_dependent(blur_y_kernel, dim3((u.ow + 31) / 32, (u.oh + kBlurRows - 1) / kBlurRows + 1),
+                       blk, smem_y, stream, b.blur1, u, reach_y, b.block_sums,
+                       render_luminance_parts(u), b.mean, b.blur2);
   if (e != cudaSuccess) return e;
-  return launch_dependent(tonemap_kernel, dim3((u.width + 31) / 32, (u.height + 7) / 8), blk, 0,
-                          stream, b.hdr, b.blur2, b.mean, u, out);
+  constexpr int kRows = 8 * kToneRows;
+  return launch_dependent(tonemap_kernel,
+                          dim3((u.width + 31) / 32, (u.height + kRows - 1) / kRows), blk, 0, stream,
+                          b.hdr, b.blur2, b.mean, u, out);
 }
 
 }  // namespace nbg
