@@ -30,18 +30,22 @@ struct RenderUniforms {
 // Light is additive in two terms: a sprite's colour is (t, 0.4 (1 - t) + 0.2 t, 1) times
 // its alpha, so sums of alpha and of alpha t give all three channels (light_rgb).
 struct RenderBuffers {
-  float2* hdr = nullptr;     // pitch x bh
+  float2* hdr = nullptr;     // copies x (pitch x bh); the sum of them in the first
   float2* blur1 = nullptr;   // ow x oh
   float2* blur2 = nullptr;   // ow x oh (bloom)
   double* block_sums = nullptr;
   float* mean = nullptr;
   float* flare = nullptr;    // flare_n x flare_n
   int32_t width = 0, height = 0;
+  int32_t copies = 1;
 };
 
 cudaError_t launch_render(const float* pos, const float4* vel, int64_t n_pad,
                           const RenderUniforms& u, const RenderBuffers& b, float4* out,
                           cudaStream_t stream);
+
+// Copies of the HDR buffer that pay for n particles.
+int render_copies(const RenderUniforms& u, int64_t n);
 
 // Partial luminance sums of a frame.
 int64_t render_luminance_parts(const RenderUniforms& u);

@@ -179,7 +179,10 @@ int nb_sim_render(nb_sim* s, const float view[16], const float proj[16], int32_t
   RenderBuffers& b = s->render;
   if (b.width != width || b.height != height) {
     release_render(b);
-    NB_TRY(dev_alloc(&b.hdr, static_cast<size_t>(u.pitch) * u.bh));
+    const size_t pixels = static_cast<size_t>(u.pitch) * u.bh;
+    b.copies = render_copies(u, static_cast<int64_t>(s->n_real));
+    if (b.copies > 1 && dev_alloc(&b.hdr, pixels * b.copies) != NB_OK) b.copies = 1;
+    if (b.copies == 1) NB_TRY(dev_alloc(&b.hdr, pixels));
     NB_TRY(dev_alloc(&b.blur1, static_cast<size_t>(u.ow) * u.oh));
     NB_TRY(dev_alloc(&b.blur2, static_cast<size_t>(u.ow) * u.oh));
     NB_TRY(dev_alloc(&b.block_sums, static_cast<size_t>(render_luminance_parts(u))));
