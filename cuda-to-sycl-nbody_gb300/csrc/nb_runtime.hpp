@@ -200,7 +200,8 @@ int ensure_staging(nb_sim* s);
 int ensure_accel(nb_sim* s);
 // Upload a symmetric plan for i-tiles of bi particles and make its scratch: rows, and
 // `rec` float4 records per slot and i-particle.
-int upload_symmetric(nb_sim* s, const SymPlanHost& h, int bi, int rec, WorkListDev* out);
+int upload_symmetric(nb_sim* s, const SymPlanHost& h, const KernelShape& sh, int rec,
+                     int diag_cost, int pair_cost, WorkListDev* out);
 // Launch the force kernel with arguments `a` over work list `w`.
 int launch_with(nb_sim* s, ForceArgs a, const WorkListDev& w);
 

@@ -90,7 +90,7 @@ int ensure_adjoint_buffers(nb_sim* s, int32_t ncp, int32_t every) {
     const SymPlanHost h =
         plan_symmetric(s->sys_h.data(), 0, static_cast<int32_t>(s->sys_h.size()), sh.bi(), sh.bj,
                        grid, kSymScratchBytes / kSymRowBytes, kAdjDiagCost, kAdjPairCost);
-    NB_TRY(upload_symmetric(s, h, sh.bi(), 1, &a.wl));
+    NB_TRY(upload_symmetric(s, h, sh, 1, kAdjDiagCost, kAdjPairCost, &a.wl));
   }
   return NB_OK;
 }

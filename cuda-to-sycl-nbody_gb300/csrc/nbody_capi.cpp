@@ -293,7 +293,8 @@ static int plan_tuned(nb_sim* s, int cfg, int32_t first, int32_t count, int grid
   return NB_OK;
 }
 
-int upload_symmetric(nb_sim* s, const SymPlanHost& h, int bi, int rec, WorkListDev* out) {
+int upload_symmetric(nb_sim* s, const SymPlanHost& h, const KernelShape& sh, int rec,
+                     int diag_cost, int pair_cost, WorkListDev* out) {
   WorkListDev w;
   w.grid = h.bands[0].grid;
   w.nseg = static_cast<int32_t>(h.segs.size());
@@ -301,10 +302,11 @@ int upload_symmetric(nb_sim* s, const SymPlanHost& h, int bi, int rec, WorkListD
   w.split = h.split_tiles;
   w.bands = h.bands;
   w.row_values = h.row_values;
-  const std::vector<SymSegment> segs = link_segments(h);
+  const std::vector<SymSegment> segs = link_segments(
+      h, sh.bi() / sh.bj, sh.threads == 32 ? 4 * s->sms : 0, diag_cost, pair_cost);
   int st = dev_alloc(&w.sym_segs, segs.size());
   if (st == NB_OK) st = dev_alloc(&w.sym_tiles, h.tiles.size());
-  if (st == NB_OK) st = ensure_scratch(s, w, bi, rec);
+  if (st == NB_OK) st = ensure_scratch(s, w, sh.bi(), rec);
   if (st != NB_OK) {
     free_worklist(w);
     return st;
@@ -328,7 +330,7 @@ static int plan_sym(nb_sim* s, int cfg, int32_t first, int32_t count, WorkListDe
   const KernelShape sh = shape_of(cfg);
   const SymPlanHost h = plan_symmetric(s->sys_h.data(), first, count, sh.bi(), sh.bj,
                                        max_grid_for(s, cfg), kSymScratchBytes / kSymRowBytes);
-  NB_TRY(upload_symmetric(s, h, sh.bi(), part_records(s, cfg), out));
+  NB_TRY(upload_symmetric(s, h, sh, part_records(s, cfg), kSymDiagCost, kSymPairCost, out));
   out->cfg = cfg;
   return NB_OK;
 }
@@ -566,9 +568,9 @@ static bool sharded(const nb_sim* s) {
 // are measured at N = 1,048,576 (229.9, 251.8, 267.2 and 373.1 ms per step, where all
 // are balanced and nearly nothing is diagonal); the blocks per CTA, at the sizes of
 // single systems where two neighbouring shapes meet (thin disks, us per step with the
-// larger / the smaller i-tiles): 36,000 319 / 315 and 50,000 587 / 598 for 4,096 against
-// 512 particles; 12,800 55.2 / 50.7 and 25,600 167.4 / 172.5 for 512 against 256; 4,096
-// 14.7 / 14.0 and 8,192 25.7 / 30.3 for 256 against 64.
+// larger / the smaller i-tiles): 45,000 484 / 471 and 55,000 683 / 691 for 4,096 against
+// 512 particles; 16,000 74.1 / 70.8 and 17,000 77.4 / 80.1 for 512 against 256; 4,096
+// 12.9 / 11.9 and 5,000 13.9 / 14.6 for 256 against 64.
 static int default_symmetric_for(nb_sim* s, int32_t first, int32_t count) {
   static constexpr double kRates[][2] = {{1.0, 12.0}, {0.913, 7.0}, {0.86, 0.8}, {0.617, 0.0}};
   constexpr int kCount = sizeof(kRates) / sizeof(kRates[0]);

@@ -134,6 +134,7 @@ struct DeviceSetup {
   bool ready = false;
   unsigned char* scratch = nullptr;  // device address of g_noalloc_scratch
   int grid[kNaCount] = {};           // largest grid of each shape
+  int schedulers = 0;
   // The plan in the scratch: for `n` particles, `tag` at its start; n = 0: none.
   uint64_t n = 0;
   uint32_t tag = 0;
@@ -168,6 +169,7 @@ int na_setup(int dev) {
     NB_CUDA(symmetric_xyzm_blocks_per_sm(kNaShapes[k], &blocks));
     d.grid[k] = std::max(1, std::min(blocks * sms, kNaMaxGrid));
   }
+  d.schedulers = 4 * sms;
   d.scratch = static_cast<unsigned char*>(p);
   d.ready = true;
   return NB_OK;
@@ -200,7 +202,8 @@ bool na_plan(const SystemDesc& sd, const DeviceSetup& d, int k, bool copied, Lay
       at->copy = copied ? end : 0;
       if (end + static_cast<size_t>(copy) <= kScratchBytes) {
         g_na_linked.n = static_cast<int>(g_na_plan.segs.size());
-        link_segments_into(g_na_plan, g_na_linked);
+        link_segments_into(g_na_plan, sh.bi() / sh.bj, sh.threads == 32 ? d.schedulers : 0,
+                           kSymDiagCost, kSymPairCost, g_na_linked);
         return true;
       }
     }

@@ -41,9 +41,10 @@ SymPlanHost plan_symmetric(const SystemDesc* sys, int32_t first, int32_t count, 
   return plan;
 }
 
-std::vector<SymSegment> link_segments(const SymPlanHost& plan) {
+std::vector<SymSegment> link_segments(const SymPlanHost& plan, int32_t tiles_per_i,
+                                      int32_t schedulers, int diag_cost, int pair_cost) {
   std::vector<SymSegment> out(plan.segs.size());
-  link_segments_into(plan, out);
+  link_segments_into(plan, tiles_per_i, schedulers, diag_cost, pair_cost, out);
   return out;
 }
 

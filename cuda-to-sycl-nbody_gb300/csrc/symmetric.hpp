@@ -82,7 +82,19 @@ struct SymPlanHost {
 
 // The segments in the order the kernel wants them: per band, the first of every CTA and
 // then the others, linked by `next` (counted from the band's seg0).
-std::vector<SymSegment> link_segments(const SymPlanHost& plan);
+//
+// `schedulers` > 0: CTAs of one warp, more of them than the GPU's warp schedulers.  CTA b
+// then shares its scheduler with b + schedulers and so on (to within a few places, as
+// the clocks at which the warps end show), and of the two the older runs at nearly its
+// full rate, so what counts is the charge per scheduler.  Its units are coarse (N =
+// 8,192: 3 or 4 per CTA, 6.8 per scheduler), so the CTAs are given out by charge,
+// heaviest round first and every other round the other way about (us per step, in list
+// order / by charge: 8,192 25.4 / 23.8, 12,800 50.5 / 47.9, 20,000 107.5 / 103.4; the
+// adjoint at 16,384 133 / 127; 25,600, where 34 units meet 33.2 on average, 163 either
+// way).  `tiles_per_i`: j-tiles per i-tile.
+std::vector<SymSegment> link_segments(const SymPlanHost& plan, int32_t tiles_per_i,
+                                      int32_t schedulers, int diag_cost = kSymDiagCost,
+                                      int pair_cost = kSymPairCost);
 
 // Plan systems [first, first + count) (whole systems, no shards) for i-tiles of bi and
 // j-tiles of bj particles (bi % bj == 0) on at most max_grid CTAs, with at most

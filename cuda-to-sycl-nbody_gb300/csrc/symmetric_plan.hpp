@@ -123,16 +123,42 @@ void plan_symmetric_into(const SystemDesc* sys, int32_t first, int32_t count, in
   }
 }
 
-// `out` holds plan.segs.size() segments.
+// Largest grid that link_segments_into orders (it sorts on the stack).
+constexpr int32_t kSymMaxOrdered = 8192;
+
+// `out` holds plan.segs.size() segments.  The rest as link_segments.
 template <class Plan, class Out>
-void link_segments_into(const Plan& plan, Out& out) {
+void link_segments_into(const Plan& plan, int32_t tiles_per_i, int32_t schedulers, int diag_cost,
+                        int pair_cost, Out& out) {
+  uint64_t order[kSymMaxOrdered];  // charge of a CTA above its index
   for (const SymBand& b : plan.bands) {
+    const auto first = plan.seg_begin.begin() + b.begin0;
+    const bool ordered = schedulers > 0 && b.grid > schedulers && b.grid <= kSymMaxOrdered;
+    for (int32_t k = 0; ordered && k < b.grid; ++k) {
+      uint64_t charge = 0;
+      for (int32_t q = first[k]; q < first[k + 1]; ++q) {
+        const SymSegment& sg = plan.segs[q];
+        const int32_t td = std::max(sg.jt0, std::min(sg.jt1, (sg.itile + 1) * tiles_per_i));
+        charge += static_cast<uint64_t>(td - sg.jt0) * diag_cost +
+                  static_cast<uint64_t>(sg.jt1 - td) * pair_cost + pair_cost / 5;
+      }
+      order[k] = charge << 32 | static_cast<uint32_t>(b.grid - 1 - k);
+    }
+    if (ordered) std::sort(order, order + b.grid);  // backwards: heaviest last
     int32_t more = b.grid;  // the next free place behind the first segments
-    for (int32_t k = 0; k < b.grid; ++k) {
-      int32_t at = k;
-      for (int32_t q = plan.seg_begin[b.begin0 + k]; q < plan.seg_begin[b.begin0 + k + 1]; ++q) {
+    for (int32_t p = 0; p < b.grid; ++p) {
+      int32_t k = p;
+      if (ordered) {
+        // Heaviest round first, its heaviest CTA last; every other round the other way about.
+        const int32_t round = p / schedulers, p0 = round * schedulers;
+        const int32_t len = std::min(schedulers, b.grid - p0);
+        const int32_t rank = round % 2 == 1 ? p : p0 + len - 1 - (p - p0);
+        k = b.grid - 1 - static_cast<int32_t>(order[b.grid - 1 - rank] & 0xffffffffu);
+      }
+      int32_t at = p;
+      for (int32_t q = first[k]; q < first[k + 1]; ++q) {
         SymSegment sg = plan.segs[q];
-        const bool last = q + 1 == plan.seg_begin[b.begin0 + k + 1];
+        const bool last = q + 1 == first[k + 1];
         sg.next = last ? 0 : ++more;
         out[b.seg0 + at] = sg;
         at = sg.next - 1;
