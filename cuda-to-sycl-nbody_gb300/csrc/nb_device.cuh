@@ -38,16 +38,15 @@ cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, s
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// Integrate (or write accelerations for) one real particle.
+// Integrate (or write accelerations for) one real particle at (xi, yi, zi) of velocity v.
 __device__ __forceinline__ void finish_particle(const ForceArgs& a, const SystemDesc& sd,
                                                 int64_t gi, float fx, float fy, float fz,
-                                                float xi, float yi, float zi) {
+                                                float xi, float yi, float zi, float4 v) {
   const float g = sd.gscale;
   if (a.accel_out != nullptr) {
     a.accel_out[gi] = make_float4(fx * g, fy * g, fz * g, 0.f);
     return;
   }
-  float4 v = a.vel[gi];
   // v = v * damping; v += (F * dt) * G   (simulator.cu:214-216)
   v.x = fmaf(fx * a.dt, g, v.x * a.damping);
   v.y = fmaf(fy * a.dt, g, v.y * a.damping);
@@ -58,6 +57,12 @@ __device__ __forceinline__ void finish_particle(const ForceArgs& a, const System
   a.pos_next[pair_index(gi, 1)] = fmaf(v.y, a.dt, yi);
   a.pos_next[pair_index(gi, 2)] = fmaf(v.z, a.dt, zi);
   a.pos_next[pair_index(gi, 3)] = a.pos[pair_index(gi, 3)];
+}
+__device__ __forceinline__ void finish_particle(const ForceArgs& a, const SystemDesc& sd,
+                                                int64_t gi, float fx, float fy, float fz,
+                                                float xi, float yi, float zi) {
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+  finish_particle(a, sd, gi, fx, fy, fz, xi, yi, zi, a.accel_out ? none : a.vel[gi]);
 }
 
 }  // namespace nbg

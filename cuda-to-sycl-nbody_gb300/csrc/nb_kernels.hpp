@@ -44,6 +44,24 @@ cudaError_t launch_symmetric_xyzm(int index, const SymArgs& a, int grid, cudaStr
 cudaError_t launch_symmetric_add(bool compensated, const SymArgs& a, int tiles, int bi,
                                  cudaStream_t stream);
 
+// ---- direct force step of small systems (direct_kernel.cu) ----------------------------
+struct DirectArgs {
+  ForceArgs f;        // pos, pos_next, vel, accel_out, sys, eps2, dt, ...
+  const int2* tiles;  // (system, i-tile) of each CTA; NULL: CTA b is i-tile b of `sys`
+  int32_t sys;
+  int32_t n;          // launch_direct_xyzm: particles, and what their sums are times
+  float gscale;
+};
+int num_direct_shapes();
+// Threads, i-particles of a CTA (every thread holds them all), j-particles per pass, 1.
+KernelShape direct_shape(int index);
+// The shape for `count` systems; *pays: it beats the symmetric kernel.
+int choose_direct(const SystemDesc* sys, int32_t count, int sms, bool* pays);
+cudaError_t launch_direct(int index, bool compensated, bool per_pair_mass, const DirectArgs& a,
+                          int grid, cudaStream_t stream);
+// Positions as for launch_symmetric_xyzm, one system.
+cudaError_t launch_direct_xyzm(int index, const DirectArgs& a, int grid, cudaStream_t stream);
+
 // ---- compatibility kernel (aux_kernels.cu) ------------------------------------------
 // The reference's PREDICATED variant as shipped, one thread per i-particle over one
 // system (simulator.cu:186-229 with the (i == id) mask of :208-209).

@@ -30,6 +30,8 @@ struct WorkListDev {
   int32_t split = 0;
   Segment* segs = nullptr;
   int32_t* seg_begin = nullptr;
+  int2* direct_tiles = nullptr;  // direct kernel: its i-tiles, NULL for one system:
+  int32_t direct_sys = 0;        // this one
   Fixup* fix = nullptr;
   // Symmetric kernel: its segments and i-tiles, and the bands they run in.
   SymSegment* sym_segs = nullptr;

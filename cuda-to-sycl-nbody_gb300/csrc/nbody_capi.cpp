@@ -72,6 +72,7 @@ int check_device(int* sms, cudaDeviceProp* out_prop, int* device) {
 void free_worklist(WorkListDev& w) {
   dev_free(w.segs);
   dev_free(w.seg_begin);
+  dev_free(w.direct_tiles);
   dev_free(w.fix);
   dev_free(w.sym_segs);
   dev_free(w.sym_tiles);
@@ -181,12 +182,18 @@ static void drop_graphs(nb_sim* s) {
   s->retired.clear();
 }
 
-// Config indices: the tuned kernel's shapes, then the symmetric kernel's.
-static int num_configs() { return num_force_configs() + num_symmetric_shapes(); }
-static bool is_symmetric(int cfg) { return cfg >= num_force_configs(); }
+// Config indices: the tuned kernel's shapes, then the symmetric kernel's, then the direct
+// kernel's.
+static int first_direct() { return num_force_configs() + num_symmetric_shapes(); }
+static int num_configs() { return first_direct() + num_direct_shapes(); }
+static bool is_direct(int cfg) { return cfg >= first_direct(); }
+static bool is_symmetric(int cfg) { return cfg >= num_force_configs() && !is_direct(cfg); }
+// Not the tuned kernel: whole systems only, and no bounded waits.
+static bool is_untuned(int cfg) { return cfg >= num_force_configs(); }
 
 // Shape of work-list config `cfg` (>= 0: tuned or symmetric kernel; < 0: reference order).
 static KernelShape shape_of(int cfg) {
+  if (is_direct(cfg)) return direct_shape(cfg - first_direct());
   if (is_symmetric(cfg)) return symmetric_shape(cfg - num_force_configs());
   return cfg >= 0 ? force_config_shape(cfg) : reference_order_shape(-1 - cfg);
 }
@@ -335,10 +342,41 @@ static int plan_sym(nb_sim* s, int cfg, int32_t first, int32_t count, WorkListDe
   return NB_OK;
 }
 
+// The i-tiles of r particles of systems [first, first + count).
+static std::vector<int2> direct_tiles(const SystemDesc* sys, int32_t first, int32_t count, int r) {
+  std::vector<int2> tiles;
+  for (int32_t k = first; k < first + count; ++k)
+    for (int32_t t = 0; t * r < sys[k].n; ++t) tiles.push_back(make_int2(k, t));
+  return tiles;
+}
+
+static int plan_direct(nb_sim* s, int cfg, int32_t first, int32_t count, WorkListDev* out) {
+  const int r = shape_of(cfg).r;
+  WorkListDev w;
+  w.cfg = cfg;
+  w.grid = w.nseg = (s->sys_h[first].n + r - 1) / r;
+  w.direct_sys = first;
+  if (count > 1) {
+    const std::vector<int2> tiles = direct_tiles(s->sys_h.data(), first, count, r);
+    w.grid = w.nseg = static_cast<int32_t>(tiles.size());
+    NB_TRY(dev_alloc(&w.direct_tiles, tiles.size()));
+    cudaError_t e = cudaMemcpyAsync(w.direct_tiles, tiles.data(), tiles.size() * sizeof(int2),
+                                    cudaMemcpyHostToDevice, s->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);  // the host vector dies
+    if (e != cudaSuccess) {
+      free_worklist(w);
+      return cuda_error(e, "upload work list");
+    }
+  }
+  *out = w;
+  return NB_OK;
+}
+
 // Plan systems [first, first + count) for config `cfg` >= 0 at its full grid.
 static int plan_config(nb_sim* s, int cfg, int32_t first, int32_t count, WorkListDev* out) {
-  return is_symmetric(cfg) ? plan_sym(s, cfg, first, count, out)
-                           : plan_tuned(s, cfg, first, count, 0, out);
+  return is_direct(cfg)      ? plan_direct(s, cfg, first, count, out)
+         : is_symmetric(cfg) ? plan_sym(s, cfg, first, count, out)
+                             : plan_tuned(s, cfg, first, count, 0, out);
 }
 
 // (Re)build the all-systems work list for kernel config `cfg`.
@@ -444,8 +482,14 @@ ForceArgs base_args(nb_sim* s) {
 int launch_with(nb_sim* s, ForceArgs a, const WorkListDev& list) {
   a.inject = s->inject;
   s->inject = 0;
-  // The failure hooks make a bounded wait run out; the symmetric kernel has none.
-  const WorkListDev& w = a.inject != 0 && is_symmetric(list.cfg) ? s->inject_wl : list;
+  // The failure hooks make a bounded wait run out; only the tuned kernel has them.
+  const WorkListDev& w = a.inject != 0 && is_untuned(list.cfg) ? s->inject_wl : list;
+  if (is_direct(w.cfg)) {
+    NB_CUDA(launch_direct(w.cfg - first_direct(),
+                          s->params.accumulator == NB_ACC_COMPENSATED, s->per_pair_mass,
+                          DirectArgs{a, w.direct_tiles, w.direct_sys, 0, 0.f}, w.grid, s->stream));
+    return NB_OK;
+  }
   if (is_symmetric(w.cfg)) {
     const int shape = w.cfg - num_force_configs();
     const int bi = shape_of(w.cfg).bi();
@@ -582,11 +626,11 @@ static int default_symmetric_for(nb_sim* s, int32_t first, int32_t count) {
                                                 kSymDiagCost, kSymPairCost);
 }
 
-// Default kernel shape of systems [first, first + count), judged alone: a symmetric one,
-// at every size (thin disks, us per step, tuned / symmetric: N = 64 4.9 / 4.1, 2,048
-// 12.3 / 8.5, 25,600 242 / 167, 262,144 21,712 / 14,494, 1,048,576 346,673 / 229,887;
-// ensembles of 4,096 systems up to 8,192 particles 10,577 / 7,739, of 2,000 up to 300
-// 49.8 / 43.4).  Deterministic (the autotuner may pick otherwise, and shapes round
+// Default kernel shape of systems [first, first + count), judged alone: a direct one
+// where that pays (choose_direct), a symmetric one otherwise (thin disks, us per step,
+// tuned / symmetric: N = 64 4.9 / 3.8, 2,048 12.3 / 7.4, 25,600 242 / 163, 262,144 21,712
+// / 14,420, 1,048,576 346,673 / 228,700; ensembles of 4,096 systems up to 8,192 particles
+// 10,577 / 7,504, of 2,000 up to 300 49.8 / 42.3).  Deterministic (the autotuner may pick otherwise, and shapes round
 // differently).  A shard integrates part of a system against all of it, which is not
 // symmetric, and launches that must fail on purpose need the tuned kernel's waits
 // (`symmetric` false): there, the tuned shape with the largest tiles whose work list
@@ -595,7 +639,11 @@ static int default_symmetric_for(nb_sim* s, int32_t first, int32_t count) {
 // autotuner's pick among the tuned shapes: N = 25,600 -> 256 x 2 x 256 (0.24 ms, the 1M
 // shape takes 0.32), 65,536 -> 256 x 4 x 1024, 262,144 and 1M -> 256 x 4 x 2048.
 static int default_config_for(nb_sim* s, int32_t first, int32_t count, bool symmetric) {
-  if (symmetric && !sharded(s)) return default_symmetric_for(s, first, count);
+  if (symmetric && !sharded(s)) {
+    bool pays = false;
+    const int shape = choose_direct(s->sys_h.data() + first, count, s->sms, &pays);
+    return pays ? first_direct() + shape : default_symmetric_for(s, first, count);
+  }
   static const int kCandidates[] = {9, 8, 10, 3, 4};  // largest tiles first
   for (const int cfg : kCandidates) {
     const KernelShape sh = force_config_shape(cfg);
@@ -616,7 +664,7 @@ static int build_default_worklist(nb_sim* s) {
   const int32_t nsys = static_cast<int32_t>(s->sys_h.size());
   int cfg = default_config_for(s, 0, nsys);
   int st = build_main_worklist(s, cfg);
-  if (st == NB_ERR_OUT_OF_MEMORY && is_symmetric(cfg)) {
+  if (st == NB_ERR_OUT_OF_MEMORY && is_untuned(cfg)) {
     cfg = default_config_for(s, 0, nsys, false);
     st = build_main_worklist(s, cfg);
   }
@@ -1155,8 +1203,9 @@ int nb_sim_set_kernel_config(nb_sim* s, int32_t index) {
   if (index < -1 || index >= num_configs())
     return set_error(NB_ERR_INVALID_ARGUMENT, "bad config index");
   if (index < 0) return build_default_worklist(s);
-  if (is_symmetric(index) && sharded(s))
-    return set_error(NB_ERR_INVALID_ARGUMENT, "the symmetric shapes need the whole system");
+  if (is_untuned(index) && sharded(s))
+    return set_error(NB_ERR_INVALID_ARGUMENT,
+                     "the symmetric and direct shapes need the whole system");
   NB_TRY(build_main_worklist(s, index));
   s->cfg = index;
   s->cfg_default = false;
@@ -1213,9 +1262,16 @@ int nb_sim_autotune(nb_sim* s, int32_t* chosen) {
   }
   int best = s->cfg;
   float best_ms = 1e30f;
-  for (int c = 0; c < (sharded(s) ? num_force_configs() : num_configs()); ++c) {
+  // The direct kernel evaluates a pair twice: no candidate where pairs are all that counts
+  // (100 systems of 8.7e8 pairs: 359 to 401 us per step, the symmetric kernel 224).
+  double pairs = 0;
+  for (const SystemDesc& d : s->sys_h) pairs += static_cast<double>(d.n) * d.n;
+  const int configs = sharded(s)    ? num_force_configs()
+                      : pairs > 1e9 ? first_direct()
+                                    : num_configs();
+  for (int c = 0; c < configs; ++c) {
     const int st = build_main_worklist(s, c);
-    if (st == NB_ERR_OUT_OF_MEMORY && is_symmetric(c)) continue;  // no room for its rows
+    if (st == NB_ERR_OUT_OF_MEMORY && is_untuned(c)) continue;  // no room for its rows
     NB_TRY(st);
     s->cfg = c;
     NB_TRY(force_pass(s, s->acc_d, kPerSystemNone));  // warm-up
@@ -1268,6 +1324,27 @@ int nb_plan_work(uint32_t num_systems, const uint32_t* sizes, int32_t config_ind
   }
   const bool tuned = config_index >= 0;
   const KernelShape sh = shape_of(config_index);
+  if (is_direct(config_index)) {
+    int64_t ctas = 0;  // one per i-tile
+    for (const SystemDesc& q : sys) ctas += (q.n + sh.r - 1) / sh.r;
+    if (ctas > max_grid)
+      return set_error(NB_ERR_INVALID_ARGUMENT,
+                       "the direct kernel has a CTA per i-tile: max_grid is too small");
+    const std::vector<int2> tiles =
+        direct_tiles(sys.data(), 0, static_cast<int32_t>(num_systems), sh.r);
+    const int32_t count = static_cast<int32_t>(ctas);
+    if (grid) *grid = count;
+    if (num_segments) *num_segments = count;
+    if (num_fixups) *num_fixups = 0;
+    if (num_partial_slots) *num_partial_slots = 0;
+    if (segments && max_segments < count)
+      return set_error(NB_ERR_INVALID_ARGUMENT, "segments buffer too small");
+    for (int32_t k = 0; segments && k < count; ++k)
+      segments[k] = nb_segment{tiles[k].x, tiles[k].y, 0,
+                               (sys[tiles[k].x].npad + sh.bj - 1) / sh.bj, -1, 0};
+    for (int32_t k = 0; seg_begin && k <= count; ++k) seg_begin[k] = k;
+    return NB_OK;
+  }
   if (is_symmetric(config_index)) {
     // One band: the list of a simulation whose rows fit the scratch.
     const SymPlanHost h = plan_symmetric(sys.data(), 0, static_cast<int32_t>(num_systems), sh.bi(),
@@ -1334,7 +1411,7 @@ int nb_sim_set_shard(nb_sim* s, uint64_t first, uint64_t count) {
   d.shard_count = (first == 0 && count == n) ? 0 : static_cast<int32_t>(count);
   NB_TRY(upload_systems(s));
   // The symmetric shapes need the whole system.
-  if (s->cfg_default || (sharded(s) && is_symmetric(s->cfg)))
+  if (s->cfg_default || (sharded(s) && is_untuned(s->cfg)))
     NB_TRY(build_default_worklist(s));
   else
     NB_TRY(build_main_worklist(s, s->cfg));
@@ -1462,7 +1539,7 @@ int nb_sim_inject_failure(nb_sim* s, int32_t kind) {
     return set_error(NB_ERR_STATE, "the failure hooks cover the BRANCH kernels only");
   if (kind == NB_INJECT_HAND_OVER_WITHHELD && !reference_order_mode(s))
     return set_error(NB_ERR_STATE, "hand-overs exist in NB_ACC_REFERENCE_ORDER only");
-  if (is_symmetric(s->cfg) && s->inject_wl.segs == nullptr) {
+  if (is_untuned(s->cfg) && s->inject_wl.segs == nullptr) {
     const int32_t nsys = static_cast<int32_t>(s->sys_h.size());
     NB_TRY(plan_tuned(s, default_config_for(s, 0, nsys, false), 0, nsys, 0, &s->inject_wl));
   }

@@ -12,7 +12,8 @@
 // list, the partial sums and the rows of j-side sums -- lives in one file-scope device
 // array, kScratchBytes (13 MiB) long; larger systems run in bands of i-tiles that take
 // turns in it (20,000 particles 223 us per call with the tuned kernel and its list
-// uploaded on every call, 154 now).  Every GPU that loads this module keeps that array
+// uploaded on every call, 149 now).  Small systems run the direct kernel, which needs
+// none of it.  Every GPU that loads this module keeps that array
 // until the process exits.  All calls share it and it keeps the last call's contents:
 // the work list stays for the next call of the same size, checked by a tag that is read
 // back with every call.  Two calls whose work overlapped on the GPU would race on it, so
@@ -134,7 +135,7 @@ struct DeviceSetup {
   bool ready = false;
   unsigned char* scratch = nullptr;  // device address of g_noalloc_scratch
   int grid[kNaCount] = {};           // largest grid of each shape
-  int schedulers = 0;
+  int sms = 0;
   // The plan in the scratch: for `n` particles, `tag` at its start; n = 0: none.
   uint64_t n = 0;
   uint32_t tag = 0;
@@ -169,7 +170,7 @@ int na_setup(int dev) {
     NB_CUDA(symmetric_xyzm_blocks_per_sm(kNaShapes[k], &blocks));
     d.grid[k] = std::max(1, std::min(blocks * sms, kNaMaxGrid));
   }
-  d.schedulers = 4 * sms;
+  d.sms = sms;
   d.scratch = static_cast<unsigned char*>(p);
   d.ready = true;
   return NB_OK;
@@ -202,7 +203,7 @@ bool na_plan(const SystemDesc& sd, const DeviceSetup& d, int k, bool copied, Lay
       at->copy = copied ? end : 0;
       if (end + static_cast<size_t>(copy) <= kScratchBytes) {
         g_na_linked.n = static_cast<int>(g_na_plan.segs.size());
-        link_segments_into(g_na_plan, sh.bi() / sh.bj, sh.threads == 32 ? d.schedulers : 0,
+        link_segments_into(g_na_plan, sh.bi() / sh.bj, sh.threads == 32 ? 4 * d.sms : 0,
                            kSymDiagCost, kSymPairCost, g_na_linked);
         return true;
       }
@@ -284,6 +285,29 @@ extern "C" int nb_accelerations_noalloc(const float* pos_xyzm_device, uint64_t n
   const uintptr_t in = reinterpret_cast<uintptr_t>(pos_xyzm_device);
   const uintptr_t out = reinterpret_cast<uintptr_t>(accel_xyzw_device);
   const bool copied = in < out + 16 * n && out < in + 16 * n;
+  SystemDesc whole{};
+  whole.n = static_cast<int32_t>(n);
+  bool direct = false;
+  const int small = choose_direct(&whole, 1, d.sms, &direct);
+  if (direct) {
+    // One launch without a plan.
+    DirectArgs a{};
+    a.f.pos = pos_xyzm_device;
+    if (copied) {
+      d.n = 0;  // the copy takes the plan's place
+      NB_CUDA(cudaMemcpyAsync(d.scratch, pos_xyzm_device, 16 * n, cudaMemcpyDeviceToDevice, st));
+      a.f.pos = reinterpret_cast<const float*>(d.scratch);
+    }
+    a.f.accel_out = reinterpret_cast<float4*>(accel_xyzw_device);
+    a.f.eps2 = dist_eps;
+    a.f.mask_self = dist_eps * dist_eps * dist_eps >= FLT_MIN ? 0 : 1;
+    a.n = whole.n;
+    a.gscale = G;
+    const int r = direct_shape(small).r;
+    NB_CUDA(launch_direct_xyzm(small, a, (whole.n + r - 1) / r, st));
+    NB_CUDA(cudaStreamSynchronize(st));
+    return NB_OK;
+  }
   // Twice where the scratch does not hold the plan any more (a device reset).
   for (int attempt = 0; attempt < 2; ++attempt) {
     if (d.n != n || d.G != G || d.copied != copied) NB_TRY(na_upload(d, n, G, copied, st));

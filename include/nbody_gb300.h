@@ -104,7 +104,8 @@ typedef struct nb_kernel_info {
   int32_t particles_per_thread; /* i-particles held in registers per thread */
   int32_t j_tile;               /* j-particles per shared-memory tile       */
   int32_t stages;               /* depth of the shared-memory tile ring; 0 for the
-                                   symmetric kernel, whose tiles stay in registers */
+                                   symmetric and 1 for the direct kernel, whose
+                                   j-particles pass through registers */
   int32_t grid;                 /* persistent CTAs per launch               */
   int32_t segments;             /* work-list entries                        */
   int32_t split_tiles;          /* i-tiles whose j-range spans several CTAs */
@@ -283,15 +284,17 @@ int nb_sim_load_state_block(nb_sim* s, uint64_t first, uint64_t count, int32_t w
 /* ---- kernel selection ---------------------------------------------------------- */
 /* The compiled kernel shapes (index 0 .. nb_num_kernel_configs() - 1): first those of
  * the tuned kernel, then those of the symmetric kernel (nb_kernel_info.stages = 0),
- * which evaluates each unordered pair once and applies it to both particles;
+ * which evaluates each unordered pair once and applies it to both particles, then
+ * those of the direct kernel (stages = 1) for small systems, whose CTAs each take
+ * particles_per_thread particles through to the integration;
  * nb_kernel_config_info and nb_plan_work also take -1 - k for shape k of the
  * reference-order kernel.  No reference counterpart: the reference launches
  * ceil(N / gwSize) blocks of gwSize threads (simulator.cu:49-50), and gwSize is only
  * reported here (nb_sim_gw_size). */
 int nb_num_kernel_configs(void);
 int nb_kernel_config_info(int32_t index, nb_kernel_info* info);
-/* Select a kernel shape by index (-1 = the built-in default for this size, a symmetric
- * shape except for shards, which need the tuned kernel).  With
+/* Select a kernel shape by index (-1 = the built-in default for this size, a direct or
+ * symmetric shape except for shards, which need the tuned kernel).  With
  * NB_ACC_REFERENCE_ORDER the index selects one of the reference-order kernel's
  * shapes (0 = the largest i-tiles; nb_sim_kernel_info reports it as -1 - index). */
 int nb_sim_set_kernel_config(nb_sim* s, int32_t index);
@@ -311,7 +314,9 @@ int nb_sim_autotune(nb_sim* s, int32_t* chosen);
  * only in a system's last, partly filled i-tile); a block of the reference-order
  * kernel costs its j-tile length.  The symmetric kernel's list holds the blocks on and
  * above the diagonal, i-tile I against the j-tiles from its own first particle on; a
- * block costs its j-tile length times 11 inside the i-tile and 14 behind it.  `segments`
+ * block costs its j-tile length times 11 inside the i-tile and 14 behind it.  The direct
+ * kernel has one CTA per i-tile of particles_per_thread particles: fewer than that many
+ * CTAs (max_grid) are an error.  `segments`
  * (capacity max_segments) and `seg_begin` (capacity max_grid + 1) may be NULL to
  * query the counts only.  No reference counterpart (the reference launches one
  * thread per particle, simulator.cu:49-50). */
