@@ -10,6 +10,7 @@
 // 152 SMs; 1.2 us of pairs in 4.2).
 #include <cuda_runtime.h>
 
+#include "direct.cuh"
 #include "nb_device.cuh"
 #include "nb_kernels.hpp"
 
@@ -158,34 +159,13 @@ __global__ void __launch_bounds__(W * 32, B) direct_kernel(const DirectArgs a) {
         direct_meet<P, kMass, false>(nx, ny, nz, ax, ay, az, x1, y1, z1, m1, e2, 0);
       }
     }
-    // The warp's sums: halve the particles a lane holds while it adds its partner's, then add
-    // over the lanes that hold the same one (lane / (32 / R)).
     float t[R][3];
 #pragma unroll
     for (int p = 0; p < P; ++p) {
       t[2 * p][0] = ax[p].x, t[2 * p][1] = ay[p].x, t[2 * p][2] = az[p].x;
       t[2 * p + 1][0] = ax[p].y, t[2 * p + 1][1] = ay[p].y, t[2 * p + 1][2] = az[p].y;
     }
-    int cnt = R;
-#pragma unroll
-    for (int m = 16; m > 0; m >>= 1) {
-      const bool upper = (lane & m) != 0;
-      if (cnt > 1) {
-        cnt /= 2;
-#pragma unroll
-        for (int k = 0; k < R / 2; ++k)
-          if (k < cnt)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              const float give = upper ? t[k][c] : t[k + cnt][c];
-              const float keep = upper ? t[k + cnt][c] : t[k][c];
-              t[k][c] = keep + __shfl_xor_sync(0xffffffffu, give, m);
-            }
-      } else {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) t[0][c] += __shfl_xor_sync(0xffffffffu, t[0][c], m);
-      }
-    }
+    warp_sums<R>(t);
 #pragma unroll
     for (int c = 0; c < 3; ++c) sum[c].add(t[0][c]);
   }
@@ -257,7 +237,8 @@ KernelShape direct_shape(int index) {
 // 2.0 1.7 1.7 1.9 2.9; 2,048 4.2 4.8 5.5 8.7 15.3; 4,096 10.5 9.8 10.6 16.6 29.7; 40
 // systems up to 512 8.3 5.4 5.4 4.5 6.1, 16 up to 2,048 12.4 9.7 9.5 10.3 15.8, 100 up to
 // 512 19.5 12.1 10.4 8.4 7.7.
-int choose_direct(const SystemDesc* sys, int32_t count, int sms, bool* pays) {
+int choose_direct(const SystemDesc* sys, int32_t count, int sms, double max_pairs,
+                  int64_t max_tiles, bool* pays) {
   double pairs = 0;
   int64_t t4 = 0, t8 = 0;
   int32_t longest = 0;
@@ -267,7 +248,7 @@ int choose_direct(const SystemDesc* sys, int32_t count, int sms, bool* pays) {
     t8 += (sys[k].n + 7) / 8;
     longest = sys[k].n > longest ? sys[k].n : longest;
   }
-  *pays = pairs <= 2.2e7 && t8 <= 16000;
+  *pays = pairs <= max_pairs && t8 <= max_tiles;
   if (t8 <= 2 * sms && longest >= 512) return 0;
   if (t4 <= 7 * sms) return 1;
   if (t8 <= 5 * sms || longest > 1024) return 2;

@@ -55,8 +55,14 @@ struct DirectArgs {
 int num_direct_shapes();
 // Threads, i-particles of a CTA (every thread holds them all), j-particles per pass, 1.
 KernelShape direct_shape(int index);
-// The shape for `count` systems; *pays: it beats the symmetric kernel.
-int choose_direct(const SystemDesc* sys, int32_t count, int sms, bool* pays);
+// The shape for `count` systems; *pays: they have at most max_pairs pairs and max_tiles
+// i-tiles of 8 particles.  Up to these the direct kernel beats the symmetric one:
+constexpr double kDirectPairs = 2.2e7;
+constexpr int64_t kDirectTiles = 16000;
+constexpr double kAdjDirectPairs = 6.5e6;  // the same of the adjoint
+constexpr int64_t kAdjDirectTiles = 5000;
+int choose_direct(const SystemDesc* sys, int32_t count, int sms, double max_pairs,
+                  int64_t max_tiles, bool* pays);
 cudaError_t launch_direct(int index, bool compensated, bool per_pair_mass, const DirectArgs& a,
                           int grid, cudaStream_t stream);
 // Positions as for launch_symmetric_xyzm, one system.
@@ -152,6 +158,9 @@ KernelShape adjoint_shape(int index);  // threads, i-particles per thread, j-til
 cudaError_t adjoint_blocks_per_sm(int index, bool per_pair_mass, int* blocks);
 cudaError_t launch_adjoint(int index, bool per_pair_mass, const AdjointArgs& a, int grid,
                            cudaStream_t stream);
+// Small systems: shape `index` of choose_direct, its i-tiles as in DirectArgs.
+cudaError_t launch_adjoint_direct(int index, bool per_pair_mass, const AdjointArgs& a,
+                                  const int2* tiles, int sys, int grid, cudaStream_t stream);
 // Add the rows and parts of the band's i-tiles and write lam_x_out and lam_v_out.
 cudaError_t launch_adjoint_add(const AdjointArgs& a, int tiles, int bi, cudaStream_t stream);
 // n x 3 interleaved (user order) <-> padded float4.

@@ -54,7 +54,8 @@ struct AdjointState {
   float4* mu = nullptr;
   float4* tmp = nullptr;
   float4* vel = nullptr;            // velocities of the recomputed segment
-  int shape = 0;                    // of the pair kernel
+  bool direct = false;              // the direct kernel
+  int shape = 0;                    // of it or of the pair kernel
   WorkListDev wl;                   // its list (the scratch is the simulation's)
   bool valid = false;
 };
@@ -204,6 +205,8 @@ int ensure_accel(nb_sim* s);
 // `rec` float4 records per slot and i-particle.
 int upload_symmetric(nb_sim* s, const SymPlanHost& h, const KernelShape& sh, int rec,
                      int diag_cost, int pair_cost, WorkListDev* out);
+// The direct kernels' list: a CTA per i-tile of r particles of systems [first, first + count).
+int plan_direct(nb_sim* s, int r, int32_t first, int32_t count, WorkListDev* out);
 // Launch the force kernel with arguments `a` over work list `w`.
 int launch_with(nb_sim* s, ForceArgs a, const WorkListDev& w);
 

@@ -69,7 +69,7 @@ int ensure_adjoint_buffers(nb_sim* s, int32_t ncp, int32_t every) {
     a.ckpt_vel.push_back(v);
   }
   if (!a.vel) NB_TRY(dev_alloc(&a.vel, np));
-  while (static_cast<int32_t>(a.seg_pos.size()) < every) {
+  while (static_cast<int32_t>(a.seg_pos.size()) < every - 1) {
     float* p = nullptr;
     NB_TRY(dev_alloc(&p, 4 * np));
     // Padding particles must sit far away with zero mass in every buffer the
@@ -83,13 +83,23 @@ int ensure_adjoint_buffers(nb_sim* s, int32_t ncp, int32_t every) {
     NB_TRY(dev_alloc(&a.mu, np));
     NB_TRY(dev_alloc(&a.tmp, np));
   }
-  if (a.wl.bands.empty()) {
+  if (a.wl.grid == 0) {
+    const int32_t nsys = static_cast<int32_t>(s->sys_h.size());
+    bool pays = false;
+    // A pair of the adjoint is twice the work of a force's, so the line lies lower (us per
+    // backward step, symmetric / direct): 512 particles 6.9 / 3.7, 1,024 7.1 / 4.7, 2,048
+    // 9.0 / 8.0, 2,432 10.2 / 9.0, 3,000 11.9 / 12.6; ensembles of 6e6 pairs in 4,708
+    // i-tiles of 8 18.2 / 14.2, 7e6 in 1,720 13.8 / 15.9, 1.1e7 in 1,270 14.7 / 18.4.
+    a.shape = choose_direct(s->sys_h.data(), nsys, s->sms, kAdjDirectPairs, kAdjDirectTiles,
+                            &pays);
+    a.direct = pays;
+    if (a.direct) return plan_direct(s, direct_shape(a.shape).r, 0, nsys, &a.wl);
     int grid = 0;
     a.shape = adjoint_shape_for(s, &grid);
     const KernelShape sh = adjoint_shape(a.shape);
     const SymPlanHost h =
-        plan_symmetric(s->sys_h.data(), 0, static_cast<int32_t>(s->sys_h.size()), sh.bi(), sh.bj,
-                       grid, kSymScratchBytes / kSymRowBytes, kAdjDiagCost, kAdjPairCost);
+        plan_symmetric(s->sys_h.data(), 0, nsys, sh.bi(), sh.bj, grid,
+                       kSymScratchBytes / kSymRowBytes, kAdjDiagCost, kAdjPairCost);
     NB_TRY(upload_symmetric(s, h, sh, 1, kAdjDiagCost, kAdjPairCost, &a.wl));
   }
   return NB_OK;
@@ -225,22 +235,23 @@ static int adjoint_backward_stream(nb_sim* s, const float* gx_T, const float* gv
   for (int32_t k = a.count - 1; k >= 0; --k) {
     const int32_t t0 = k * a.every;
     const int32_t L = std::min(a.every, a.T - t0);
-    // Recompute the positions x_{t0} .. x_{t0+L-1} from the checkpoint.
-    NB_CUDA(cudaMemcpyAsync(a.seg_pos[0], a.ckpt_pos[k], 4 * np * sizeof(float),
-                            cudaMemcpyDeviceToDevice, s->stream));
-    NB_CUDA(cudaMemcpyAsync(a.vel, a.ckpt_vel[k], np * sizeof(float4), cudaMemcpyDeviceToDevice,
-                            s->stream));
+    // Recompute the positions x_{t0+1} .. x_{t0+L-1} from the checkpoint's, which are
+    // x_{t0}; each step of the recomputation replaces the velocities.
+    if (L > 1)
+      NB_CUDA(cudaMemcpyAsync(a.vel, a.ckpt_vel[k], np * sizeof(float4), cudaMemcpyDeviceToDevice,
+                              s->stream));
+    auto at = [&](int32_t t) { return t == 0 ? a.ckpt_pos[k] : a.seg_pos[t - 1]; };
     for (int32_t t = 0; t + 1 < L; ++t) {
       ForceArgs fa = base_args(s);
-      fa.pos = a.seg_pos[t];
-      fa.pos_next = a.seg_pos[t + 1];
+      fa.pos = at(t);
+      fa.pos_next = at(t + 1);
       fa.vel = a.vel;
       NB_TRY(launch_with(s, fa, s->wl));
     }
     // Reverse through the segment.
     for (int32_t t = L - 1; t >= 0; --t) {
       AdjointArgs aa{};
-      aa.pos = a.seg_pos[t];
+      aa.pos = at(t);
       aa.lam_x = a.lam_x;
       aa.lam_v = a.lam_v;
       aa.lam_x_out = a.tmp;
@@ -255,6 +266,9 @@ static int adjoint_backward_stream(nb_sim* s, const float* gx_T, const float* gv
       aa.dt = dt;
       aa.damping = s->params.damping;
       aa.mask_self = s->mask_self;
+      if (a.direct)
+        NB_CUDA(launch_adjoint_direct(a.shape, s->per_pair_mass, aa, a.wl.direct_tiles,
+                                      a.wl.direct_sys, a.wl.grid, s->stream));
       for (const SymBand& b : a.wl.bands) {
         aa.segs = a.wl.sym_segs + b.seg0;
         aa.tile0 = b.tile0;

@@ -350,10 +350,8 @@ static std::vector<int2> direct_tiles(const SystemDesc* sys, int32_t first, int3
   return tiles;
 }
 
-static int plan_direct(nb_sim* s, int cfg, int32_t first, int32_t count, WorkListDev* out) {
-  const int r = shape_of(cfg).r;
+int plan_direct(nb_sim* s, int r, int32_t first, int32_t count, WorkListDev* out) {
   WorkListDev w;
-  w.cfg = cfg;
   w.grid = w.nseg = (s->sys_h[first].n + r - 1) / r;
   w.direct_sys = first;
   if (count > 1) {
@@ -374,9 +372,13 @@ static int plan_direct(nb_sim* s, int cfg, int32_t first, int32_t count, WorkLis
 
 // Plan systems [first, first + count) for config `cfg` >= 0 at its full grid.
 static int plan_config(nb_sim* s, int cfg, int32_t first, int32_t count, WorkListDev* out) {
-  return is_direct(cfg)      ? plan_direct(s, cfg, first, count, out)
-         : is_symmetric(cfg) ? plan_sym(s, cfg, first, count, out)
-                             : plan_tuned(s, cfg, first, count, 0, out);
+  if (is_direct(cfg)) {
+    NB_TRY(plan_direct(s, shape_of(cfg).r, first, count, out));
+    out->cfg = cfg;
+    return NB_OK;
+  }
+  return is_symmetric(cfg) ? plan_sym(s, cfg, first, count, out)
+                           : plan_tuned(s, cfg, first, count, 0, out);
 }
 
 // (Re)build the all-systems work list for kernel config `cfg`.
@@ -641,7 +643,8 @@ static int default_symmetric_for(nb_sim* s, int32_t first, int32_t count) {
 static int default_config_for(nb_sim* s, int32_t first, int32_t count, bool symmetric) {
   if (symmetric && !sharded(s)) {
     bool pays = false;
-    const int shape = choose_direct(s->sys_h.data() + first, count, s->sms, &pays);
+    const int shape = choose_direct(s->sys_h.data() + first, count, s->sms, kDirectPairs,
+                                    kDirectTiles, &pays);
     return pays ? first_direct() + shape : default_symmetric_for(s, first, count);
   }
   static const int kCandidates[] = {9, 8, 10, 3, 4};  // largest tiles first

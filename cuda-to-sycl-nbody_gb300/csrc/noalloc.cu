@@ -288,7 +288,7 @@ extern "C" int nb_accelerations_noalloc(const float* pos_xyzm_device, uint64_t n
   SystemDesc whole{};
   whole.n = static_cast<int32_t>(n);
   bool direct = false;
-  const int small = choose_direct(&whole, 1, d.sms, &direct);
+  const int small = choose_direct(&whole, 1, d.sms, kDirectPairs, kDirectTiles, &direct);
   if (direct) {
     // One launch without a plan.
     DirectArgs a{};
