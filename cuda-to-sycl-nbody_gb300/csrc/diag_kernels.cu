@@ -77,17 +77,18 @@ __global__ void __launch_bounds__(kDiagThreads) moments_kernel(
 
 // ---- potential, pairs in two floats -------------------------------------------------
 // The potential needs N^2 / 2 inverse square roots in double precision, about 30 FP64
-// operations per pair on a pipe of 2 lanes per SM (FP32: 128; a third-order step from the FP32 root is no faster
-// than rsqrt: its conversions run on that pipe too).  Here a pair's term is a
-// sum of two floats (packed FP32x2, two j-particles per register pair): the coordinate
+// operations per pair on a pipe of 2 lanes per SM (FP32: 128; a third-order step from the
+// FP32 root is no faster than rsqrt: its conversions run on that pipe too).  Here a pair's
+// term is a sum of two floats (packed FP32x2, two j-particles per register pair): the coordinate
 // differences are exact (TwoSum), the squared distance and the root carry 47 bits or
 // more (two Newton steps on the MUFU rsqrt, residuals by fused multiply-add), and 128
 // terms at a time are added error-free before they go to FP64.  About 90 FP32 lane
 // operations per pair.  Errors of single terms (below 1e-14) average out over a
 // system's pairs, and the sums are no further from exact ones than the FP64 kernel's,
 // whose threads add thousands of terms one after another (RMS over disks and spheres,
-// equal and own masses, FP64 / split: 1.6e-16 / 1.2e-16 at N = 6,000, 2.0e-16 / 1.6e-16
-// at 10,011, 5.6e-16 / 2.2e-16 at 65,536).  N = 65,536: 103.5 ms before, 7.6 now.
+// equal and own masses: FP64 2.0e-16 and 1.7e-16 at N = 10,011, 4.9e-16 and 5.6e-16 at
+// 65,536; split 1.2e-16 and 8.5e-17, 1.9e-16 and 1.7e-16).  N = 65,536: 103.5 ms before,
+// 7.6 now.
 // Systems below kSplitMin particles, softenings below kSplitEps and values out of the
 // split's range keep the FP64 kernel; an i-tile whose particles are nearly at one place,
 // where all terms are rounded alike and nothing averages out, is summed in FP64 too.

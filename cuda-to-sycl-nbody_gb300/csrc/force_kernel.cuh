@@ -1,5 +1,7 @@
 // All-pairs softened-gravity force + fused integrate step for sm_103a (kernel template;
-// force_kernel.cu holds the table of compiled shapes).
+// force_kernel.cu holds the table of compiled shapes).  Whole systems run the symmetric
+// kernel (symmetric_kernel.cuh) or, small ones, the direct one (direct_kernel.cu) by
+// default; this one serves shards and the autotuner.
 //
 // Semantics follow the reference kernel particle_interaction<BRANCH>
 // (src/simulator.cu:186-229):

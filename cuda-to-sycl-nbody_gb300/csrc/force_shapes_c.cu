@@ -1,6 +1,6 @@
 // Force kernel shapes 8-12: large j-tiles (1024 and 2048 particles, 48-96 KB of tile
 // ring), which amortise the per-tile barrier, bulk-copy issue and Kahan step.
-// 9 (256 x 4, 2048-particle tiles) is the default for large systems; 11 and 12
+// 9 (256 x 4, 2048-particle tiles) is the default for shards of large systems; 11 and 12
 // (128 x 4, 512-particle i-tiles, two CTAs per SM) suit ensembles of uneven systems,
 // whose i-tiles waste fewer lanes on padding.
 #include "force_kernel.cuh"

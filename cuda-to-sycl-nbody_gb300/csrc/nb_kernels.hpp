@@ -33,6 +33,8 @@ struct SymArgs {
 };
 int num_symmetric_shapes();
 KernelShape symmetric_shape(int index);  // threads, i-particles per thread, j-tile, 0 stages
+// Compiled with compensated sums only for these masses (the faster kernel).
+bool symmetric_always_compensates(int index, bool per_pair_mass);
 cudaError_t symmetric_blocks_per_sm(int index, bool compensated, bool per_pair_mass, int* blocks);
 cudaError_t launch_symmetric(int index, bool compensated, bool per_pair_mass, const SymArgs& a,
                              int grid, cudaStream_t stream);

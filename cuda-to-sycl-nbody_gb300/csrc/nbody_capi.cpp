@@ -217,8 +217,16 @@ static int grow(nb_sim* s, T** p, size_t* cap, size_t need) {
 // Records per slot and i-particle of config `cfg`: (hi, lo) for the compensated tuned
 // and symmetric kernels, one otherwise (the reference-order kernel's hand-over holds one
 // float4 per particle).
+// Whether config `cfg` keeps compensated sums: in COMPENSATED mode, and in PLAIN where the
+// compensated kernel is the faster one.
+static bool compensates(const nb_sim* s, int cfg) {
+  return s->params.accumulator == NB_ACC_COMPENSATED ||
+         (is_symmetric(cfg) &&
+          symmetric_always_compensates(cfg - num_force_configs(), s->per_pair_mass));
+}
+
 static int part_records(const nb_sim* s, int cfg) {
-  return cfg >= 0 && s->params.accumulator == NB_ACC_COMPENSATED ? 2 : 1;
+  return cfg >= 0 && compensates(s, cfg) ? 2 : 1;
 }
 
 static int ensure_scratch(nb_sim* s, const WorkListDev& w, int bi, int rec) {
@@ -237,7 +245,7 @@ static int ensure_scratch(nb_sim* s, const WorkListDev& w, int bi, int rec) {
 
 static int max_grid_for(nb_sim* s, int cfg, bool live = false) {
   int blocks = 0;
-  const bool comp = s->params.accumulator == NB_ACC_COMPENSATED;
+  const bool comp = compensates(s, cfg);
   cudaError_t e;
   if (is_symmetric(cfg))
     e = symmetric_blocks_per_sm(cfg - num_force_configs(), comp, s->per_pair_mass, &blocks);
@@ -495,7 +503,7 @@ int launch_with(nb_sim* s, ForceArgs a, const WorkListDev& list) {
   if (is_symmetric(w.cfg)) {
     const int shape = w.cfg - num_force_configs();
     const int bi = shape_of(w.cfg).bi();
-    const bool comp = s->params.accumulator == NB_ACC_COMPENSATED;
+    const bool comp = compensates(s, w.cfg);
     SymArgs sa{};
     sa.f = a;
     sa.tiles = w.sym_tiles;
@@ -867,8 +875,7 @@ void nb_params_default(nb_params* p) {
   p->dist_eps = 1.0e-7f;
   p->gw_size = 64;
   p->calc_method = NB_BRANCH;
-  p->accumulator = NB_ACC_COMPENSATED;  // faster than plain at the default shape, and ~200x
-                                        // more accurate at N = 1M
+  p->accumulator = NB_ACC_COMPENSATED;  // the more accurate sums, for a few percent at most
 }
 
 int nb_params_parse_args(nb_params* p, int argc, const char* const* argv) {

@@ -6,9 +6,10 @@
 // What bounds it: the FP32 FMA pipe.  One side of a pair costs 11 lane operations
 // (force_kernel.cuh); both sides cost 14, because only the three multiply-adds of the
 // sum are repeated: 7 per interaction.  Measured, ms per step against the tuned kernel
-// (compensated, equal masses): N = 1,048,576 230.2 (347.1), 262,144 14.5 (21.7), 100,003
-// with per-particle masses, plain 2.52 (3.56), 25,600 0.167 (0.242); 80 % of the FMA pipe
-// at 1,048,576.
+// (compensated, equal masses): N = 1,048,576 229.2 (347.1), 262,144 14.42 (21.7), 100,003
+// with per-particle masses, plain 2.52 (3.56), 25,600 0.163 (0.242); the FMA pipe is 84 %
+// busy at 262,144 and 77 % at 25,600 (one-warp CTAs: two warps per scheduler, of which the
+// older runs at its full rate and the younger in its gaps until it is alone).
 //
 //   * Each thread holds 2 P i-particles, two per packed FP32x2 register pair.  A warp
 //     takes 32 j-particles at a time, one per lane, and rotates them through its lanes
@@ -30,8 +31,8 @@
 //     only, over all ordered pairs.  The self pair is masked there when eps2^3
 //     underflows, as in force_kernel.cuh.
 //   * Both kernels are launched as programmatic dependents: the next one is resident, its
-//     list loaded, when its predecessor ends (2,048 particles 12.3 -> 8.5 us per step,
-//     12,800 57.5 -> 50.7).
+//     list loaded, when its predecessor ends (12,800
+//     particles 57.5 -> 50.7 us per step).
 //   * Lanes past the end of a system hold a particle at kFarAway: its terms are zero.
 #pragma once
 

@@ -48,9 +48,9 @@ struct SymEntry {
 
 #define NBG_SYM(NW, P, U)                                                                         \
   {NW, P, kSymBJ<NW>,                                                                             \
-   {{launch_one<NW, P, U, false, false, false>, launch_one<NW, P, U, false, true, false>},        \
+   {{launch_one<NW, P, U, NW == 8, false, false>, launch_one<NW, P, U, false, true, false>},      \
     {launch_one<NW, P, U, true, false, false>, launch_one<NW, P, U, true, true, false>}},         \
-   {{occ_one<NW, P, U, false, false, false>, occ_one<NW, P, U, false, true, false>},              \
+   {{occ_one<NW, P, U, NW == 8, false, false>, occ_one<NW, P, U, false, true, false>},            \
     {occ_one<NW, P, U, true, false, false>, occ_one<NW, P, U, true, true, false>}},               \
    launch_one<NW, P, U, false, true, true>, occ_one<NW, P, U, false, true, true>}
 
@@ -64,6 +64,14 @@ int num_symmetric_shapes() { return static_cast<int>(sizeof(kShapes) / sizeof(kS
 KernelShape symmetric_shape(int index) {
   const SymEntry& e = kShapes[index];
   return KernelShape{e.warps * 32, 2 * e.pairs, e.bj, 0};
+}
+
+// 8 warps with equal masses: plain sums take longer than compensated ones, whose pair loop
+// ptxas schedules better (us per step, plain / compensated: 65,536 particles 977 / 954,
+// 262,144 14,925 / 14,420, 1,048,576 237,354 / 229,182).  With masses of their own, and
+// in the shapes of one warp, plain is as fast or faster.
+bool symmetric_always_compensates(int index, bool per_pair_mass) {
+  return kShapes[index].warps == 8 && !per_pair_mass;
 }
 
 cudaError_t symmetric_blocks_per_sm(int index, bool compensated, bool per_pair_mass, int* blocks) {

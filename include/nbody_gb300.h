@@ -53,15 +53,16 @@ typedef enum nb_status {
 typedef enum nb_calc_method { NB_BRANCH = 0, NB_PREDICATED = 1 } nb_calc_method;
 
 /* Per-particle force accumulator; the pair arithmetic is FP32 in every mode.
- * PLAIN and COMPENSATED run the tuned kernel, which sums each particle's terms in
- * its own order (COMPENSATED keeps a Kahan-compensated FP32 running sum).
+ * PLAIN and COMPENSATED run kernels that sum each particle's terms in their own
+ * order (COMPENSATED keeps Kahan-compensated FP32 running sums; PLAIN may, where that
+ * is as fast).
  * REFERENCE_ORDER sums them the way particle_interaction<BRANCH> does
  * (simulator.cu:196-207: one FP32 running sum over j in index order, the same
  * contracted operations), so on the same GPU its results are bit-identical to the
  * reference kernel's; it needs equal masses within each system (the reference has
  * unit masses) and does not use the kernel shapes or the autotuner.
- * nb_params_default selects COMPENSATED: at the tuned kernel's default shape it is
- * both faster than PLAIN and far more accurate. */
+ * nb_params_default selects COMPENSATED: the more accurate, at the speed of PLAIN or
+ * within a few percent of it. */
 typedef enum nb_accumulator {
   NB_ACC_PLAIN = 0,
   NB_ACC_COMPENSATED = 1,
