@@ -619,14 +619,15 @@ static bool sharded(const nb_sim* s) {
 }
 
 // Default symmetric-kernel config for systems [first, first + count).  The shapes' rates
-// are measured at N = 1,048,576 (229.9, 251.8, 267.2 and 373.1 ms per step, where all
+// are measured at N = 1,048,576 (228.5, 250.4, 277.6 and 373.1 ms per step, where all
 // are balanced and nearly nothing is diagonal); the blocks per CTA, at the sizes of
 // single systems where two neighbouring shapes meet (thin disks, us per step with the
-// larger / the smaller i-tiles): 45,000 484 / 471 and 55,000 683 / 691 for 4,096 against
-// 512 particles; 16,000 74.1 / 70.8 and 17,000 77.4 / 80.1 for 512 against 256; 4,096
-// 12.9 / 11.9 and 5,000 13.9 / 14.6 for 256 against 64.
+// larger / the smaller i-tiles): 45,000 484 / 481 and 50,000 583 / 590 for 4,096 against
+// 512 particles; 17,000 80.4 / 83.2 and 20,000 105.8 / 110.7 for 512 against 256, from
+// 17,850 on, where the longer chains of the larger tiles are no longer than the tuned
+// kernel's; 4,096 12.9 / 11.9 and 5,000 14.2 / 14.8 for 256 against 64.
 static int default_symmetric_for(nb_sim* s, int32_t first, int32_t count) {
-  static constexpr double kRates[][2] = {{1.0, 12.0}, {0.913, 7.0}, {0.86, 0.8}, {0.617, 0.0}};
+  static constexpr double kRates[][2] = {{1.0, 12.0}, {0.913, 8.2}, {0.823, 0.8}, {0.613, 0.0}};
   constexpr int kCount = sizeof(kRates) / sizeof(kRates[0]);
   SymCandidate c[kCount];
   for (int k = 0; k < kCount; ++k)
@@ -638,9 +639,9 @@ static int default_symmetric_for(nb_sim* s, int32_t first, int32_t count) {
 
 // Default kernel shape of systems [first, first + count), judged alone: a direct one
 // where that pays (choose_direct), a symmetric one otherwise (thin disks, us per step,
-// tuned / symmetric: N = 64 4.9 / 3.8, 2,048 12.3 / 7.4, 25,600 242 / 163, 262,144 21,712
-// / 14,420, 1,048,576 346,673 / 228,700; ensembles of 4,096 systems up to 8,192 particles
-// 10,577 / 7,504, of 2,000 up to 300 49.8 / 42.3).  Deterministic (the autotuner may pick otherwise, and shapes round
+// tuned / symmetric: N = 64 4.9 / 3.8, 2,048 12.3 / 7.4, 25,600 242 / 166, 262,144 21,712
+// / 14,420, 1,048,576 346,673 / 228,500; ensembles of 4,096 systems up to 8,192 particles
+// 10,577 / 7,655, of 2,000 up to 300 49.8 / 42.3).  Deterministic (the autotuner may pick otherwise, and shapes round
 // differently).  A shard integrates part of a system against all of it, which is not
 // symmetric, and launches that must fail on purpose need the tuned kernel's waits
 // (`symmetric` false): there, the tuned shape with the largest tiles whose work list

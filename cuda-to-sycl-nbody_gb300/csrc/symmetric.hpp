@@ -91,7 +91,7 @@ struct SymPlanHost {
 // heaviest round first and every other round the other way about (us per step, in list
 // order / by charge: 8,192 25.4 / 23.8, 12,800 50.5 / 47.9, 20,000 107.5 / 103.4; the
 // adjoint at 16,384 133 / 127; 25,600, where 34 units meet 33.2 on average, 163 either
-// way).  `tiles_per_i`: j-tiles per i-tile.
+// way; measured before the sums' chains were shortened).  `tiles_per_i`: j-tiles per i-tile.
 std::vector<SymSegment> link_segments(const SymPlanHost& plan, int32_t tiles_per_i,
                                       int32_t schedulers, int diag_cost = kSymDiagCost,
                                       int pair_cost = kSymPairCost);

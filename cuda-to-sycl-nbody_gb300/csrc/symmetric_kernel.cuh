@@ -6,8 +6,8 @@
 // What bounds it: the FP32 FMA pipe.  One side of a pair costs 11 lane operations
 // (force_kernel.cuh); both sides cost 14, because only the three multiply-adds of the
 // sum are repeated: 7 per interaction.  Measured, ms per step against the tuned kernel
-// (compensated, equal masses): N = 1,048,576 229.2 (347.1), 262,144 14.42 (21.7), 100,003
-// with per-particle masses, plain 2.52 (3.56), 25,600 0.163 (0.242); the FMA pipe is 84 %
+// (compensated, equal masses): N = 1,048,576 228.5 (347.1), 262,144 14.42 (21.7), 100,003
+// with per-particle masses, plain 2.52 (3.56), 25,600 0.166 (0.242); the FMA pipe is 84 %
 // busy at 262,144 and 77 % at 25,600 (one-warp CTAs: two warps per scheduler, of which the
 // older runs at its full rate and the younger in its gaps until it is alone).
 //
@@ -21,8 +21,10 @@
 //     Two j-particles in the packed registers against duplicated i-particles take 12
 //     shuffles for the same pairs and hold half the i-particles: 71 % of the FMA pipe in
 //     the pair loop alone, against 79 to 82 %.
-//   * The i-side sums stay in registers over the segment's j-range, folded once per
-//     j-tile into (compensated) running sums in shared memory.
+//   * The i-side sums stay in registers over the segment's j-range, folded every F
+//     j-particles into (compensated) running sums in shared memory; the j-side sums start
+//     anew every S rotations.  No chain of additions is longer than the tuned kernel's at
+//     the same size (symmetric_shapes.cu has the errors).
 //   * The j-side sums of a j-tile are added over the CTA's warps in shared memory, in
 //     warp order (double-buffered, one barrier per j-tile), and written to the i-tile's
 //     row of scratch.  symmetric_add_kernel adds a particle's rows and its i-side parts
@@ -32,7 +34,7 @@
 //     underflows, as in force_kernel.cuh.
 //   * Both kernels are launched as programmatic dependents: the next one is resident, its
 //     list loaded, when its predecessor ends (12,800
-//     particles 57.5 -> 50.7 us per step).
+//     particles 57.5 -> 50.7 us per step when both were new; 49.2 now).
 //   * Lanes past the end of a system hold a particle at kFarAway: its terms are zero.
 #pragma once
 
@@ -51,23 +53,16 @@ namespace {
 
 constexpr int kSymChunk = 32;  // j-particles a warp rotates at a time
 
-// j-particles between two folds of the i-side sums.  A thread's sums are one chain each
-// between folds: no longer than in the tuned kernel's shapes for the same sizes.
-template <int NW>
-constexpr int kSymFold = NW == 8 ? 512 : 128;
-
 // j-tile: what several warps add up at once; one chunk where a CTA is one warp, which
 // writes its rows itself (and whose work lists are cut more finely).
 template <int NW>
 constexpr int kSymBJ = NW == 1 ? kSymChunk : 128;
 
-__device__ __forceinline__ float2 sym_neg(float2 a) { return make_float2(-a.x, -a.y); }
-
-// Kahan step on both lanes: (s, c) += t, with s - c the compensated value.
+// Kahan step on both lanes: (s, c) += t, with s + c the compensated value.
 __device__ __forceinline__ void sym_kahan(float2& s, float2& c, float2 t) {
-  const float2 y = __fadd2_rn(t, sym_neg(c));
+  const float2 y = __fadd2_rn(t, c);
   const float2 u = __fadd2_rn(s, y);
-  c = __fadd2_rn(__fadd2_rn(u, sym_neg(s)), sym_neg(y));
+  c = __fadd2_rn(y, __ffma2_rn(u, make_float2(-1.f, -1.f), s));
   s = u;
 }
 
@@ -102,13 +97,14 @@ struct SymI {
 // i-particles.  kPair: both sides (jx, jy, jz return the sums of r * s over the i
 // side, to be subtracted from j's force); else the i side only.  kMask: leave out the
 // pair with j == i, by index: jj is the lane's j, li the thread's i-particles.
-template <int P, int U, bool kMass, bool kPair, bool kMask>
+template <int P, int U, int S, bool kMass, bool kPair, bool kMask>
 __device__ __forceinline__ void sym_chunk(SymI<P>& q, const float2* mi, float x, float y, float z,
                                           float m, float2 e2, float& jx, float& jy, float& jz,
                                           int jj, int li0, int threads) {
   const int lane = threadIdx.x & 31;
   const int src = (lane + 1) & 31;
   float2 fx = make_float2(0.f, 0.f), fy = fx, fz = fx;
+  jx = jy = jz = 0.f;
 #pragma unroll 1
   for (int k = 0; k < kSymChunk; k += U) {
 #pragma unroll
@@ -154,8 +150,15 @@ __device__ __forceinline__ void sym_chunk(SymI<P>& q, const float2* mi, float x,
         fz.y = sym_rot(fz.y, src);
       }
     }
+    if (kPair && S < kSymChunk && (S == U || (k + U) % S == 0)) {
+      const int by = (lane + S) & 31;
+      jx = sym_rot(jx, by) + (fx.x + fx.y);
+      jy = sym_rot(jy, by) + (fy.x + fy.y);
+      jz = sym_rot(jz, by) + (fz.x + fz.y);
+      fx = fy = fz = make_float2(0.f, 0.f);
+    }
   }
-  if (kPair) {
+  if (kPair && S == kSymChunk) {
     jx = fx.x + fx.y;
     jy = fy.x + fy.y;
     jz = fz.x + fz.y;
@@ -164,15 +167,17 @@ __device__ __forceinline__ void sym_chunk(SymI<P>& q, const float2* mi, float x,
 
 }  // namespace
 
-// NW warps, P i-pairs per thread (i-tiles of 64 P NW particles).
+// NW warps, P i-pairs per thread (i-tiles of 64 P NW particles), U rotations per unrolled
+// block, S per sum of the j side (every one of them moves with its j-particle), F j-particles
+// per fold of the i side.
 // kXyzm: positions are a float4 (x, y, z, m) per particle, and no padding follows them.
-template <int NW, int P, int U, bool kComp, bool kMass, bool kXyzm>
+template <int NW, int P, int U, int S, int F, bool kComp, bool kMass, bool kXyzm>
 __global__ void __launch_bounds__(NW * 32, 8 / NW) symmetric_kernel(const SymArgs a) {
   constexpr int T = NW * 32;
   constexpr int BI = T * 2 * P;
   constexpr int BJ = kSymBJ<NW>;
-  constexpr int kFoldTiles = kSymFold<NW> / BJ;
-  static_assert(BI % BJ == 0 && kSymFold<NW> % BJ == 0, "i-tiles and folds hold whole j-tiles");
+  constexpr int kFoldTiles = F / BJ;
+  static_assert(BI % BJ == 0 && F % BJ == 0, "i-tiles and folds hold whole j-tiles");
   extern __shared__ __align__(16) float sym_smem[];
   // Running i-side sums: [kComp ? 6 : 3][P] float2 per thread, and the j-side sums of
   // the warps: [2][NW][3][BJ] (one warp writes its row of scratch directly).
@@ -247,7 +252,7 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) symmetric_kernel(const SymArg
         fetch(j0 + (c + 1) * kSymChunk);
         float jx, jy, jz;
         if (!diag) {
-          sym_chunk<P, U, kMass, true, false>(q, mi, x, y, z, m, e2, jx, jy, jz, j, 0, T);
+          sym_chunk<P, U, S, kMass, true, false>(q, mi, x, y, z, m, e2, jx, jy, jz, j, 0, T);
           if (NW == 1) {
             if (j < sg.n) {
               a.rows[sg.row + j] = jx;
@@ -260,9 +265,10 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) symmetric_kernel(const SymArg
             jb[2 * BJ + c * kSymChunk + lane] = jz;
           }
         } else if (a.f.mask_self) {
-          sym_chunk<P, 1, kMass, false, true>(q, mi, x, y, z, m, e2, jx, jy, jz, j, ibase + tid, T);
+          sym_chunk<P, 1, S, kMass, false, true>(q, mi, x, y, z, m, e2, jx, jy, jz, j, ibase + tid,
+                                                 T);
         } else {
-          sym_chunk<P, U, kMass, false, false>(q, mi, x, y, z, m, e2, jx, jy, jz, j, 0, T);
+          sym_chunk<P, U, S, kMass, false, false>(q, mi, x, y, z, m, e2, jx, jy, jz, j, 0, T);
         }
       }
       // Fold the i-side sums (never where the segment is short: they stay in registers).
@@ -310,8 +316,8 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) symmetric_kernel(const SymArg
       part[i0 * kRec] = make_float4(sx.x, sy.x, sz.x, 0.f);
       part[i1 * kRec] = make_float4(sx.y, sy.y, sz.y, 0.f);
       if (kComp) {
-        part[i0 * kRec + 1] = make_float4(-cx.x, -cy.x, -cz.x, 0.f);
-        part[i1 * kRec + 1] = make_float4(-cx.y, -cy.y, -cz.y, 0.f);
+        part[i0 * kRec + 1] = make_float4(cx.x, cy.x, cz.x, 0.f);
+        part[i1 * kRec + 1] = make_float4(cx.y, cy.y, cz.y, 0.f);
       }
     }
     if (!kTop && next > 0) sg = a.segs[next - 1];
