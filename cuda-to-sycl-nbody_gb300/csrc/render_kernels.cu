@@ -66,12 +66,19 @@ __global__ void __launch_bounds__(kSplatThreads) splat_kernel(
   const int lane = threadIdx.x & 31;
   // Texels per pixel along each axis: a sprite is flare_x * bw by flare_y * bh pixels.
   const float scale_x = n / (u.flare_x * u.bw), scale_y = n / (u.flare_y * u.bh);
+  // Pixels are counted from the middle of the image, where most sprites are: there the last
+  // bit of a coordinate is worth least.  (x + 1) / 2 bw - 1/2 = half x + rest + middle; the middle
+  // column is even, as pairs of pixels start at even ones.
+  const int mid_x = u.bw / 4 * 2, mid_y = u.bh / 2;
+  const float half_x = 0.5f * u.bw, half_y = 0.5f * u.bh;
+  const float rest_x = half_x - mid_x - 0.5f, rest_y = half_y - mid_y - 0.5f;
+  hdr += static_cast<int64_t>(mid_y) * u.pitch + mid_x;
   constexpr int kWarps = kSplatThreads / 32;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kWarps * per_warp;
   for (int64_t base = (static_cast<int64_t>(blockIdx.x) * kWarps + threadIdx.x / 32) * per_warp;
        base < n_pad; base += stride) {
     const int64_t g = base + lane;
-    float sx = 0.f, sy = 0.f, t = 0.f;  // the quad's lower corner in pixels, the colour mix
+    float sx = 0.f, sy = 0.f, t = 0.f;  // the quad's lower corner, the colour mix
     int kx0 = 0, kx1 = -1, ky0 = 0, ky1 = -1;
     if (lane < per_warp && g < n_pad) {
       const float px = pos[pair_index(g, 0)], py = pos[pair_index(g, 1)],
@@ -82,20 +89,22 @@ __global__ void __launch_bounds__(kSplatThreads) splat_kernel(
       const float cy = M[1] * px + M[5] * py + M[9] * pz + M[13];
       const float cz = M[2] * px + M[6] * py + M[10] * pz + M[14];
       const float cw = M[3] * px + M[7] * py + M[11] * pz + M[15];
-      const float x0 = cx / cw - u.flare_x, x1 = cx / cw + u.flare_x;
-      const float y0 = cy / cw - u.flare_y, y1 = cy / cw + u.flare_y;
+      const float xc = cx / cw, yc = cy / cw;
+      const float x0 = xc - u.flare_x, x1 = xc + u.flare_x;
+      const float y0 = yc - u.flare_y, y1 = yc + u.flare_y;
       if (!padding && cw > 0.f && !(cz < -cw || cz > cw) && x1 > -1.f && x0 < 1.f && y1 > -1.f &&
           y0 < 1.f) {
         // slow -> blue, fast -> purple; the velocity attribute carries w = 1 (renderer_gl.cpp:169)
         const float4 v = vel[g];
         t = fminf(fmaxf((v.x * v.x + v.y * v.y + v.z * v.z + 1.f) * 0.0006f, 0.f), 1.f);
         // pixel centres (k + 0.5) inside [x0, x1) in NDC
-        sx = (x0 + 1.f) * 0.5f * u.bw - 0.5f;
-        sy = (y0 + 1.f) * 0.5f * u.bh - 0.5f;
-        kx0 = max(0, static_cast<int>(ceilf(sx)));
-        kx1 = min(u.bw - 1, static_cast<int>(ceilf((x1 + 1.f) * 0.5f * u.bw - 0.5f)) - 1);
-        ky0 = max(0, static_cast<int>(ceilf(sy)));
-        ky1 = min(u.bh - 1, static_cast<int>(ceilf((y1 + 1.f) * 0.5f * u.bh - 0.5f)) - 1);
+        const float ex = u.flare_x * half_x, ey = u.flare_y * half_y;
+        sx = fmaf(xc, half_x, rest_x - ex);
+        sy = fmaf(yc, half_y, rest_y - ey);
+        kx0 = max(-mid_x, static_cast<int>(ceilf(sx)));
+        kx1 = min(u.bw - 1 - mid_x, static_cast<int>(ceilf(fmaf(xc, half_x, rest_x + ex))) - 1);
+        ky0 = max(-mid_y, static_cast<int>(ceilf(sy)));
+        ky1 = min(u.bh - 1 - mid_y, static_cast<int>(ceilf(fmaf(yc, half_y, rest_y + ey))) - 1);
       }
     }
     unsigned todo = __ballot_sync(0xffffffffu, kx0 <= kx1 && ky0 <= ky1);
