@@ -444,7 +444,8 @@ cudaError_t launch_adjoint_add(const AdjointArgs& a, int tiles, int bi, cudaStre
   if (static_cast<int64_t>(tiles) * bi < kManyParticles)
     return launch_dependent(adjoint_add_kernel<32, 8>, add_grid<32>(tiles, bi), 256, 0, stream, a,
                             bi);
-  return launch_dependent(adjoint_add_kernel<64, 2>, add_grid<64>(tiles, bi), 128, 0, stream, a, bi);
+  return launch_dependent(adjoint_add_kernel<64, 2>, add_grid<64>(tiles, bi), 128, 0, stream, a,
+                          bi);
 }
 
 cudaError_t launch_unpack_vec3(const float* in, int64_t n, const int64_t* map, float4* out,

@@ -19,7 +19,8 @@
 // of pixels, 220 with the profile evaluated once per column and row (the splat is bound
 // by instructions then: 2 x 2 pixels per sector, a fifth fewer sectors, gain nothing),
 // 198 with the kernels as programmatic dependents and the blur's taps fixed, 185 with the
-// blur's taps as pairs from shared memory and a gamma of its own.
+// blur's taps as pairs from shared memory and a gamma of its own (187 with the sprites'
+// corners rounded more finely).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -113,8 +114,10 @@ __global__ void __launch_bounds__(kSplatThreads) splat_kernel(
       todo &= todo - 1;
       const float qx = __shfl_sync(0xffffffffu, sx, src), qy = __shfl_sync(0xffffffffu, sy, src);
       const float qt = __shfl_sync(0xffffffffu, t, src);
-      const int x_lo = __shfl_sync(0xffffffffu, kx0, src), x_hi = __shfl_sync(0xffffffffu, kx1, src);
-      const int y_lo = __shfl_sync(0xffffffffu, ky0, src), y_hi = __shfl_sync(0xffffffffu, ky1, src);
+      const int x_lo = __shfl_sync(0xffffffffu, kx0, src);
+      const int x_hi = __shfl_sync(0xffffffffu, kx1, src);
+      const int y_lo = __shfl_sync(0xffffffffu, ky0, src);
+      const int y_hi = __shfl_sync(0xffffffffu, ky1, src);
       const int p0 = x_lo >> 1, np = (x_hi >> 1) - p0 + 1, rows = y_hi - y_lo + 1;
       if (np <= 8 && rows <= 16) {
         // The usual sprite: the lanes evaluate the profile once per column and row, and
@@ -494,8 +497,8 @@ cudaError_t launch_render(const float* pos, const float4* vel, int64_t n_pad,
       (e = cudaFuncSetAttribute(blur_y_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 smem_y)) != cudaSuccess)
     return e;
-  e = launch_dependent(blur_y_kernel, dim3((u.ow + 31) / 32, (u.oh + kBlurRows - 1) / kBlurRows + 1),
-                       blk, smem_y, stream, b.blur1, u, reach_y, b.block_sums,
+  const dim3 gy((u.ow + 31) / 32, (u.oh + kBlurRows - 1) / kBlurRows + 1);
+  e = launch_dependent(blur_y_kernel, gy, blk, smem_y, stream, b.blur1, u, reach_y, b.block_sums,
                        render_luminance_parts(u), b.mean, b.blur2);
   if (e != cudaSuccess) return e;
   constexpr int kRows = 8 * kToneRows;
