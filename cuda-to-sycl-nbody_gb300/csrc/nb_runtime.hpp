@@ -195,9 +195,9 @@ constexpr int kPerSystemSimShape = 2;
 // buffer and swap (accel_out == nullptr), or write accelerations.
 int force_pass(nb_sim* s, float4* accel_out, int per_system);
 // The error word in two halves, so that one wait serves it and the results: enqueue its
-// read, and judge it once the stream has drained (clearing it if it is set).
+// read, and settle it once the stream has drained (clearing it if it is set).
 int read_error_word(nb_sim* s);
-int judge_error_word(nb_sim* s);
+int settle_error_word(nb_sim* s);
 int check_error_word(nb_sim* s);  // both, with the wait
 int ensure_staging(nb_sim* s);
 int ensure_accel(nb_sim* s);

@@ -592,7 +592,7 @@ int read_error_word(nb_sim* s) {
   return NB_OK;
 }
 
-int judge_error_word(nb_sim* s) {
+int settle_error_word(nb_sim* s) {
   int32_t err = 0;
   std::memcpy(&err, s->pinned, sizeof(err));
   if (err != 0) {
@@ -611,7 +611,7 @@ int judge_error_word(nb_sim* s) {
 int check_error_word(nb_sim* s) {
   NB_TRY(read_error_word(s));
   NB_CUDA(cudaStreamSynchronize(s->stream));
-  return judge_error_word(s);
+  return settle_error_word(s);
 }
 
 static bool sharded(const nb_sim* s) {
@@ -1057,7 +1057,7 @@ int nb_sim_time_iterations(nb_sim* s, int32_t iterations, int32_t per_system, fl
   NB_TRY(read_error_word(s));
   NB_CUDA(cudaStreamSynchronize(s->stream));
   NB_CUDA(cudaEventElapsedTime(ms, s->ev0, s->ev1));
-  return judge_error_word(s);
+  return settle_error_word(s);
 }
 
 int nb_sim_step(nb_sim* s) {
@@ -1085,7 +1085,7 @@ int nb_sim_get_state(nb_sim* s, float* x, float* y, float* z, float* vx, float* 
     NB_CUDA(cudaStreamSynchronize(s->stream));
     for (int c = 0; c < 6; ++c)
       if (outs[c]) std::memcpy(outs[c], host + c * n, n * sizeof(float));
-    return judge_error_word(s);
+    return settle_error_word(s);
   }
   NB_TRY(ensure_staging(s));
   NB_CUDA(launch_pack_state(s->pos_d[s->cur], s->vel_d, n, s->map_d, s->staging_d, s->stream));
