@@ -460,8 +460,8 @@ def run_split(args, rank, world) -> dict:
 
 
 def traffic_from_profile():
-    """DRAM bytes per launch of the force kernel from the committed ncu summary."""
-    f = ROOT / "profiles" / "force_kernel_plummer_1M.txt"
+    """DRAM bytes of a step (all launches) from the committed ncu summary."""
+    f = ROOT / "profiles" / "symmetric_kernel_plummer.txt"
     try:
         for line in f.read_text().splitlines():
             if line.startswith("traffic_bytes_per_launch_full_size:"):
