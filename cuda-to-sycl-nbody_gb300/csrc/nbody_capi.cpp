@@ -225,8 +225,14 @@ static bool compensates(const nb_sim* s, int cfg) {
           symmetric_always_compensates(cfg - num_force_configs(), s->per_pair_mass));
 }
 
+// Records of a part that config `cfg` may write.  A list outlives the masses it was planned
+// with (nb_sim_set_state), so this is the larger of both kinds of masses.
 static int part_records(const nb_sim* s, int cfg) {
-  return cfg >= 0 && compensates(s, cfg) ? 2 : 1;
+  if (cfg < 0) return 1;
+  const bool either = is_symmetric(cfg) &&
+                      (symmetric_always_compensates(cfg - num_force_configs(), false) ||
+                       symmetric_always_compensates(cfg - num_force_configs(), true));
+  return s->params.accumulator == NB_ACC_COMPENSATED || either ? 2 : 1;
 }
 
 static int ensure_scratch(nb_sim* s, const WorkListDev& w, int bi, int rec) {
