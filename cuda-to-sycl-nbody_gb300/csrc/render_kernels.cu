@@ -19,8 +19,8 @@
 // of pixels, 220 with the profile evaluated once per column and row (the splat is bound
 // by instructions then: 2 x 2 pixels per sector, a fifth fewer sectors, gain nothing),
 // 198 with the kernels as programmatic dependents and the blur's taps fixed, 185 with the
-// blur's taps as pairs from shared memory and a gamma of its own (187 with the sprites'
-// corners rounded more finely).
+// blur's taps as pairs from shared memory and a gamma of its own (188 with the sprites'
+// places rounded more finely).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -99,13 +99,12 @@ __global__ void __launch_bounds__(kSplatThreads) splat_kernel(
         const float4 v = vel[g];
         t = fminf(fmaxf((v.x * v.x + v.y * v.y + v.z * v.z + 1.f) * 0.0006f, 0.f), 1.f);
         // pixel centres (k + 0.5) inside [x0, x1) in NDC
-        const float ex = u.flare_x * half_x, ey = u.flare_y * half_y;
-        sx = fmaf(xc, half_x, rest_x - ex);
-        sy = fmaf(yc, half_y, rest_y - ey);
-        kx0 = max(-mid_x, static_cast<int>(ceilf(sx)));
-        kx1 = min(u.bw - 1 - mid_x, static_cast<int>(ceilf(fmaf(xc, half_x, rest_x + ex))) - 1);
-        ky0 = max(-mid_y, static_cast<int>(ceilf(sy)));
-        ky1 = min(u.bh - 1 - mid_y, static_cast<int>(ceilf(fmaf(yc, half_y, rest_y + ey))) - 1);
+        kx0 = max(0, static_cast<int>(ceilf((x0 + 1.f) * 0.5f * u.bw - 0.5f))) - mid_x;
+        kx1 = min(u.bw, static_cast<int>(ceilf((x1 + 1.f) * 0.5f * u.bw - 0.5f))) - 1 - mid_x;
+        ky0 = max(0, static_cast<int>(ceilf((y0 + 1.f) * 0.5f * u.bh - 0.5f))) - mid_y;
+        ky1 = min(u.bh, static_cast<int>(ceilf((y1 + 1.f) * 0.5f * u.bh - 0.5f))) - 1 - mid_y;
+        sx = fmaf(xc, half_x, rest_x - u.flare_x * half_x);
+        sy = fmaf(yc, half_y, rest_y - u.flare_y * half_y);
       }
     }
     unsigned todo = __ballot_sync(0xffffffffu, kx0 <= kx1 && ky0 <= ky1);
