@@ -440,12 +440,19 @@ cudaError_t launch_adjoint_direct(int index, bool per_pair_mass, const AdjointAr
                           tiles, sys);
 }
 
-cudaError_t launch_adjoint_add(const AdjointArgs& a, int tiles, int bi, cudaStream_t stream) {
-  if (static_cast<int64_t>(tiles) * bi < kManyParticles)
-    return launch_dependent(adjoint_add_kernel<32, 8>, add_grid<32>(tiles, bi), 256, 0, stream, a,
-                            bi);
-  return launch_dependent(adjoint_add_kernel<64, 2>, add_grid<64>(tiles, bi), 128, 0, stream, a,
-                          bi);
+template <int kLanes, int kGroups>
+static cudaError_t adjoint_add_one(const AdjointArgs& a, int tiles, int bi, cudaStream_t stream) {
+  return launch_dependent(adjoint_add_kernel<kLanes, kGroups>, add_grid<kLanes>(tiles, bi),
+                          kLanes * kGroups, 0, stream, a, bi);
+}
+
+cudaError_t launch_adjoint_add(const AdjointArgs& a, int tiles, int bi, float terms,
+                               cudaStream_t stream) {
+  const AddShape sh = add_shape(static_cast<int64_t>(tiles) * bi, terms);
+  return sh.groups == 1   ? adjoint_add_one<64, 1>(a, tiles, bi, stream)
+         : sh.groups == 2 ? adjoint_add_one<64, 2>(a, tiles, bi, stream)
+         : sh.groups == 4 ? adjoint_add_one<32, 4>(a, tiles, bi, stream)
+                          : adjoint_add_one<32, 8>(a, tiles, bi, stream);
 }
 
 cudaError_t launch_unpack_vec3(const float* in, int64_t n, const int64_t* map, float4* out,

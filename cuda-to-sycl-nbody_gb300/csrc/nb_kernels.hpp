@@ -42,9 +42,10 @@ cudaError_t launch_symmetric(int index, bool compensated, bool per_pair_mass, co
 // (plain sums, per-particle masses; accelerations only).
 cudaError_t symmetric_xyzm_blocks_per_sm(int index, int* blocks);
 cudaError_t launch_symmetric_xyzm(int index, const SymArgs& a, int grid, cudaStream_t stream);
-// Add the rows and parts of the band's i-tiles and integrate; `tiles` i-tiles from a.tile0.
+// Add the rows and parts of the band's i-tiles and integrate; `tiles` i-tiles from a.tile0,
+// `terms` rows and parts per particle on average.
 cudaError_t launch_symmetric_add(bool compensated, const SymArgs& a, int tiles, int bi,
-                                 cudaStream_t stream);
+                                 float terms, cudaStream_t stream);
 
 // ---- direct force step of small systems (direct_kernel.cu) ----------------------------
 struct DirectArgs {
@@ -164,7 +165,8 @@ cudaError_t launch_adjoint(int index, bool per_pair_mass, const AdjointArgs& a, 
 cudaError_t launch_adjoint_direct(int index, bool per_pair_mass, const AdjointArgs& a,
                                   const int2* tiles, int sys, int grid, cudaStream_t stream);
 // Add the rows and parts of the band's i-tiles and write lam_x_out and lam_v_out.
-cudaError_t launch_adjoint_add(const AdjointArgs& a, int tiles, int bi, cudaStream_t stream);
+cudaError_t launch_adjoint_add(const AdjointArgs& a, int tiles, int bi, float terms,
+                               cudaStream_t stream);
 // n x 3 interleaved (user order) <-> padded float4.
 cudaError_t launch_unpack_vec3(const float* in, int64_t n, const int64_t* map, float4* out,
                                cudaStream_t stream);

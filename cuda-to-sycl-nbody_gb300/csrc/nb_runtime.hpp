@@ -30,6 +30,7 @@ struct WorkListDev {
   int32_t split = 0;
   Segment* segs = nullptr;
   int32_t* seg_begin = nullptr;
+  float terms = 0.f;             // symmetric: rows and parts per particle (add_terms)
   int2* direct_tiles = nullptr;  // direct kernel: its i-tiles, NULL for one system:
   int32_t direct_sys = 0;        // this one
   Fixup* fix = nullptr;

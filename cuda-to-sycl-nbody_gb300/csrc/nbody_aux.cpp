@@ -274,7 +274,8 @@ static int adjoint_backward_stream(nb_sim* s, const float* gx_T, const float* gv
         aa.tile0 = b.tile0;
         aa.tile1 = b.tile1;
         NB_CUDA(launch_adjoint(a.shape, s->per_pair_mass, aa, b.grid, s->stream));
-        NB_CUDA(launch_adjoint_add(aa, b.end - b.tile0, adjoint_shape(a.shape).bi(), s->stream));
+        NB_CUDA(launch_adjoint_add(aa, b.end - b.tile0, adjoint_shape(a.shape).bi(), a.wl.terms,
+                                   s->stream));
       }
       std::swap(a.lam_x, a.tmp);
       std::swap(a.lam_v, a.mu);

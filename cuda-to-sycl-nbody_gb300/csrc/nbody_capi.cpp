@@ -323,6 +323,7 @@ int upload_symmetric(nb_sim* s, const SymPlanHost& h, const KernelShape& sh, int
   w.split = h.split_tiles;
   w.bands = h.bands;
   w.row_values = h.row_values;
+  w.terms = terms_per_particle(h, sh.bi());
   const std::vector<SymSegment> segs = link_segments(
       h, sh.bi() / sh.bj, sh.threads == 32 ? 4 * s->sms : 0, diag_cost, pair_cost);
   int st = dev_alloc(&w.sym_segs, segs.size());
@@ -521,7 +522,7 @@ int launch_with(nb_sim* s, ForceArgs a, const WorkListDev& list) {
       sa.tile0 = b.tile0;
       sa.tile1 = b.tile1;
       NB_CUDA(launch_symmetric(shape, comp, s->per_pair_mass, sa, b.grid, s->stream));
-      NB_CUDA(launch_symmetric_add(comp, sa, b.end - b.tile0, bi, s->stream));
+      NB_CUDA(launch_symmetric_add(comp, sa, b.end - b.tile0, bi, w.terms, s->stream));
     }
     return NB_OK;
   }

@@ -143,6 +143,7 @@ struct DeviceSetup {
   bool copied = false;
   int shape = 0;
   int64_t plane = 0;
+  float terms = 0.f;
   int nbands = 0;
   SymBand bands[kNaMaxBands];
   Layout at;
@@ -245,6 +246,7 @@ int na_upload(DeviceSetup& d, uint64_t n, float G, bool copied, cudaStream_t st)
   d.copied = copied;
   d.shape = kNaShapes[k];
   d.plane = g_na_plan.row_values;
+  d.terms = terms_per_particle(g_na_plan, symmetric_shape(kNaShapes[k]).bi());
   d.nbands = static_cast<int>(g_na_plan.bands.size());
   for (int b = 0; b < d.nbands; ++b) d.bands[b] = g_na_plan.bands[b];
   d.at = at;
@@ -336,7 +338,7 @@ extern "C" int nb_accelerations_noalloc(const float* pos_xyzm_device, uint64_t n
       a.tile0 = band.tile0;
       a.tile1 = band.tile1;
       NB_CUDA(launch_symmetric_xyzm(d.shape, a, band.grid, st));
-      NB_CUDA(launch_symmetric_add(false, a, band.end - band.tile0, bi, st));
+      NB_CUDA(launch_symmetric_add(false, a, band.end - band.tile0, bi, d.terms, st));
     }
     uint32_t tag = 0;
     NB_CUDA(cudaMemcpyAsync(&tag, base, sizeof(tag), cudaMemcpyDeviceToHost, st));

@@ -80,6 +80,14 @@ struct SymPlanHost {
   int32_t split_tiles = 0;
 };
 
+// Rows and parts per particle of the first band, on average.
+template <class Plan>
+float terms_per_particle(const Plan& plan, int bi) {
+  const double particles = static_cast<double>(plan.bands[0].tile1 - plan.bands[0].tile0) * bi;
+  return static_cast<float>(
+      (static_cast<double>(plan.row_values) + static_cast<double>(plan.slots) * bi) / particles);
+}
+
 // The segments in the order the kernel wants them: per band, the first of every CTA and
 // then the others, linked by `next` (counted from the band's seg0).
 //

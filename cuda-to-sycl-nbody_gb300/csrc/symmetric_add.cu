@@ -40,10 +40,12 @@ cudaError_t add_one(bool compensated, const SymArgs& a, int tiles, int bi, cudaS
 }  // namespace
 
 cudaError_t launch_symmetric_add(bool compensated, const SymArgs& a, int tiles, int bi,
-                                 cudaStream_t stream) {
-  return static_cast<int64_t>(tiles) * bi < kManyParticles
-             ? add_one<32, 8>(compensated, a, tiles, bi, stream)
-             : add_one<64, 2>(compensated, a, tiles, bi, stream);
+                                 float terms, cudaStream_t stream) {
+  const AddShape sh = add_shape(static_cast<int64_t>(tiles) * bi, terms);
+  return sh.groups == 1   ? add_one<64, 1>(compensated, a, tiles, bi, stream)
+         : sh.groups == 2 ? add_one<64, 2>(compensated, a, tiles, bi, stream)
+         : sh.groups == 4 ? add_one<32, 4>(compensated, a, tiles, bi, stream)
+                          : add_one<32, 8>(compensated, a, tiles, bi, stream);
 }
 
 }  // namespace nbg

@@ -7,9 +7,8 @@
 // terms of 12 to 32 bytes, a few MB in all, from L2), not bandwidth.  So a CTA is 32
 // particles by 8 groups, each group adding a contiguous range of the terms, eight loads
 // in flight, and the groups' sums are added in order: 4,096 particles took 45 us per
-// step with one thread per particle, 18 with 8 groups.  Large systems and ensembles have
-// enough particles for the latency, and fewer terms than threads: 64 particles by 2
-// groups (4,096 systems of up to 1,024 particles 529 -> 349 us per step).
+// step with one thread per particle, 18 with 8 groups.  With more particles or fewer terms
+// the latency is hidden without so many groups (add_shape).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -21,8 +20,21 @@
 namespace nbg {
 
 constexpr int kAddBatch = 8;
-// From here on two groups (of 64 particles) fill the GPU.
-constexpr int64_t kManyParticles = 1 << 17;
+// Particles by groups of a CTA, for bands of `padded` particles (tiles times bi) with
+// `terms` rows and parts per particle on average.  us per step, 32 x 8, 32 x 4, 64 x 2 and
+// 64 x 1: ensembles of 4,096 systems of up to 1,024 particles (1.6 terms) 515 384 338 303,
+// 640 of up to 4,096 (3.0) 452 400 381 369, 100 of up to 1,024 (7.2) 19.1 16.1 15.1 15.1, 40
+// of up to 4,096 (11) 32.9 29.4 28.2 29.0; single systems of 5,000 particles (70) 14.7
+// 15.5 18.3 24.2, 8,192 (54) 25.0 25.3 26.5 30.2, 10,000 35.0 34.8 36.2 39.1, 20,000 105.5
+// 103.5 104.3 107.0, 40,000 380.0 376.6 375.8 378.3, 100,000 (18) 2,173 2,164 2,161 2,160.
+struct AddShape {
+  int lanes, groups;
+};
+inline AddShape add_shape(int64_t padded, float terms) {
+  if (terms < 8.f) return {64, 1};
+  if (terms < 32.f || padded >= 32768) return {64, 2};
+  return padded >= 10000 ? AddShape{32, 4} : AddShape{32, 8};
+}
 
 // What the pass reads: the band [tile0, tile1) of i-tiles, its rows and parts.
 struct AddTerms {
