@@ -227,9 +227,10 @@ KernelShape direct_shape(int index) {
 // Against the symmetric kernel (its two launches take 3.8 us for 64 particles, and it needs
 // thousands of particles to have a block for every warp): single systems (us per step,
 // symmetric / direct) 64 3.8 / 1.7, 512 5.6 / 2.0, 2,048 7.4 / 4.2, 4,096 12.2 / 9.8, 4,500
-// 13.2 / 11.7, 5,000 14.0 / 14.4; ensembles, from all pairs and i-tiles of 8 particles:
-// 2.2e6 pairs in 1,091 tiles 7.7 / 4.5, 1.4e7 in 11,407 25.2 / 14.8, 1.7e7 in 7,351
-// 21.0 / 14.3, 2.2e7 in 2,792 15.8 / 17.6, 1.4e7 in 19,111 19.3 / 21.7.
+// 12.8 / 11.7, 5,000 14.1 / 15.0; ensembles, from all pairs and i-tiles of 8 particles:
+// 2.4e6 pairs in 1,091 tiles 7.8 / 4.5, 7e6 in 1,720 9.5 / 8.2, 1.1e7 in 1,270 11.9 / 9.4
+// and in 4,760 11.2 / 11.3, 1.4e7 in 11,407 12.8 / 14.8, 2.2e7 in 2,792 14.7 / 16.9, 3.6e6
+// in 4,830 7.8 / 7.1, 5.7e6 in 7,692 9.4 / 10.0.
 //
 // The shapes in the order of their warps: as many per i-tile as one wave of CTAs allows,
 // and their passes over the longest system are worth (a warp meets 64 particles a pass).

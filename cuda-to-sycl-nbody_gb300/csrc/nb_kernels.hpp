@@ -60,10 +60,12 @@ int num_direct_shapes();
 KernelShape direct_shape(int index);
 // The shape for `count` systems; *pays: they have at most max_pairs pairs and max_tiles
 // i-tiles of 8 particles.  Up to these the direct kernel beats the symmetric one:
-constexpr double kDirectPairs = 2.2e7;
-constexpr int64_t kDirectTiles = 16000;
+constexpr double kDirectPairs = 2.2e7;          // one system
+constexpr double kDirectEnsemblePairs = 1.2e7;  // several
+constexpr int64_t kDirectTiles = 6000;
 constexpr double kAdjDirectPairs = 6.5e6;  // the same of the adjoint
-constexpr int64_t kAdjDirectTiles = 5000;
+constexpr double kAdjDirectEnsemblePairs = 3.5e6;
+constexpr int64_t kAdjDirectTiles = 3000;
 int choose_direct(const SystemDesc* sys, int32_t count, int sms, double max_pairs,
                   int64_t max_tiles, bool* pays);
 cudaError_t launch_direct(int index, bool compensated, bool per_pair_mass, const DirectArgs& a,

@@ -88,10 +88,12 @@ int ensure_adjoint_buffers(nb_sim* s, int32_t ncp, int32_t every) {
     bool pays = false;
     // A pair of the adjoint is twice the work of a force's, so the line lies lower (us per
     // backward step, symmetric / direct): 512 particles 6.9 / 3.7, 1,024 7.1 / 4.7, 2,048
-    // 9.0 / 8.0, 2,432 10.2 / 9.0, 3,000 11.9 / 12.6; ensembles of 6e6 pairs in 4,708
-    // i-tiles of 8 18.2 / 14.2, 7e6 in 1,720 13.8 / 15.9, 1.1e7 in 1,270 14.7 / 18.4.
-    a.shape = choose_direct(s->sys_h.data(), nsys, s->sms, kAdjDirectPairs, kAdjDirectTiles,
-                            &pays);
+    // 9.0 / 8.0, 2,432 10.2 / 9.0, 3,000 11.9 / 12.6; ensembles of 2.4e6 pairs in
+    // 1,091 i-tiles of 8 10.0 / 8.8, in 3,129 10.2 / 9.4, 3.6e6 in 414 10.5 / 9.5 and in 4,830
+    // 11.0 / 11.4, 4.1e6 in 1,808 10.6 / 10.8, 7e6 in 1,720 12.4 / 16.1.
+    a.shape = choose_direct(s->sys_h.data(), nsys, s->sms,
+                            nsys == 1 ? kAdjDirectPairs : kAdjDirectEnsemblePairs,
+                            kAdjDirectTiles, &pays);
     a.direct = pays;
     if (a.direct) return plan_direct(s, direct_shape(a.shape).r, 0, nsys, &a.wl);
     int grid = 0;

@@ -659,7 +659,8 @@ static int default_symmetric_for(nb_sim* s, int32_t first, int32_t count) {
 static int default_config_for(nb_sim* s, int32_t first, int32_t count, bool symmetric) {
   if (symmetric && !sharded(s)) {
     bool pays = false;
-    const int shape = choose_direct(s->sys_h.data() + first, count, s->sms, kDirectPairs,
+    const int shape = choose_direct(s->sys_h.data() + first, count, s->sms,
+                                    count == 1 ? kDirectPairs : kDirectEnsemblePairs,
                                     kDirectTiles, &pays);
     return pays ? first_direct() + shape : default_symmetric_for(s, first, count);
   }

@@ -33,7 +33,7 @@ def test_gradients_at_edges(n, mass, eps):
 
 
 @pytest.mark.parametrize("sizes", [[1, 300, 17, 256], [64, 700] * 12, [1100, 130] * 3 + [90] * 300,
-                                   [40, 500, 16] * 30])
+                                   [40, 500, 16] * 30, [300] * 30, [100] * 130 + [150] * 20])
 def test_gradients_of_ensembles(sizes):
     parts = [disk_case(s, seed=70 + k) for k, s in enumerate(sizes)]
     pos, vel = ([np.concatenate([p[q][c] for p in parts]) for c in range(3)] for q in (0, 1))
