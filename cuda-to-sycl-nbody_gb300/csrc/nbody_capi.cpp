@@ -646,10 +646,10 @@ static int default_symmetric_for(nb_sim* s, int32_t first, int32_t count) {
 
 // Default kernel shape of systems [first, first + count), judged alone: a direct one
 // where that pays (choose_direct), a symmetric one otherwise (thin disks, us per step,
-// tuned / symmetric: N = 64 4.9 / 3.8, 2,048 12.3 / 7.4, 25,600 242 / 166, 262,144 21,712
+// tuned / symmetric: N = 64 4.9 / 3.8, 2,048 12.3 / 7.4, 25,600 242 / 164, 262,144 21,712
 // / 14,420, 1,048,576 346,673 / 228,500; ensembles of 4,096 systems up to 8,192 particles
-// 10,577 / 7,655, of 2,000 up to 300 49.8 / 42.3).  Deterministic (the autotuner may pick otherwise, and shapes round
-// differently).  A shard integrates part of a system against all of it, which is not
+// 10,577 / 7,466, of 2,000 up to 300 49.8 / 35.6).  Deterministic (the autotuner may pick
+// otherwise, and shapes round differently).  A shard integrates part of a system against all of it, which is not
 // symmetric, and launches that must fail on purpose need the tuned kernel's waits
 // (`symmetric` false): there, the tuned shape with the largest tiles whose work list
 // still gives every CTA at least 16 (i-tile, j-tile) blocks, so that the stream-K split

@@ -12,7 +12,7 @@
 // list, the partial sums and the rows of j-side sums -- lives in one file-scope device
 // array, kScratchBytes (13 MiB) long; larger systems run in bands of i-tiles that take
 // turns in it (20,000 particles 223 us per call with the tuned kernel and its list
-// uploaded on every call, 149 now).  Small systems run the direct kernel, which needs
+// uploaded on every call, 146 now).  Small systems run the direct kernel, which needs
 // none of it.  Every GPU that loads this module keeps that array
 // until the process exits.  All calls share it and it keeps the last call's contents:
 // the work list stays for the next call of the same size, checked by a tag that is read
