@@ -1,7 +1,7 @@
 // FP64 diagnostics on the GPU: kinetic and potential energy, linear and angular
 // momentum, and FP64 accelerations of selected rows.  Sums are double precision, and
 // so is the pair arithmetic, except the potential's of large systems, whose terms are
-// sums of two floats; reductions use fixed-order trees over per-block partials, so
+// sums of three floats; reductions use fixed-order trees over per-block partials, so
 // results are deterministic.
 #include <cuda_runtime.h>
 
@@ -75,32 +75,33 @@ __global__ void __launch_bounds__(kDiagThreads) moments_kernel(
   }
 }
 
-// ---- potential, pairs in two floats -------------------------------------------------
+// ---- potential, pairs in three floats -----------------------------------------------
 // The potential needs N^2 / 2 inverse square roots in double precision, about 30 FP64
 // operations per pair on a pipe of 2 lanes per SM (FP32: 128; a third-order step from the
 // FP32 root is no faster than rsqrt: its conversions run on that pipe too).  Here a pair's
-// term is a sum of two floats (packed FP32x2, two j-particles per register pair): the coordinate
-// differences are exact (TwoSum), the squared distance and the root carry 47 bits or
-// more (two Newton steps on the MUFU rsqrt, residuals by fused multiply-add), and 128
-// terms at a time are added error-free before they go to FP64.  About 90 FP32 lane
-// operations per pair.  Errors of single terms (below 1e-14) average out over a
-// system's pairs, and the sums are no further from exact ones than the FP64 kernel's,
-// whose threads add thousands of terms one after another (RMS over disks and spheres,
-// equal and own masses: FP64 2.0e-16 and 1.7e-16 at N = 10,011, 4.9e-16 and 5.6e-16 at
-// 65,536; split 1.2e-16 and 8.5e-17, 1.9e-16 and 1.7e-16).  N = 65,536: 103.5 ms before,
-// 7.6 now.
+// term is a sum of three floats (packed FP32x2, two j-particles per register pair).  The
+// coordinate differences and their squares are exact (TwoSum, fused multiply-add); every
+// sum is carried with its errors, so that the squared distance, the root's residual and
+// the term keep more than 60 bits, and 128 terms at a time are added error-free before
+// they go to FP64.  A term is then no further from exact than FP64's (over 8e6 pairs,
+// emulated: 5e-19 at worst, FP64's 2.8e-16, 7e-17 RMS), whatever the distances are: where
+// few distinct ones dominate nothing averages out, and terms of two floats (7.6 ms at N =
+// 65,536) left errors up to 3.8e-13 of the sum (4,096 particles at two points).
+// About 160 FP32 lane operations per pair, of which the FMA pipe takes 8.7 ms at N = 65,536:
+// 103.5 ms with FP64 pairs, 9.6 now.
 // Systems below kSplitMin particles, softenings below kSplitEps and values out of the
-// split's range keep the FP64 kernel; an i-tile whose particles are nearly at one place,
-// where all terms are rounded alike and nothing averages out, is summed in FP64 too.
+// split's range keep the FP64 kernel.
 constexpr int kSplitMin = 4096;  // below, FP64's sums are the more exact ones
 constexpr float kSplitEps = 1e-12f;
 constexpr int kSplitThreads = 256;
-constexpr int kSplitR = 1;                          // i-particles per thread
-constexpr int kSplitBI = kSplitThreads * kSplitR;   // i-tile and j-tile
-constexpr int kSplitFlush = 64;                     // j-pairs between two sums into FP64
+constexpr int kSplitBI = kSplitThreads;  // i-tile (a particle per thread) and j-tile
+constexpr int kSplitFlush = 64;          // j-pairs between two sums into FP64
 
-__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, neg2(b)); }
+__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
+// Signs as products: the packed operations take no negated operand, and a sign flip per lane
+// costs more (9.6 ms; as flips and additions 13.7).
+__device__ __forceinline__ float2 neg2(float2 a) { return __fmul2_rn(a, both(-1.f)); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, both(-1.f), a); }
 
 // a + b = s + e exactly (Knuth's TwoSum).
 __device__ __forceinline__ float2 two_sum(float2 a, float2 b, float2& e) {
@@ -110,122 +111,109 @@ __device__ __forceinline__ float2 two_sum(float2 a, float2 b, float2& e) {
   return s;
 }
 
-// One squared difference: a - b = h + l exactly, its square as p + q + l^2.
-__device__ __forceinline__ void square_diff(float2 a, float2 nb, float2& p, float2& q, float2& l) {
+// a * b = p + e exactly.
+__device__ __forceinline__ float2 two_prod(float2 a, float2 b, float2& e) {
+  const float2 p = __fmul2_rn(a, b);
+  e = __ffma2_rn(a, b, neg2(p));
+  return p;
+}
+
+// sum += t, for |t| < |sum| (Dekker's FastTwoSum): what is rounded away goes to low.  A sum
+// that starts at a value well above all terms stays in its binade, so their high parts add
+// without error and `sum` less that value is their sum.
+__device__ __forceinline__ void add_low(float2& sum, float2& low, float2 t) {
+  const float2 s = __fadd2_rn(sum, t);
+  low = __fadd2_rn(low, sub2(t, sub2(s, sum)));
+  sum = s;
+}
+
+// One squared difference: a - b = h + l exactly, its square p + q + r + what goes to low.
+__device__ __forceinline__ float2 square_diff(float2 a, float2 nb, float2& q, float2& r,
+                                              float2& low) {
+  float2 l, s;
   const float2 h = two_sum(a, nb, l);
-  p = __fmul2_rn(h, h);
-  q = __ffma2_rn(h, h, neg2(p));
-  q = __ffma2_rn(__fadd2_rn(h, h), l, q);
+  const float2 p = two_prod(h, h, q);
+  r = two_prod(__fadd2_rn(h, h), l, s);
+  low = __ffma2_rn(l, l, __fadd2_rn(low, s));
+  return p;
 }
 
-// 1 - (h + l) y^2, for y near the inverse square root of h + l.
-__device__ __forceinline__ float2 root_residual(float2 h, float2 l, float2 y) {
-  const float2 p = __fmul2_rn(h, y);
-  const float2 pe = __ffma2_rn(h, y, neg2(p));
-  const float2 ny = neg2(y);
-  float2 e = __ffma2_rn(p, ny, make_float2(1.f, 1.f));
-  e = __ffma2_rn(pe, ny, e);
-  return __ffma2_rn(__fmul2_rn(l, y), ny, e);
+// The inverse square root of D = dx^2 + dy^2 + dz^2 + e2 as y + w + v.
+__device__ __forceinline__ float2 split_root(float2 ax, float2 nx, float2 ay, float2 ny, float2 az,
+                                             float2 nz, float2 e2, float2& w, float2& v) {
+  // D = H + L + T, each below 2^-22 of the one before: the squares, then what their sum
+  // and their own low parts leave (below 6 2^-24 D in all, so 2^-20 D holds them).
+  float2 T = both(0.f), a, b, c, qx, qy, qz, rx, ry, rz;
+  const float2 px = square_diff(ax, nx, qx, rx, T);
+  const float2 py = square_diff(ay, ny, qy, ry, T);
+  const float2 pz = square_diff(az, nz, qz, rz, T);
+  const float2 h = two_sum(two_sum(two_sum(px, py, a), pz, b), e2, c);
+  const float2 base = __fmul2_rn(h, both(0x1p-20f));
+  float2 mid = base;
+  add_low(mid, T, a);
+  add_low(mid, T, b);
+  add_low(mid, T, c);
+  add_low(mid, T, qx);
+  add_low(mid, T, qy);
+  add_low(mid, T, qz);
+  add_low(mid, T, rx);
+  add_low(mid, T, ry);
+  add_low(mid, T, rz);
+  mid = sub2(mid, base);
+  const float2 H = __fadd2_rn(h, mid);
+  const float2 L = sub2(mid, sub2(H, h));
+  // y is within 2^-22 of the root; e = 1 - D y^2 as E + F, from y^2 = s + t.
+  const float2 y = make_float2(rsqrtf(H.x), rsqrtf(H.y));
+  float2 t, pe, ce, de;
+  const float2 s = two_prod(y, y, t);
+  const float2 p = two_prod(H, s, pe), cp = two_prod(H, t, ce), dp = two_prod(L, s, de);
+  float2 F = neg2(__ffma2_rn(T, s, __ffma2_rn(L, t, __fadd2_rn(ce, de))));
+  const float2 scale = both(0x1.8p-20f);
+  float2 E = __fadd2_rn(sub2(both(1.f), p), scale);
+  add_low(E, F, neg2(pe));
+  add_low(E, F, neg2(cp));
+  add_low(E, F, neg2(dp));
+  E = sub2(E, scale);
+  // y (1 - e)^(-1/2) = y + y e / 2 + y 3/8 e^2, the next term below 2^-64.
+  const float2 half = __fmul2_rn(y, both(0.5f));
+  w = two_prod(half, E, v);
+  v = __ffma2_rn(half, __ffma2_rn(__fmul2_rn(E, both(0.75f)), E, F), v);
+  return y;
 }
 
-// j-pairs [p0, p1) of the shared tile against the thread's i-particles, added to
-// (s, l, k): the sum is s + l - k / 2.
-// kMask: leave out j == i and j >= cnt.
+// j-pairs [p0, p1) of the shared tile against the thread's i-particle, added to s + l + k.
+// kMask: leave out j == self and j >= cnt.
 template <bool kMass, bool kMask>
-__device__ __forceinline__ void split_pairs(const float4* tile, int p0, int p1, int cnt,
-                                            const float2 (&nx)[kSplitR],
-                                            const float2 (&ny)[kSplitR],
-                                            const float2 (&nz)[kSplitR], float2 e2, int self,
-                                            float2 (&s)[kSplitR], float2 (&l)[kSplitR],
-                                            float2 (&k)[kSplitR]) {
+__device__ __forceinline__ void split_pairs(const float4* tile, int p0, int p1, int cnt, float2 nx,
+                                            float2 ny, float2 nz, float2 e2, int self, float2& s,
+                                            float2& l, float2& k) {
 #pragma unroll 2
   for (int p = p0; p < p1; ++p) {
     const float4 A = tile[2 * p], B = tile[2 * p + 1];
-#pragma unroll
-    for (int r = 0; r < kSplitR; ++r) {
-      float2 px, qx, lx, py, qy, ly, pz, qz, lz, a, b, c;
-      square_diff(make_float2(A.x, A.y), nx[r], px, qx, lx);
-      square_diff(make_float2(A.z, A.w), ny[r], py, qy, ly);
-      square_diff(make_float2(B.x, B.y), nz[r], pz, qz, lz);
-      // What the differences' low words add to the square, at most 2^-48 of it: never
-      // negative, so rounding it away would shift every term the same way (1e-16).
-      const float2 ll = __ffma2_rn(lz, lz, __ffma2_rn(ly, ly, __fmul2_rn(lx, lx)));
-      float2 h = two_sum(px, py, a);
-      h = two_sum(h, pz, b);
-      h = two_sum(h, e2, c);
-      const float2 low = __fadd2_rn(__fadd2_rn(__fadd2_rn(a, b), c),
-                                    __fadd2_rn(__fadd2_rn(qx, qy), qz));
-      const float2 H = __fadd2_rn(h, low);
-      const float2 L = sub2(low, sub2(H, h));
-      float2 y = make_float2(rsqrtf(H.x), rsqrtf(H.y));
-      // y + y e (1/2 + 3/8 e) rounded to one float, then what is left of it.  (Without
-      // its 3/8 e^2 the second step would be off by 4e-16 on average, always to one side.)
-      const float2 c3 = make_float2(0.375f, 0.375f), c1 = make_float2(0.5f, 0.5f);
-      float2 e = root_residual(H, L, y);
-      y = __ffma2_rn(y, __fmul2_rn(e, __ffma2_rn(c3, e, c1)), y);
-      e = root_residual(H, L, y);
-      float2 w = __fmul2_rn(y, __fmul2_rn(e, __ffma2_rn(c3, e, c1)));
-      float2 v = __fmul2_rn(__fmul2_rn(__fmul2_rn(y, y), y), ll);
-      if (kMass) {
-        const float2 m = make_float2(B.z, B.w);
-        v = __fmul2_rn(m, v);
-        const float2 my = __fmul2_rn(m, y);
-        w = __ffma2_rn(m, w, __ffma2_rn(m, y, neg2(my)));
-        y = my;
-      }
-      if (kMask) {
-        if (2 * p == self + r * kSplitThreads || 2 * p >= cnt) y.x = w.x = v.x = 0.f;
-        if (2 * p + 1 == self + r * kSplitThreads || 2 * p + 1 >= cnt) y.y = w.y = v.y = 0.f;
-      }
-      float2 t;
-      s[r] = two_sum(s[r], y, t);
-      l[r] = __fadd2_rn(l[r], __fadd2_rn(t, w));
-      k[r] = __fadd2_rn(k[r], v);
+    float2 w, v, u, t;
+    float2 y = split_root(make_float2(A.x, A.y), nx, make_float2(A.z, A.w), ny,
+                          make_float2(B.x, B.y), nz, e2, w, v);
+    float2 low = both(0.f);
+    if (kMass) {
+      const float2 m = make_float2(B.z, B.w);
+      y = two_prod(m, y, low);
+      w = two_prod(m, w, u);
+      v = __ffma2_rn(m, v, u);
+    }
+    if (kMask) {
+      if (2 * p == self || 2 * p >= cnt) y.x = w.x = v.x = low.x = 0.f;
+      if (2 * p + 1 == self || 2 * p + 1 >= cnt) y.y = w.y = v.y = low.y = 0.f;
+    }
+    s = two_sum(s, y, t);
+    l = two_sum(l, t, u);
+    k = __fadd2_rn(k, __fadd2_rn(u, v));
+    l = two_sum(l, w, u);
+    k = __fadd2_rn(k, u);
+    if (kMass) {
+      l = two_sum(l, low, u);
+      k = __fadd2_rn(k, u);
     }
   }
-}
-
-// Whether the block's particles nearly coincide: within 2^-10 of their coordinates in
-// every component, or within 2^-20 softening lengths.
-__device__ __forceinline__ bool nearly_coincident(float x, float y, float z, float eps2) {
-  __shared__ float ext[kSplitThreads / 32][6];
-  float v[6] = {x, y, z, -x, -y, -z};
-#pragma unroll
-  for (int c = 0; c < 6; ++c) {
-    for (int d = 16; d > 0; d >>= 1) v[c] = fmaxf(v[c], __shfl_xor_sync(0xffffffffu, v[c], d));
-    if (threadIdx.x % 32 == 0) ext[threadIdx.x / 32][c] = v[c];
-  }
-  __syncthreads();
-  float extent2 = 0.f;
-  bool near = true;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    float hi = ext[0][c], lo = -ext[0][c + 3];
-    for (int w = 1; w < kSplitThreads / 32; ++w) {
-      hi = fmaxf(hi, ext[w][c]);
-      lo = fminf(lo, -ext[w][c + 3]);
-    }
-    near = near && hi - lo <= 0x1p-10f * fmaxf(fabsf(hi), fabsf(lo));
-    extent2 = fmaf(hi - lo, hi - lo, extent2);
-  }
-  return near || extent2 <= 0x1p-40f * eps2;
-}
-
-// One i-particle's sum over j in [j0, j1) of its system, j > i, in FP64.
-__device__ __noinline__ double fp64_row(const float* __restrict__ pos, int64_t offset, int li,
-                                        int j0, int j1, double eps2) {
-  const int64_t gi = offset + li;
-  const double xi = pos[pair_index(gi, 0)], yi = pos[pair_index(gi, 1)],
-               zi = pos[pair_index(gi, 2)];
-  double sum = 0.0;
-  for (int j = max(j0, li + 1); j < j1; ++j) {
-    const int64_t g = offset + j;
-    const double dx = pos[pair_index(g, 0)] - xi, dy = pos[pair_index(g, 1)] - yi,
-                 dz = pos[pair_index(g, 2)] - zi;
-    const double d2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-    sum = fma(static_cast<double>(pos[pair_index(g, 3)]), rsqrt(d2), sum);
-  }
-  return sum;
 }
 
 // blockIdx.x: i-tile tiles[x] = (system, tile); blockIdx.y: one of gridDim.y spans of the
@@ -251,30 +239,13 @@ __global__ void __launch_bounds__(kSplitThreads) potential_split_kernel(
     return;
   }
   const float4* recs = reinterpret_cast<const float4*>(pos + 4 * sd.offset);
-  const float2 e2 = make_float2(eps2, eps2);
-  float2 nx[kSplitR], ny[kSplitR], nz[kSplitR];
-  double acc[kSplitR], mi[kSplitR];
-#pragma unroll
-  for (int r = 0; r < kSplitR; ++r) {
-    const int li = tl.y * kSplitBI + r * kSplitThreads + tid;
-    const int64_t g = sd.offset + min(li, sd.n - 1);
-    const float x = pos[pair_index(g, 0)], y = pos[pair_index(g, 1)], z = pos[pair_index(g, 2)];
-    nx[r] = make_float2(-x, -x);
-    ny[r] = make_float2(-y, -y);
-    nz[r] = make_float2(-z, -z);
-    mi[r] = li < sd.n ? static_cast<double>(pos[pair_index(g, 3)]) : 0.0;
-    acc[r] = 0.0;
-  }
-  static_assert(kSplitR == 1, "the block's particles are its threads'");
-  if (nearly_coincident(-nx[0].x, -ny[0].x, -nz[0].x, eps2)) {
-    const int li = tl.y * kSplitBI + tid;
-    const double v = li < sd.n ? fp64_row(pos, sd.offset, li, t0 * kSplitBI,
-                                          min(sd.n, t1 * kSplitBI), eps2)
-                               : 0.0;
-    const double total = block_sum(-G * mi[0] * v, sh);
-    if (tid == 0) *out = total;
-    return;
-  }
+  const float2 e2 = both(eps2);
+  const int li = tl.y * kSplitBI + tid;
+  const int64_t g = sd.offset + min(li, sd.n - 1);
+  const float2 nx = both(-pos[pair_index(g, 0)]), ny = both(-pos[pair_index(g, 1)]),
+               nz = both(-pos[pair_index(g, 2)]);
+  const double mi = li < sd.n ? static_cast<double>(pos[pair_index(g, 3)]) : 0.0;
+  double acc = 0.0;
   for (int t = t0; t < t1; ++t) {
     const int cnt = min(kSplitBI, sd.n - t * kSplitBI);
     const int npairs = (cnt + 1) / 2;
@@ -284,28 +255,19 @@ __global__ void __launch_bounds__(kSplitThreads) potential_split_kernel(
     __syncthreads();
     const bool diag = t == tl.y;
     for (int p = 0; p < npairs; p += kSplitFlush) {
-      float2 s[kSplitR], l[kSplitR], k[kSplitR];
-#pragma unroll
-      for (int r = 0; r < kSplitR; ++r) s[r] = l[r] = k[r] = make_float2(0.f, 0.f);
+      float2 s = both(0.f), l = s, k = s;
       const int p1 = min(npairs, p + kSplitFlush);
       if (diag || cnt < kSplitBI)
-        split_pairs<kMass, true>(tile, p, p1, cnt, nx, ny, nz, e2,
-                                 diag ? tid : -2 * kSplitBI, s, l, k);
+        split_pairs<kMass, true>(tile, p, p1, cnt, nx, ny, nz, e2, diag ? tid : -2, s, l, k);
       else
         split_pairs<kMass, false>(tile, p, p1, cnt, nx, ny, nz, e2, 0, s, l, k);
-#pragma unroll
-      for (int r = 0; r < kSplitR; ++r)
-        acc[r] += (static_cast<double>(s[r].x) + static_cast<double>(s[r].y)) +
-                  (static_cast<double>(l[r].x) + static_cast<double>(l[r].y) -
-                   0.5 * static_cast<double>(k[r].x + k[r].y));
+      acc += (static_cast<double>(s.x) + static_cast<double>(s.y)) +
+             ((static_cast<double>(l.x) + static_cast<double>(l.y)) +
+              static_cast<double>(k.x + k.y));
     }
-    if (diag)
-#pragma unroll
-      for (int r = 0; r < kSplitR; ++r) acc[r] *= 0.5;
+    if (diag) acc *= 0.5;
   }
-  double v = 0.0;
-#pragma unroll
-  for (int r = 0; r < kSplitR; ++r) v += mi[r] * acc[r];
+  double v = mi * acc;
   if (!kMass) v *= static_cast<double>(pos[pair_index(sd.offset, 3)]);  // the common m_j
   const double total = block_sum(-G * v, sh);
   if (tid == 0) *out = total;

@@ -341,7 +341,9 @@ int nb_sim_graph_launch(nb_sim* s);
 /* No reference counterpart: the reference reports only kernel times
  * (nbody.cpp:108-123). */
 /* Energy and momenta of system `system` (-1 = all systems together, without the
- * cross-system potential).  FP64 pair arithmetic and reductions on the GPU. */
+ * cross-system potential).  FP64 reductions on the GPU, and FP64 pair arithmetic or, in
+ * the potential of systems from 4,096 particles on, sums of three floats that are no
+ * less precise. */
 int nb_sim_diagnostics(nb_sim* s, int32_t system, nb_diagnostics* out);
 /* FP64 accelerations for `count` particle indices (global, system-concatenated),
  * computed on the GPU against all particles of each row's system. */
