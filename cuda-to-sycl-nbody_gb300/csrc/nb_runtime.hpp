@@ -168,8 +168,13 @@ int dev_alloc(T** p, size_t count) {
   *p = nullptr;
   if (count == 0) return NB_OK;
   if (g_alloc_failure_countdown.load(std::memory_order_relaxed) > 0 &&
-      g_alloc_failure_countdown.fetch_sub(1) == 1)
+      g_alloc_failure_countdown.fetch_sub(1) == 1) {
+    // A request that no device can serve: it leaves what a real failure leaves.
+    void* none = nullptr;
+    const cudaError_t e = cudaMalloc(&none, size_t{1} << 60);
+    if (e != cudaSuccess) (void)cuda_error(e, "cudaMalloc");
     return set_error(NB_ERR_OUT_OF_MEMORY, "injected allocation failure (nb_inject_alloc_failure)");
+  }
   const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), count * sizeof(T));
   if (e != cudaSuccess) {
     *p = nullptr;

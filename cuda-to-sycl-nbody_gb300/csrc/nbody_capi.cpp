@@ -38,6 +38,9 @@ int set_error(int code, const std::string& msg) {
 }
 
 int cuda_error(cudaError_t e, const char* what) {
+  // What is reported here is not the next launch's error: a caller that goes on without the
+  // allocation that failed checks its launches with cudaGetLastError.
+  cudaGetLastError();
   const int code = (e == cudaErrorMemoryAllocation) ? NB_ERR_OUT_OF_MEMORY : NB_ERR_CUDA;
   return set_error(code, std::string(what) + ": " + cudaGetErrorString(e));
 }
