@@ -424,11 +424,19 @@ static bool sequential_order_mode(const nb_sim* s) {
   return reference_order_mode(s) || s->params.calc_method == NB_PREDICATED;
 }
 
-// (Re)build the reference-order work list for shape `shape` (all systems).
+// The duplicated j-layout buffer of the reference-order kernel.
+static int ensure_reference_order_dup(nb_sim* s) {
+  if (!s->ro_dup_d) NB_TRY(dev_alloc(&s->ro_dup_d, 2 * static_cast<size_t>(s->n_pad)));
+  return NB_OK;
+}
+
 static int reference_order_grid(nb_sim* s, int shape, int32_t first, int32_t count);
 
+// (Re)build the reference-order work list for shape `shape` (all systems), with the
+// buffer that the shape needs: a captured step cannot allocate it.
 static int build_reference_order_worklist(nb_sim* s, int shape) {
   const int cfg = -1 - shape;
+  if (reference_order_needs_dup(shape)) NB_TRY(ensure_reference_order_dup(s));
   const KernelShape sh = reference_order_shape(shape);
   const int32_t nsys = static_cast<int32_t>(s->sys_h.size());
   const WorkListHost h = plan_worklist(s->sys_h.data(), 0, nsys, sh.bi(), sh.bj,
@@ -472,12 +480,6 @@ static int build_per_system_worklists(nb_sim* s, int policy) {
   }
   s->wl_sys_policy = policy;
   s->wl_sys_cfg = sim_cfg;
-  return NB_OK;
-}
-
-// The duplicated j-layout buffer of the reference-order kernel.
-static int ensure_reference_order_dup(nb_sim* s) {
-  if (!s->ro_dup_d) NB_TRY(dev_alloc(&s->ro_dup_d, 2 * static_cast<size_t>(s->n_pad)));
   return NB_OK;
 }
 
@@ -844,8 +846,6 @@ static int create_impl(const nb_params* p, uint32_t num_systems, const uint32_t*
   if (sequential_order_mode(s)) {
     s->ro_shape = default_reference_order_for(s, 0, static_cast<int32_t>(s->sys_h.size()));
     if ((st = build_reference_order_worklist(s, s->ro_shape)) != NB_OK) return fail(st);
-    if (reference_order_needs_dup(s->ro_shape) && (st = ensure_reference_order_dup(s)) != NB_OK)
-      return fail(st);
   }
   if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) return fail(cuda_error(e, "create"));
   *out = s;
