@@ -490,8 +490,6 @@ ForceArgs base_args(nb_sim* s) {
   a.vel = s->vel_d;
   a.accel_out = nullptr;
   a.sys = s->sys_d;
-  a.partials = s->partials_d;
-  a.counters = s->counters_d;
   a.err = s->err_d;
   a.eps2 = s->params.dist_eps;
   a.dt = s->params.dt;
@@ -502,6 +500,9 @@ ForceArgs base_args(nb_sim* s) {
 }
 
 int launch_with(nb_sim* s, ForceArgs a, const WorkListDev& list) {
+  // The scratch as it is now: lists that were planned since may have made it larger.
+  a.partials = s->partials_d;
+  a.counters = s->counters_d;
   a.inject = s->inject;
   s->inject = 0;
   // The failure hooks make a bounded wait run out; only the tuned kernel has them.
