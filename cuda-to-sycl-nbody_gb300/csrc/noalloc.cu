@@ -15,10 +15,10 @@
 // uploaded on every call, 146 now).  Small systems run the direct kernel, which needs
 // none of it.  Every GPU that loads this module keeps that array
 // until the process exits.  All calls share it and it keeps the last call's contents:
-// the work list stays for the next call of the same size, checked by a tag that is read
-// back with every call.  Two calls whose work overlapped on the GPU would race on it, so
-// each call holds a process-wide lock until its stream has drained: the calls of one
-// process run one after another, whatever streams and threads they come from.
+// the work list stays for the next call of the same size, unless a call fails on the way.
+// Two calls whose work overlapped on the GPU would race on it, so each call holds a
+// process-wide lock until its stream has drained: the calls of one process run one after
+// another, whatever streams and threads they come from.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -128,7 +128,7 @@ constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 // Where the current plan's parts lie in the scratch; `copy`: of the caller's positions,
 // 0 where they are read in place.
 struct Layout {
-  size_t sys = 256, segs = 512, tiles = 0, partials = 0, rows = 0, copy = 0;  // the tag is at 0
+  size_t sys = 0, segs = 256, tiles = 0, partials = 0, rows = 0, copy = 0;
 };
 
 struct DeviceSetup {
@@ -136,9 +136,8 @@ struct DeviceSetup {
   unsigned char* scratch = nullptr;  // device address of g_noalloc_scratch
   int grid[kNaCount] = {};           // largest grid of each shape
   int sms = 0;
-  // The plan in the scratch: for `n` particles, `tag` at its start; n = 0: none.
+  // The plan in the scratch: for `n` particles; n = 0: none.
   uint64_t n = 0;
-  uint32_t tag = 0;
   float G = 0.f;
   bool copied = false;
   int shape = 0;
@@ -153,7 +152,21 @@ std::mutex g_na_mutex;            // guards the host-side tables below
 DeviceSetup g_na_setup[kNaMaxDevices];
 FixedPlan g_na_plan;
 FixedTable<SymSegment, kNaMaxSegments> g_na_linked;
-uint32_t g_na_tag = 0;
+
+// What a call does when it ends early, by an error after its first enqueue: nothing may be
+// left in flight when the lock goes, and the plan may not be in the scratch.  (A call on a
+// stream that is being captured fails so: its uploads were recorded, not made.)
+struct Drain {
+  DeviceSetup& d;
+  cudaStream_t stream;
+  bool done = false;
+  ~Drain() {
+    if (done) return;
+    d.n = 0;
+    cudaStreamSynchronize(stream);
+    cudaGetLastError();
+  }
+};
 
 // Once per device, with that device current: the scratch's device address and the
 // shapes' grids.
@@ -233,15 +246,12 @@ int na_upload(DeviceSetup& d, uint64_t n, float G, bool copied, cudaStream_t st)
   if (!na_plan(sd, d, k, copied, &at) && !na_plan(sd, d, k = 0, copied, &at))
     return set_error(NB_ERR_INVALID_ARGUMENT, "work list exceeds the no-allocation scratch");
   unsigned char* base = d.scratch;
-  const uint32_t tag = ++g_na_tag;
   // Host sources are pageable: each copy has read them before it returns.
   NB_CUDA(cudaMemcpyAsync(base + at.segs, g_na_linked.data, g_na_linked.n * sizeof(SymSegment),
                           cudaMemcpyHostToDevice, st));
   NB_CUDA(cudaMemcpyAsync(base + at.tiles, g_na_plan.tiles.data,
                           g_na_plan.tiles.size() * sizeof(SymTile), cudaMemcpyHostToDevice, st));
   NB_CUDA(cudaMemcpyAsync(base + at.sys, &sd, sizeof(sd), cudaMemcpyHostToDevice, st));
-  NB_CUDA(cudaMemcpyAsync(base, &tag, sizeof(tag), cudaMemcpyHostToDevice, st));
-  d.tag = tag;
   d.G = G;
   d.copied = copied;
   d.shape = kNaShapes[k];
@@ -291,6 +301,7 @@ extern "C" int nb_accelerations_noalloc(const float* pos_xyzm_device, uint64_t n
   whole.n = static_cast<int32_t>(n);
   bool direct = false;
   const int small = choose_direct(&whole, 1, d.sms, kDirectPairs, kDirectTiles, &direct);
+  Drain drain{d, st};
   if (direct) {
     // One launch without a plan.
     DirectArgs a{};
@@ -308,47 +319,38 @@ extern "C" int nb_accelerations_noalloc(const float* pos_xyzm_device, uint64_t n
     const int r = direct_shape(small).r;
     NB_CUDA(launch_direct_xyzm(small, a, (whole.n + r - 1) / r, st));
     NB_CUDA(cudaStreamSynchronize(st));
+    drain.done = true;
     return NB_OK;
   }
-  // Twice where the scratch does not hold the plan any more (a device reset).
-  for (int attempt = 0; attempt < 2; ++attempt) {
-    if (d.n != n || d.G != G || d.copied != copied) NB_TRY(na_upload(d, n, G, copied, st));
-    unsigned char* base = d.scratch;
-    SymArgs a{};
-    a.f.pos = pos_xyzm_device;
-    if (copied) {
-      NB_CUDA(cudaMemcpyAsync(base + d.at.copy, pos_xyzm_device, 16 * n, cudaMemcpyDeviceToDevice,
-                              st));
-      a.f.pos = reinterpret_cast<const float*>(base + d.at.copy);
-    }
-    a.f.accel_out = reinterpret_cast<float4*>(accel_xyzw_device);
-    a.f.sys = reinterpret_cast<const SystemDesc*>(base + d.at.sys);
-    a.f.partials = reinterpret_cast<float4*>(base + d.at.partials);
-    a.f.eps2 = dist_eps;
-    const float e3 = dist_eps * dist_eps * dist_eps;
-    a.f.mask_self = (e3 >= FLT_MIN) ? 0 : 1;
-    a.tiles = reinterpret_cast<const SymTile*>(base + d.at.tiles);
-    a.rows = reinterpret_cast<float*>(base + d.at.rows);
-    a.plane = d.plane;
-    a.carry = a.f.accel_out;  // a particle's place is free until its last band
-    const int bi = symmetric_shape(d.shape).bi();
-    for (int b = 0; b < d.nbands; ++b) {
-      const SymBand& band = d.bands[b];
-      a.segs = reinterpret_cast<const SymSegment*>(base + d.at.segs) + band.seg0;
-      a.tile0 = band.tile0;
-      a.tile1 = band.tile1;
-      NB_CUDA(launch_symmetric_xyzm(d.shape, a, band.grid, st));
-      NB_CUDA(launch_symmetric_add(false, a, band.end - band.tile0, bi, d.terms, st));
-    }
-    uint32_t tag = 0;
-    NB_CUDA(cudaMemcpyAsync(&tag, base, sizeof(tag), cudaMemcpyDeviceToHost, st));
-    const cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) {
-      d.n = 0;
-      return cuda_error(e, "cudaStreamSynchronize");
-    }
-    if (tag == d.tag) return NB_OK;
-    d.n = 0;
+  if (d.n != n || d.G != G || d.copied != copied) NB_TRY(na_upload(d, n, G, copied, st));
+  unsigned char* base = d.scratch;
+  SymArgs a{};
+  a.f.pos = pos_xyzm_device;
+  if (copied) {
+    NB_CUDA(cudaMemcpyAsync(base + d.at.copy, pos_xyzm_device, 16 * n, cudaMemcpyDeviceToDevice,
+                            st));
+    a.f.pos = reinterpret_cast<const float*>(base + d.at.copy);
   }
-  return set_error(NB_ERR_STATE, "the no-allocation scratch was overwritten");
+  a.f.accel_out = reinterpret_cast<float4*>(accel_xyzw_device);
+  a.f.sys = reinterpret_cast<const SystemDesc*>(base + d.at.sys);
+  a.f.partials = reinterpret_cast<float4*>(base + d.at.partials);
+  a.f.eps2 = dist_eps;
+  const float e3 = dist_eps * dist_eps * dist_eps;
+  a.f.mask_self = (e3 >= FLT_MIN) ? 0 : 1;
+  a.tiles = reinterpret_cast<const SymTile*>(base + d.at.tiles);
+  a.rows = reinterpret_cast<float*>(base + d.at.rows);
+  a.plane = d.plane;
+  a.carry = a.f.accel_out;  // a particle's place is free until its last band
+  const int bi = symmetric_shape(d.shape).bi();
+  for (int b = 0; b < d.nbands; ++b) {
+    const SymBand& band = d.bands[b];
+    a.segs = reinterpret_cast<const SymSegment*>(base + d.at.segs) + band.seg0;
+    a.tile0 = band.tile0;
+    a.tile1 = band.tile1;
+    NB_CUDA(launch_symmetric_xyzm(d.shape, a, band.grid, st));
+    NB_CUDA(launch_symmetric_add(false, a, band.end - band.tile0, bi, d.terms, st));
+  }
+  NB_CUDA(cudaStreamSynchronize(st));
+  drain.done = true;
+  return NB_OK;
 }

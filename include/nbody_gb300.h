@@ -382,7 +382,7 @@ int nb_sim_adjoint_backward_device(nb_sim* s, const float* gx_T_device,
  * keeps until the process exits.  The first call on a device looks that array up
  * and should come before any stream capture.  All calls share the array, which
  * keeps the last call's contents (a call of the same n and G finds its work list
- * there); calls whose work overlapped on the GPU would race on it, so each call holds a
+ * there, unless the last call failed); calls whose work overlapped on the GPU would race on it, so each call holds a
  * process-wide lock until its work has finished: calls from several threads or
  * streams of one process run one after another.  Runs on `stream` and waits for
  * it before returning.  Both pointers may be the same buffer. */
