@@ -80,9 +80,18 @@ void plan_symmetric_into(const SystemDesc* sys, int32_t first, int32_t count, in
     }
     b.grid = static_cast<int32_t>(std::max<int64_t>(1, std::min<int64_t>(max_grid, units)));
     b.begin0 = static_cast<int32_t>(plan.seg_begin.size());
-    // CTA k takes the units whose starting charge is in [k, k + 1) * total / grid.
-    auto bound = [&](int64_t k) {
-      return static_cast<int64_t>((static_cast<__int128>(k) * total + b.grid - 1) / b.grid);
+    // CTA k takes the units whose starting charge is in [k, k + 1) * total / grid: `bound`
+    // is (k + 1) * total / grid rounded up, kept as quotient and remainder, as a division
+    // per segment (two, of 128 bits) took most of the planning.
+    const int64_t share = total / b.grid, rest = total % b.grid;
+    int64_t k = 0, quot = share, rem = rest;
+    int64_t bound = quot + (rem > 0);
+    auto next_bound = [&] {
+      ++k;
+      quot += share;
+      rem += rest;
+      if (rem >= b.grid) rem -= b.grid, ++quot;
+      bound = quot + (rem > 0);
     };
     int64_t c0 = 0;
     int32_t next_cta = 0, slot = 0;
@@ -94,10 +103,9 @@ void plan_symmetric_into(const SystemDesc* sys, int32_t first, int32_t count, in
       int32_t jt = c.t0;
       while (jt < c.t1) {
         const int64_t at = c0 + c.upto(jt);
-        int64_t k = std::min<int64_t>(b.grid - 1,
-                                      static_cast<int64_t>(static_cast<__int128>(at) * b.grid / total));
+        while (k + 1 < b.grid && at >= bound) next_bound();
         int32_t end = c.t1;
-        if (k + 1 < b.grid) end = std::max(jt + 1, c.reach(bound(k + 1) - c0));
+        if (k + 1 < b.grid) end = std::max(jt + 1, c.reach(bound - c0));
         while (next_cta <= k) {
           plan.seg_begin.push_back(static_cast<int32_t>(plan.segs.size()));
           ++next_cta;
@@ -126,25 +134,49 @@ void plan_symmetric_into(const SystemDesc* sys, int32_t first, int32_t count, in
 // Largest grid that link_segments_into orders (it sorts on the stack).
 constexpr int32_t kSymMaxOrdered = 8192;
 
+// `order` receives the indices of `charge` (n of them), the lightest first and of equal
+// ones the last first.  Charges are the same to within a unit or two, so they are counted
+// where their range allows (1,216 of them: 4 us, 31 with std::sort).
+inline void order_by_charge(const uint32_t* charge, int32_t n, int32_t* order) {
+  constexpr uint32_t kBins = 2048;
+  uint32_t lo = charge[0], hi = charge[0];
+  for (int32_t k = 1; k < n; ++k) {
+    lo = std::min(lo, charge[k]);
+    hi = std::max(hi, charge[k]);
+  }
+  if (hi - lo < kBins) {
+    int32_t at[kBins + 1] = {};
+    for (int32_t k = 0; k < n; ++k) ++at[charge[k] - lo + 1];
+    for (uint32_t c = 0; c <= hi - lo; ++c) at[c + 1] += at[c];
+    for (int32_t k = n - 1; k >= 0; --k) order[at[charge[k] - lo]++] = k;
+    return;
+  }
+  for (int32_t k = 0; k < n; ++k) order[k] = k;
+  std::sort(order, order + n, [charge](int32_t a, int32_t b) {
+    return charge[a] != charge[b] ? charge[a] < charge[b] : a > b;
+  });
+}
+
 // `out` holds plan.segs.size() segments.  The rest as link_segments.
 template <class Plan, class Out>
 void link_segments_into(const Plan& plan, int32_t tiles_per_i, int32_t schedulers, int diag_cost,
                         int pair_cost, Out& out) {
-  uint64_t order[kSymMaxOrdered];  // charge of a CTA above its index
+  uint32_t charge[kSymMaxOrdered];
+  int32_t order[kSymMaxOrdered];
   for (const SymBand& b : plan.bands) {
     const auto first = plan.seg_begin.begin() + b.begin0;
     const bool ordered = schedulers > 0 && b.grid > schedulers && b.grid <= kSymMaxOrdered;
     for (int32_t k = 0; ordered && k < b.grid; ++k) {
-      uint64_t charge = 0;
+      uint64_t sum = 0;
       for (int32_t q = first[k]; q < first[k + 1]; ++q) {
         const SymSegment& sg = plan.segs[q];
         const int32_t td = std::max(sg.jt0, std::min(sg.jt1, (sg.itile + 1) * tiles_per_i));
-        charge += static_cast<uint64_t>(td - sg.jt0) * diag_cost +
-                  static_cast<uint64_t>(sg.jt1 - td) * pair_cost + pair_cost / 5;
+        sum += static_cast<uint64_t>(td - sg.jt0) * diag_cost +
+               static_cast<uint64_t>(sg.jt1 - td) * pair_cost + pair_cost / 5;
       }
-      order[k] = charge << 32 | static_cast<uint32_t>(b.grid - 1 - k);
+      charge[k] = static_cast<uint32_t>(std::min<uint64_t>(sum, UINT32_MAX));
     }
-    if (ordered) std::sort(order, order + b.grid);  // backwards: heaviest last
+    if (ordered) order_by_charge(charge, b.grid, order);
     int32_t more = b.grid;  // the next free place behind the first segments
     for (int32_t p = 0; p < b.grid; ++p) {
       int32_t k = p;
@@ -153,7 +185,7 @@ void link_segments_into(const Plan& plan, int32_t tiles_per_i, int32_t scheduler
         const int32_t round = p / schedulers, p0 = round * schedulers;
         const int32_t len = std::min(schedulers, b.grid - p0);
         const int32_t rank = round % 2 == 1 ? p : p0 + len - 1 - (p - p0);
-        k = b.grid - 1 - static_cast<int32_t>(order[b.grid - 1 - rank] & 0xffffffffu);
+        k = order[b.grid - 1 - rank];
       }
       int32_t at = p;
       for (int32_t q = first[k]; q < first[k + 1]; ++q) {
