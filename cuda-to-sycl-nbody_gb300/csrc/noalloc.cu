@@ -12,7 +12,7 @@
 // list, the partial sums and the rows of j-side sums -- lives in one file-scope device
 // array, kNaScratchBytes long; larger systems run in bands of i-tiles that take turns in
 // it (20,000 particles 216 us per call with the tuned kernel and its list uploaded on
-// every call, 131 now).  Small systems run the direct kernel, which needs
+// every call, 126 now).  Small systems run the direct kernel, which needs
 // none of it.  Every GPU that loads this module keeps that array
 // until the process exits.  All calls share it and it keeps the last call's contents:
 // the work list stays for the next call of the same size, unless a call fails on the way.
@@ -117,7 +117,7 @@ int na_upload_system(DeviceSetup& d, uint64_t n, float G, cudaStream_t st) {
 
 // Plan n particles and put the plan into the scratch, in one copy.  A call of another size
 // than the last takes that much longer (us per call, the same size / sizes in turn: 5,000
-// particles 24 / 51, 20,000 131 / 190, 25,000 206 / 315; planned by trial, with 128-bit
+// particles 24 / 51, 20,000 126 / 158, 25,000 193 / 253; planned by trial, with 128-bit
 // divisions and four copies, 84, 296 and 538; the tuned kernel with its list uploaded on
 // every call 55, 216 and 284).
 int na_upload(DeviceSetup& d, uint64_t n, float G, bool copied, cudaStream_t st) {
@@ -160,7 +160,7 @@ extern "C" int nb_accelerations_noalloc(const float* pos_xyzm_device, uint64_t n
   if (n == 0 || n > static_cast<uint64_t>(kNaMaxParticles))
     return set_error(NB_ERR_INVALID_ARGUMENT,
                      "nb_accelerations_noalloc takes 1 to 262144 particles (its fixed "
-                     "13 MiB device scratch); use nb_sim_accelerations for more");
+                     "18 MiB device scratch); use nb_sim_accelerations for more");
   if (!std::isfinite(G) || !std::isfinite(dist_eps) || dist_eps < 0.f)
     return set_error(NB_ERR_INVALID_ARGUMENT, "G and dist_eps must be finite, dist_eps >= 0");
   int dev = 0;

@@ -15,7 +15,11 @@
 namespace nbg {
 
 constexpr int64_t kNaMaxParticles = 1 << 18;  // 262,144
-constexpr size_t kNaScratchBytes = 13u << 20;
+// What the largest plans take on a full grid: 262,144 particles in one buffer for input and
+// output, 10 MB of parts (152 CTAs), 3.1 MB for an i-tile's row, 4.2 MB for the copy of the
+// positions, 0.5 MB for the list.  13 MiB left them 83 CTAs (us per call: 30,900 and 18,930
+// now; one i-tile per band either way), and put 20,000 particles into two bands (131 / 126).
+constexpr size_t kNaScratchBytes = 18u << 20;
 
 // Bounds: at most 64 i-tiles of 4,096 particles, each a band of its own on up to 152
 // CTAs; the smaller shapes are chosen for at most about 128 i-tiles, in a few bands on

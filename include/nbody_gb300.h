@@ -377,7 +377,7 @@ int nb_sim_adjoint_backward_device(nb_sim* s, const float* gx_T_device,
  * `pos_xyzm_device` and receives float4 (ax, ay, az, 0) in `accel_xyzw_device`
  * (both device memory, 16-byte aligned); a = G * sum_{j != i} m_j r_ij /
  * (|r_ij|^2 + dist_eps)^(3/2).  The call allocates no memory: its scratch is one
- * fixed 13 MiB device array inside the library, which limits n to 262,144
+ * fixed 18 MiB device array inside the library, which limits n to 262,144
  * (larger n: NB_ERR_INVALID_ARGUMENT) and which every GPU that loads the library
  * keeps until the process exits.  The first call on a device looks that array up
  * and should come before any stream capture.  All calls share the array, which

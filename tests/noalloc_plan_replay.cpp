@@ -1,7 +1,7 @@
 // Replays the planner of nb_accelerations_noalloc (csrc/noalloc_plan.hpp) on the host.
 // Arguments: threads, i-particles per thread and j-tile of its kNaCount shapes, then SMs and
 // the CTAs per SM of each shape, then the sizes from, to and step.  Prints the first plan
-// that is refused, does not fit or does not cover every block once.
+// that is refused, does not fit, leaves SMs idle or does not cover every block once.
 #include <cstdio>
 #include <cstdlib>
 #include <vector>
@@ -22,6 +22,7 @@ const char* check(const SystemDesc& sd, const SymCandidate& c) {
         at.rows + 12 * static_cast<size_t>(plan.row_values) <= (at.copy ? at.copy : at.end) &&
         at.end <= kNaScratchBytes && at.partials <= kNaMaxImage))
     return "layout";
+  if (plan.bands[0].grid != c.max_grid) return "idle CTAs";
   const SymSegment* segs = reinterpret_cast<const SymSegment*>(image + at.segs);
   const SymTile* tiles = reinterpret_cast<const SymTile*>(image + at.tiles);
   std::vector<char> seen(static_cast<size_t>(njt));

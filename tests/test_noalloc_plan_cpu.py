@@ -1,6 +1,6 @@
 """The planner of nb_accelerations_noalloc (csrc/noalloc_plan.hpp), replayed on the host over
-its whole range: no plan is refused, each fits the fixed tables and the scratch, and
-covers every (i-tile, j-tile) block once."""
+its whole range: no plan is refused, each fits the fixed tables and the scratch on the
+full grid, and covers every (i-tile, j-tile) block once."""
 from __future__ import annotations
 
 import os
@@ -40,7 +40,7 @@ def replay(tmp_path_factory):
 # smallest that plans (smaller ones run the direct kernel) to the largest.
 @pytest.mark.parametrize("sms,per_sm", [(152, (1, 8, 8)), (152, (1, 8, 16)), (152, (1, 9, 16)),
                                         (160, (1, 8, 16)), (148, (1, 8, 12))])
-def test_every_plan_fits(replay, sms, per_sm):
+def test_every_plan_fits_on_the_full_grid(replay, sms, per_sm):
     replay(sms, per_sm, 4690, 32768, 61)
     replay(sms, per_sm, 32768, LARGEST, 1021)
     replay(sms, per_sm, LARGEST - 1, LARGEST, 1)
