@@ -449,6 +449,17 @@ static int build_reference_order_worklist(nb_sim* s, int shape) {
   return NB_OK;
 }
 
+// The tuned-kernel list of an armed failure, for whatever shape is selected by the time of
+// the launch.
+static int build_inject_worklist(nb_sim* s) {
+  const int32_t nsys = static_cast<int32_t>(s->sys_h.size());
+  WorkListDev w;
+  NB_TRY(plan_tuned(s, default_config_for(s, 0, nsys, false), 0, nsys, 0, &w));
+  free_worklist(s->inject_wl);
+  s->inject_wl = w;
+  return NB_OK;
+}
+
 // One work list per system for the one-launch-per-system baseline.  Policy
 // kPerSystemOwnShape plans each system with the shape it would get as a
 // simulation of its own (default_config_for / default_reference_order_for), the
@@ -505,8 +516,9 @@ int launch_with(nb_sim* s, ForceArgs a, const WorkListDev& list) {
   a.counters = s->counters_d;
   a.inject = s->inject;
   s->inject = 0;
-  // The failure hooks make a bounded wait run out; only the tuned kernel has them.
+  // The failure hooks make a bounded wait run out; the symmetric and direct kernels have none.
   const WorkListDev& w = a.inject != 0 && is_untuned(list.cfg) ? s->inject_wl : list;
+  if (w.grid < 1) return set_error(NB_ERR_STATE, "no work list for this launch");
   if (is_direct(w.cfg)) {
     NB_CUDA(launch_direct(w.cfg - first_direct(),
                           s->params.accumulator == NB_ACC_COMPENSATED, s->per_pair_mass,
@@ -546,6 +558,24 @@ int launch_with(nb_sim* s, ForceArgs a, const WorkListDev& list) {
   return NB_OK;
 }
 
+// One launch per system.  The hooked launch of an armed failure covers its system alone.
+static int launch_each_system(nb_sim* s, const ForceArgs& a) {
+  for (int32_t k = 0; k < static_cast<int32_t>(s->wl_sys.size()); ++k) {
+    if (s->inject == 0 || !is_untuned(s->wl_sys[k].cfg)) {
+      NB_TRY(launch_with(s, a, s->wl_sys[k]));
+      continue;
+    }
+    WorkListDev w;
+    NB_TRY(plan_tuned(s, default_config_for(s, k, 1, false), k, 1, 0, &w));
+    const int st = launch_with(s, a, w);
+    const cudaError_t e = cudaStreamSynchronize(s->stream);
+    free_worklist(w);
+    NB_TRY(st);
+    NB_CUDA(e);
+  }
+  return NB_OK;
+}
+
 // One force evaluation: integrate into the other buffer (accel_out == nullptr)
 // or write accelerations.  `per_system` (kPerSystem*) issues one launch per system.
 int force_pass(nb_sim* s, float4* accel_out, int per_system) {
@@ -565,13 +595,13 @@ int force_pass(nb_sim* s, float4* accel_out, int per_system) {
       NB_CUDA(launch_reference_order_dup(a.pos, s->n_pad, s->ro_dup_d, s->stream));
     }
     if (per_system) {
-      for (const auto& w : s->wl_sys) NB_TRY(launch_with(s, a, w));
+      NB_TRY(launch_each_system(s, a));
     } else {
       NB_TRY(launch_with(s, a, s->ro_wl));
     }
   } else if (per_system) {
     NB_TRY(build_per_system_worklists(s, per_system));
-    for (const auto& w : s->wl_sys) NB_TRY(launch_with(s, a, w));
+    NB_TRY(launch_each_system(s, a));
   } else {
     NB_TRY(launch_with(s, a, s->wl));
   }
@@ -1442,6 +1472,7 @@ int nb_sim_set_shard(nb_sim* s, uint64_t first, uint64_t count) {
   for (auto& w : s->wl_sys) free_worklist(w);
   s->wl_sys.clear();
   s->wl_sys_policy = -1;
+  if (s->inject != 0) NB_TRY(build_inject_worklist(s));
   s->adj.valid = false;
   NB_CUDA(cudaStreamSynchronize(s->stream));
   return NB_OK;
@@ -1562,10 +1593,7 @@ int nb_sim_inject_failure(nb_sim* s, int32_t kind) {
     return set_error(NB_ERR_STATE, "the failure hooks cover the BRANCH kernels only");
   if (kind == NB_INJECT_HAND_OVER_WITHHELD && !reference_order_mode(s))
     return set_error(NB_ERR_STATE, "hand-overs exist in NB_ACC_REFERENCE_ORDER only");
-  if (is_untuned(s->cfg) && s->inject_wl.segs == nullptr) {
-    const int32_t nsys = static_cast<int32_t>(s->sys_h.size());
-    NB_TRY(plan_tuned(s, default_config_for(s, 0, nsys, false), 0, nsys, 0, &s->inject_wl));
-  }
+  NB_TRY(build_inject_worklist(s));
   s->inject = kind == NB_INJECT_TILE_NEVER_COPIED ? kInjectSkipFirstTile : kInjectWithholdHandOver;
   return NB_OK;
 }
