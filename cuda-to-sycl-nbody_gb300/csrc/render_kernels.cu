@@ -23,6 +23,7 @@
 // places rounded more finely).
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 #include "nb_device.cuh"
@@ -439,6 +440,25 @@ int blur_y_reach(const RenderUniforms& u) {
   return static_cast<int>(u.offset[u.taps - 1] * u.size_y * u.oh) + 2;
 }
 
+// Images lower than about 60 rows: taps so far apart that the rows need more shared memory
+// than a kernel has by default, 48 KB with its static arrays (94 KB at 16 rows, the lowest
+// image).  The limit belongs to the kernel on the device, not to a simulation: it is
+// raised once and never lowered, as another thread may be about to launch a lower image.
+constexpr int kBlurMaxSmem = 112 * 1024;
+
+cudaError_t blur_y_opt_in() {
+  static std::atomic<uint64_t> opted{0};  // once per device ordinal (>= 64: every call)
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = dev >= 0 && dev < 64 ? uint64_t{1} << dev : 0;
+  if (bit != 0 && (opted.load(std::memory_order_acquire) & bit) != 0) return cudaSuccess;
+  e = cudaFuncSetAttribute(blur_y_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           kBlurMaxSmem);
+  if (e == cudaSuccess && bit != 0) opted.fetch_or(bit, std::memory_order_release);
+  return e;
+}
+
 }  // namespace
 
 int64_t render_luminance_parts(const RenderUniforms& u) {
@@ -488,14 +508,9 @@ cudaError_t launch_render(const float* pos, const float4* vel, int64_t n_pad,
                        b.blur1, b.block_sums);
   if (e != cudaSuccess) return e;
   const dim3 blk(32, 8);
-  // Images lower than about 60 rows: taps so far apart that the rows need more shared
-  // memory than a kernel has by default (98 KB at 16 rows), 48 KB with its static arrays.
   const int reach_y = blur_y_reach(u);
   const int smem_y = static_cast<int>(sizeof(float2)) * 32 * (kBlurRows + 2 * reach_y);
-  if (smem_y > 40 * 1024 &&
-      (e = cudaFuncSetAttribute(blur_y_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                smem_y)) != cudaSuccess)
-    return e;
+  if (smem_y > 40 * 1024 && (e = blur_y_opt_in()) != cudaSuccess) return e;
   const dim3 gy((u.ow + 31) / 32, (u.oh + kBlurRows - 1) / kBlurRows + 1);
   e = launch_dependent(blur_y_kernel, gy, blk, smem_y, stream, b.blur1, u, reach_y, b.block_sums,
                        render_luminance_parts(u), b.mean, b.blur2);
