@@ -39,6 +39,7 @@ struct WorkListDev {
   SymTile* sym_tiles = nullptr;
   std::vector<SymBand> bands;
   int64_t row_values = 0;
+  size_t parts = 0;              // float4 records of partial sums that its launches write
 };
 
 // Checkpoints and work buffers of the adjoint (allocated on first use).

@@ -238,10 +238,10 @@ static int part_records(const nb_sim* s, int cfg) {
   return s->params.accumulator == NB_ACC_COMPENSATED || either ? 2 : 1;
 }
 
-static int ensure_scratch(nb_sim* s, const WorkListDev& w, int bi, int rec) {
-  const size_t need = static_cast<size_t>(w.slots) * bi * rec;
+static int ensure_scratch(nb_sim* s, WorkListDev& w, int bi, int rec) {
+  w.parts = static_cast<size_t>(w.slots) * bi * rec;
   NB_TRY(grow(s, &s->rows_d, &s->rows_cap, 3 * static_cast<size_t>(w.row_values)));
-  NB_TRY(grow(s, &s->partials_d, &s->partials_cap, need));
+  NB_TRY(grow(s, &s->partials_d, &s->partials_cap, w.parts));
   if (w.bands.size() > 1 && !s->carry_d)
     NB_TRY(dev_alloc(&s->carry_d, 2 * static_cast<size_t>(s->n_pad)));
   if (static_cast<size_t>(w.nfix) > s->counters_cap) {
@@ -250,6 +250,28 @@ static int ensure_scratch(nb_sim* s, const WorkListDev& w, int bi, int rec) {
     NB_CUDA(cudaMemsetAsync(s->counters_d, 0, w.nfix * sizeof(int32_t), s->stream));
   }
   return NB_OK;
+}
+
+// Give back the symmetric kernel's scratch (up to 256 MiB of rows, and its parts) once no
+// list needs rows: after another shape was selected, and where the fall-back to the tuned
+// kernel left a part of it behind.  The graphs are gone by then.
+static void trim_scratch(nb_sim* s) {
+  bool rows = s->wl.row_values > 0 || s->adj.wl.row_values > 0;
+  size_t parts = std::max({s->wl.parts, s->inject_wl.parts, s->ro_wl.parts, s->adj.wl.parts});
+  for (const auto& w : s->wl_sys) {
+    rows = rows || w.row_values > 0;
+    parts = std::max(parts, w.parts);
+  }
+  if (rows || !s->rows_d) return;
+  dev_free(s->rows_d);
+  s->rows_cap = 0;
+  dev_free(s->carry_d);
+  float4* smaller = nullptr;
+  if (s->partials_cap > parts && dev_alloc(&smaller, parts) == NB_OK) {
+    dev_free(s->partials_d);
+    s->partials_d = smaller;
+    s->partials_cap = parts;
+  }
 }
 
 static int max_grid_for(nb_sim* s, int cfg, bool live = false) {
@@ -727,6 +749,7 @@ static int build_default_worklist(nb_sim* s) {
   NB_TRY(st);
   s->cfg = cfg;
   s->cfg_default = true;
+  trim_scratch(s);
   return NB_OK;
 }
 
@@ -1262,6 +1285,7 @@ int nb_sim_set_kernel_config(nb_sim* s, int32_t index) {
   NB_TRY(build_main_worklist(s, index));
   s->cfg = index;
   s->cfg_default = false;
+  trim_scratch(s);
   return NB_OK;
 }
 
@@ -1353,6 +1377,7 @@ int nb_sim_autotune(nb_sim* s, int32_t* chosen) {
   s->cfg = best;
   s->cfg_default = false;
   if (chosen) *chosen = best;
+  trim_scratch(s);
   return NB_OK;
 }
 
@@ -1474,6 +1499,8 @@ int nb_sim_set_shard(nb_sim* s, uint64_t first, uint64_t count) {
   s->wl_sys_policy = -1;
   if (s->inject != 0) NB_TRY(build_inject_worklist(s));
   s->adj.valid = false;
+  free_worklist(s->adj.wl);  // a shard has no adjoint; a whole system plans it again
+  trim_scratch(s);
   NB_CUDA(cudaStreamSynchronize(s->stream));
   return NB_OK;
 }
