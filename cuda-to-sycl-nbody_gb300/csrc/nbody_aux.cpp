@@ -60,11 +60,14 @@ int adjoint_shape_for(const nb_sim* s, int* grid) {
 int ensure_adjoint_buffers(nb_sim* s, int32_t ncp, int32_t every) {
   AdjointState& a = s->adj;
   const size_t np = static_cast<size_t>(s->n_pad);
+  // Each buffer by itself: a call that failed between two of them leaves the first.
   while (static_cast<int32_t>(a.ckpt_pos.size()) < ncp) {
     float* p = nullptr;
-    float4* v = nullptr;
     NB_TRY(dev_alloc(&p, 4 * np));
     a.ckpt_pos.push_back(p);
+  }
+  while (static_cast<int32_t>(a.ckpt_vel.size()) < ncp) {
+    float4* v = nullptr;
     NB_TRY(dev_alloc(&v, np));
     a.ckpt_vel.push_back(v);
   }
@@ -77,12 +80,8 @@ int ensure_adjoint_buffers(nb_sim* s, int32_t ncp, int32_t every) {
     NB_CUDA(launch_fill_padding(p, a.vel, s->n_pad, s->stream));
     a.seg_pos.push_back(p);
   }
-  if (!a.lam_x) {
-    NB_TRY(dev_alloc(&a.lam_x, np));
-    NB_TRY(dev_alloc(&a.lam_v, np));
-    NB_TRY(dev_alloc(&a.mu, np));
-    NB_TRY(dev_alloc(&a.tmp, np));
-  }
+  for (float4** p : {&a.lam_x, &a.lam_v, &a.mu, &a.tmp})
+    if (!*p) NB_TRY(dev_alloc(p, np));
   if (a.wl.grid == 0) {
     const int32_t nsys = static_cast<int32_t>(s->sys_h.size());
     bool pays = false;
