@@ -98,10 +98,17 @@ int ensure_adjoint_buffers(nb_sim* s, int32_t ncp, int32_t every) {
     int grid = 0;
     a.shape = adjoint_shape_for(s, &grid);
     const KernelShape sh = adjoint_shape(a.shape);
-    const SymPlanHost h =
-        plan_symmetric(s->sys_h.data(), 0, nsys, sh.bi(), sh.bj, grid,
-                       kSymScratchBytes / kSymRowBytes, kAdjDiagCost, kAdjPairCost);
-    NB_TRY(upload_symmetric(s, h, sh, 1, kAdjDiagCost, kAdjPairCost, &a.wl));
+    // In as few bands as the device has room for, down to one i-tile's row.
+    for (int64_t values = kSymScratchBytes / kSymRowBytes;;) {
+      const SymPlanHost h = plan_symmetric(s->sys_h.data(), 0, nsys, sh.bi(), sh.bj, grid, values,
+                                           kAdjDiagCost, kAdjPairCost);
+      const int st = upload_symmetric(s, h, sh, 1, kAdjDiagCost, kAdjPairCost, &a.wl);
+      if (st != NB_ERR_OUT_OF_MEMORY || values == 0) {
+        NB_TRY(st);
+        break;
+      }
+      values = std::min(values, h.row_values) / 2;
+    }
   }
   return NB_OK;
 }

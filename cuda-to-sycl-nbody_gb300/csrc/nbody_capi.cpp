@@ -502,7 +502,11 @@ static int build_per_system_worklists(nb_sim* s, int policy) {
       cfg = ro ? -1 - default_reference_order_for(s, k, 1) : default_config_for(s, k, 1);
     WorkListDev w;
     if (cfg >= 0) {
-      NB_TRY(plan_config(s, cfg, k, 1, &w));
+      int st = plan_config(s, cfg, k, 1, &w);
+      // As build_default_worklist: the tuned kernel where there is no room for the rows.
+      if (st == NB_ERR_OUT_OF_MEMORY && is_untuned(cfg))
+        st = plan_tuned(s, default_config_for(s, k, 1, false), k, 1, 0, &w);
+      NB_TRY(st);
     } else {
       const KernelShape sh = shape_of(cfg);
       const WorkListHost h = plan_worklist(s->sys_h.data(), k, 1, sh.bi(), sh.bj,
