@@ -432,8 +432,10 @@ __device__ __forceinline__ void roj_step(const float4 A, const float4 B, float2 
   }
 }
 
-// U j-pairs' differences and roots.
-template <int U>
+// U j-pairs' differences and roots, none of them the thread's own particle: PREDICATED
+// multiplies their terms by zero, which leaves zero or NaN whatever the order, so they are
+// added in pairs.
+template <int U, bool kPred>
 struct RojBlock {
   float2 rx[U], ry[U], rz[U], inv[U];
   __device__ __forceinline__ void roots(const float4* __restrict__ tile, float2 nx, float2 ny,
@@ -451,9 +453,28 @@ struct RojBlock {
       float2 t = __fmul2_rn(d2, d2);
       t = __fmul2_rn(t, d2);
       inv[u] = make_float2(rsqrtf(t.x), rsqrtf(t.y));
+      if (kPred) {
+        rx[u] = __fmul2_rn(rx[u], inv[u]);
+        ry[u] = __fmul2_rn(ry[u], inv[u]);
+        rz[u] = __fmul2_rn(rz[u], inv[u]);
+      }
     }
   }
   __device__ __forceinline__ void add(float3& f) const {
+    if (kPred) {
+      const float2 zero = make_float2(0.f, 0.f);
+      float2 zx = zero, zy = zero, zz = zero;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        zx = __ffma2_rn(rx[u], zero, zx);
+        zy = __ffma2_rn(ry[u], zero, zy);
+        zz = __ffma2_rn(rz[u], zero, zz);
+      }
+      f.x += zx.x + zx.y;
+      f.y += zy.x + zy.y;
+      f.z += zz.x + zz.y;
+      return;
+    }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       f.x = __fmaf_rn(rx[u].x, inv[u].x, f.x);
@@ -469,16 +490,17 @@ struct RojBlock {
 // j = j0 .. j0 + count - 1 of the staged tile, in order.  Without masks, blocks of U
 // j-pairs are pipelined: the next block's roots are independent of the sums the current
 // one is added to, which hides part of a lone warp's latencies (12,800 particles: 135 ->
-// 127 us per step).
+// 127 us per step; PREDICATED 50,000: 1,276 -> 1,153,
+// an i-pair per thread 1,176).
 template <bool kDiag, bool kPred, int U>
 __device__ __forceinline__ void roj_tile(const float4* __restrict__ tile, int count, int j0,
                                          float2 e2, float2 nx, float2 ny, float2 nz, float3& f,
                                          int li) {
   const int pairs = count >> 1;
   int p = 0;
-  if constexpr (!kDiag && !kPred) {
+  if constexpr (!kDiag) {
     if (pairs >= 2 * U) {
-      RojBlock<U> b0, b1;
+      RojBlock<U, kPred> b0, b1;
       b0.roots(tile, nx, ny, nz, e2);
 #pragma unroll 1
       for (; p + 4 * U <= pairs; p += 2 * U) {
