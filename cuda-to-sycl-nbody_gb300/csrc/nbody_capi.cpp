@@ -741,10 +741,11 @@ static int default_config_for(nb_sim* s, int32_t first, int32_t count, bool symm
 }
 
 // The all-systems work list of the default config.  Where the symmetric kernel's
-// scratch does not fit the device any more, the tuned kernel's shape instead.
+// scratch does not fit the device any more, the tuned kernel's shape instead, and in
+// PREDICATED mode, which runs neither and needs no scratch.
 static int build_default_worklist(nb_sim* s) {
   const int32_t nsys = static_cast<int32_t>(s->sys_h.size());
-  int cfg = default_config_for(s, 0, nsys);
+  int cfg = default_config_for(s, 0, nsys, s->params.calc_method == NB_BRANCH);
   int st = build_main_worklist(s, cfg);
   if (st == NB_ERR_OUT_OF_MEMORY && is_untuned(cfg)) {
     cfg = default_config_for(s, 0, nsys, false);

@@ -96,3 +96,16 @@ def test_nothing_stays_of_a_scratch_that_failed(case):
             held.append(start - free_bytes())
             check_step(sim, pos, vel, m)
     assert len(held) >= 3 and max(held) - min(held) <= SLACK, held
+
+
+def test_predicated_holds_no_scratch(case):
+    # Its kernels need a list of work and, for the i-pair shapes, 32 bytes per particle.
+    pos, vel, _ = case
+    held = []
+    for method in (nb.PREDICATED, nb.BRANCH):
+        start = free_bytes()
+        with nb.Simulation(params(N, method=method, acc=nb.ACC_COMPENSATED), pos, vel, None) as sim:
+            held.append(start - free_bytes())
+            sim.advance(1)
+            sim.synchronize()
+    assert held[0] + ROWS - SLACK <= held[1], held
