@@ -217,9 +217,6 @@ static int grow(nb_sim* s, T** p, size_t* cap, size_t need) {
   return NB_OK;
 }
 
-// Records per slot and i-particle of config `cfg`: (hi, lo) for the compensated tuned
-// and symmetric kernels, one otherwise (the reference-order kernel's hand-over holds one
-// float4 per particle).
 // Whether config `cfg` keeps compensated sums: in COMPENSATED mode, and in PLAIN where the
 // compensated kernel is the faster one.
 static bool compensates(const nb_sim* s, int cfg) {
@@ -228,8 +225,10 @@ static bool compensates(const nb_sim* s, int cfg) {
           symmetric_always_compensates(cfg - num_force_configs(), s->per_pair_mass));
 }
 
-// Records of a part that config `cfg` may write.  A list outlives the masses it was planned
-// with (nb_sim_set_state), so this is the larger of both kinds of masses.
+// Records per slot and i-particle that config `cfg` may write: (hi, lo) for compensated sums,
+// one otherwise (the reference-order kernel's hand-over holds one float4 per particle).  A
+// list outlives the masses it was planned with (nb_sim_set_state), so this is the larger
+// of both kinds of masses.
 static int part_records(const nb_sim* s, int cfg) {
   if (cfg < 0) return 1;
   const bool either = is_symmetric(cfg) &&
@@ -711,9 +710,9 @@ static int default_symmetric_for(nb_sim* s, int32_t first, int32_t count) {
 // tuned / symmetric: N = 64 4.9 / 3.8, 2,048 12.3 / 7.4, 25,600 242 / 164, 262,144 21,712
 // / 14,420, 1,048,576 346,673 / 228,500; ensembles of 4,096 systems up to 8,192 particles
 // 10,577 / 7,466, of 2,000 up to 300 49.8 / 35.6).  Deterministic (the autotuner may pick
-// otherwise, and shapes round differently).  A shard integrates part of a system against all of it, which is not
-// symmetric, and launches that must fail on purpose need the tuned kernel's waits
-// (`symmetric` false): there, the tuned shape with the largest tiles whose work list
+// otherwise, and shapes round differently).  A shard integrates part of a system against
+// all of it, which is not symmetric, and launches that must fail on purpose need the tuned
+// kernel's waits (`symmetric` false): there, the tuned shape with the largest tiles whose work list
 // still gives every CTA at least 16 (i-tile, j-tile) blocks, so that the stream-K split
 // balances to within a few percent; the smallest shape otherwise.  Measured against the
 // autotuner's pick among the tuned shapes: N = 25,600 -> 256 x 2 x 256 (0.24 ms, the 1M

@@ -6,9 +6,9 @@
 // What bounds it: the FP32 FMA pipe.  One side of a pair costs 11 lane operations
 // (force_kernel.cuh); both sides cost 14, because only the three multiply-adds of the
 // sum are repeated: 7 per interaction.  Measured, ms per step against the tuned kernel
-// (compensated, equal masses): N = 1,048,576 228.5 (347.1), 262,144 14.42 (21.7), 100,003
+// (compensated, equal masses): N = 1,048,576 229.0 (347.1), 262,144 14.42 (21.7), 100,003
 // with per-particle masses, plain 2.52 (3.56), 25,600 0.164 (0.242); the FMA pipe is 84 %
-// busy at 262,144 and 77 % at 25,600 (one-warp CTAs: two warps per scheduler, of which the
+// busy at 262,144 and 75 % at 25,600 (one-warp CTAs: two warps per scheduler, of which the
 // older runs at its full rate and the younger in its gaps until it is alone).
 //
 //   * Each thread holds 2 P i-particles, two per packed FP32x2 register pair.  A warp

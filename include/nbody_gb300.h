@@ -212,8 +212,8 @@ typedef enum nb_inject_kind {
 int nb_sim_inject_failure(nb_sim* s, int32_t kind);
 /* Failure-detection test hook, host side only: the `nth` device allocation the
  * library makes from now on (1 = the next one, in any thread) fails with
- * NB_ERR_OUT_OF_MEMORY without calling cudaMalloc; 0 disarms it.  Lets tests
- * drive every clean-up path.  No reference counterpart (the reference exits on
+ * NB_ERR_OUT_OF_MEMORY, by a request that no device can serve; 0 disarms it.  Lets
+ * tests drive every clean-up path.  No reference counterpart (the reference exits on
  * any CUDA error, simulator.cuh:22-31). */
 int nb_inject_alloc_failure(int32_t nth);
 /* Wait for the stream and report any device-side error (e.g. a wait that timed out). */
@@ -381,10 +381,10 @@ int nb_sim_adjoint_backward_device(nb_sim* s, const float* gx_T_device,
  * (larger n: NB_ERR_INVALID_ARGUMENT) and which every GPU that loads the library
  * keeps until the process exits.  The first call on a device looks that array up
  * and should come before any stream capture.  All calls share the array, which
- * keeps the last call's contents (a call of the same n and G finds its work list
- * there, unless the last call failed); calls whose work overlapped on the GPU would race on it, so each call holds a
- * process-wide lock until its work has finished: calls from several threads or
- * streams of one process run one after another.  Runs on `stream` and waits for
+ * keeps the last call's contents (a call of the same n finds its work list there,
+ * unless the last call failed); calls whose work overlapped on the GPU would race on
+ * it, so each call holds a process-wide lock until its work has finished: calls from
+ * several threads or streams of one process run one after another.  Runs on `stream` and waits for
  * it before returning.  Both pointers may be the same buffer. */
 int nb_accelerations_noalloc(const float* pos_xyzm_device, uint64_t n, float G, float dist_eps,
                              float* accel_xyzw_device, void* stream);
